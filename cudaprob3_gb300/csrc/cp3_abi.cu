@@ -83,7 +83,8 @@ struct cp3_propagator {
     DevBuf<float2> d_ph_hm;
     bool avg_dirty = true;
     DevBuf<float2> d_seg_len_df;
-    DevBuf<double> d_table64;
+    DevBuf<double> d_table64;   // FP64 with production-height averaging
+    DevBuf<int2> d_table_fx;    // FP64 without
     DevBuf<double> d_plane;  // getProbabilityArr: one channel, transposed on the device
     DevBuf<float> d_table32;
     DevBuf<char> d_result;
@@ -303,11 +304,9 @@ int prepare_atmos(cp3_propagator* h) {
         CP3_CUDA(h, cudaMemcpy(h->d_cls_rho_df.ptr, pairs.data(), sizeof(float2) * pairs.size(),
                                cudaMemcpyHostToDevice), "upload classes");
     }
-    const size_t cells = (size_t)h->ncls_used * pad_energies(h->ne);
-    if (h->precision == CP3_FP64)
-        CP3_CUDA(h, h->d_table64.reserve(cells * kF64Fields), "allocate eigen table");
-    else
-        CP3_CUDA(h, h->d_table32.reserve(cells * kMixFields), "allocate eigen table");
+    if (h->precision == CP3_MIXED)
+        CP3_CUDA(h, h->d_table32.reserve((size_t)h->ncls_used * pad_energies(h->ne) * kMixFields),
+                 "allocate eigen table");
     h->traj_dirty = false;
     return CP3_OK;
 }
@@ -420,10 +419,21 @@ int launch(cp3_propagator* h, int type, cudaStream_t s, void* host_dst = nullptr
         AvgMixed avm;
         rc = prepare_averaging(h, &av, &avm);
         if (rc) return rc;
-        mark(0);
         const bool mixed = h->precision == CP3_MIXED;
+        // FP64 with constant densities: the averaging reads the FP64 table, everything else
+        // the fixed-point one
+        const bool fx = !mixed && !h->model.poly && av.n_bins == 0;
+        if (fx)
+            CP3_CUDA(h, h->d_table_fx.reserve(table_fx_words(h->ncls_used, h->ne)), "allocate eigen table");
+        else if (!mixed && !h->model.poly)
+            CP3_CUDA(h, h->d_table64.reserve((size_t)h->ncls_used * pad_energies(h->ne) * kF64Fields),
+                     "allocate eigen table");
+        mark(0);
         if (!h->model.poly) {
-            if (mixed)
+            if (fx)
+                e = launch_table_fx(p, h->d_energies.ptr, h->ne, h->d_cls_rho.ptr, h->ncls_used,
+                                    h->d_table_fx.ptr, s);
+            else if (mixed)
                 e = launch_table_mixed(p, h->d_energies_df.ptr, h->ne, h->d_cls_rho_df.ptr,
                                        h->ncls_used, h->d_table32.ptr, s);
             else
@@ -449,6 +459,10 @@ int launch(cp3_propagator* h, int type, cudaStream_t s, void* host_dst = nullptr
                 return launch_atmos_mixed(p, h->d_table32.ptr, h->ne, h->d_seg_off.ptr,
                                           h->d_seg_len_df.ptr, h->nc,
                                           (float*)h->d_result.ptr, s, rr);
+            if (fx)
+                return launch_atmos_fx(p, h->d_energies.ptr, h->ne, h->d_table_fx.ptr,
+                                       h->d_cls_rho.ptr, h->ncls_used, h->d_seg_off.ptr,
+                                       h->d_seg_len.ptr, h->nc, (double*)h->d_result.ptr, s, rr);
             return launch_atmos_f64(p, h->d_energies.ptr, h->ne, h->d_table64.ptr,
                                     h->d_seg_off.ptr, h->d_seg_len.ptr, h->nc,
                                     av, (double*)h->d_result.ptr, s, rr);

@@ -1,0 +1,565 @@
+// cp3_fixed.cuh -- the FP64 atmospheric bins in 64-bit fixed point, on the integer pipe.
+//
+// Why: GB300 retires one FP64 multiply-add per sub-partition and warp in 64 cycles (measured;
+// an FP32 one takes one), and the FP64 per-bin kernel was bound by it (89 % of the pipe active).
+// Everything after the eigen tables is bounded arithmetic: entries of unitary matrices, sines
+// and cosines, probabilities, all at most 1 in magnitude.  As fixed-point numbers with 62
+// fraction bits they carry 9 bits more than a double near 1, and a product costs three 32 x 32
+// -> 64-bit integer multiply-adds (4.5 cycles each), a quarter of an FP64 one's time.
+//
+// A value is h 2^-30 + l 2^-62 with both words signed; products keep h h and the two cross
+// terms (the dropped l l is below 2^-62).  Sums of products accumulate in 64 bits: by
+// Cauchy-Schwarz a dot product of unit vectors with three terms (or two complex ones) keeps
+// the cross terms below 2^63 in one accumulator, longer ones use two.
+//
+// All functions are plain integer arithmetic but for the phase reduction (four FP64 operations
+// a phase), and run on the host as well.
+#pragma once
+
+#include <cstring>
+
+#include "cp3_device.cuh"
+
+namespace cp3 {
+
+// Table fields (8 bytes each, [class][field][ne_pad], so that a warp reads 256 contiguous bytes
+// a field): R_c = U_{c+1}^T U_c row by row as fixed-point word pairs (the rotation from the
+// eigenbasis of class c to that of class c + 1; none for the last class), then the phase rates
+// of eigenstates 1 and 2 in turns per km as doubles.
+constexpr int kFxRates = 9;
+constexpr int kFxFields = 11;
+// After the classes, once per energy: the electron and muon rows of W U_1 and of W U_0 (three
+// real, three complex numbers each; U_c = [u0 u1 u2] of class c, class 0 the air), and the
+// vacuum coefficients of a bin that crosses no shell.
+constexpr int kFxV1 = 0, kFxV0 = 9, kFxVac = 18, kFxExtra = 31;
+
+struct fx {
+    int h, l;
+};
+struct cfx {
+    fx re, im;
+};
+
+CP3_HD fx fx_split(long long v) {
+    return fx{(int)(v >> 32) + (int)((unsigned int)v >> 31), (int)v};
+}
+CP3_HD long long fx_value(fx a) { return (long long)(((unsigned long long)(long long)a.h << 32) + (unsigned long long)(long long)a.l); }
+CP3_HD fx fx_neg(fx a) { return fx{-a.h, -a.l}; }
+CP3_HD fx fx_of(int2 v) { return fx{v.x, v.y}; }
+
+// |v| < 2
+CP3_HD long long fx_from_double(double v) {
+#ifdef __CUDA_ARCH__
+    return __double2ll_rn(__dmul_rn(v, 4611686018427387904.0));
+#else
+    return (long long)llrint(v * 4611686018427387904.0);
+#endif
+}
+
+CP3_HD long long fx_bits(double v) {
+#ifdef __CUDA_ARCH__
+    return __double_as_longlong(v);
+#else
+    long long b;
+    std::memcpy(&b, &v, sizeof b);
+    return b;
+#endif
+}
+CP3_HD double fx_bits_to_double(long long b) {
+#ifdef __CUDA_ARCH__
+    return __longlong_as_double(b);
+#else
+    double v;
+    std::memcpy(&v, &b, sizeof v);
+    return v;
+#endif
+}
+
+// A fixed-point number in [0, 2) as a double (below 0, by the last bits of its sums: 0).
+CP3_HD double fx_to_double(long long v) {
+    if (v <= 0) return 0.0;
+    return fx_bits_to_double(fx_bits((double)v) - (62LL << 52));
+}
+
+// Accumulators: fxacc for at most three products of unit-vector entries (two of complex ones),
+// fxacc2, whose cross terms have an accumulator each, for up to three complex products.
+struct fxacc {
+    long long hh = 0, x = 0;
+};
+struct fxacc2 {
+    long long hh = 0, x = 0, y = 0;
+};
+CP3_HD void fx_mac(fxacc& s, fx a, fx b) {
+    s.hh += (long long)a.h * b.h;
+    s.x += (long long)a.h * b.l;
+    s.x += (long long)a.l * b.h;
+}
+CP3_HD void fx_mac(fxacc2& s, fx a, fx b) {
+    s.hh += (long long)a.h * b.h;
+    s.x += (long long)a.h * b.l;
+    s.y += (long long)a.l * b.h;
+}
+CP3_HD long long fx_sum(const fxacc& s) { return s.hh * 4 + (s.x >> 30); }
+CP3_HD long long fx_sum(const fxacc2& s) { return s.hh * 4 + (s.x >> 30) + (s.y >> 30); }
+template <class Acc>
+CP3_HD fx fx_res(const Acc& s) {
+    return fx_split(fx_sum(s));
+}
+
+// a b for |a| = 1
+CP3_HD cfx fx_cmul(cfx a, cfx b) {
+    const fx n = fx_neg(a.im);
+    fxacc r, i;
+    fx_mac(r, a.re, b.re);
+    fx_mac(r, n, b.im);
+    fx_mac(i, a.re, b.im);
+    fx_mac(i, a.im, b.re);
+    return cfx{fx_res(r), fx_res(i)};
+}
+
+// ---- sine and cosine --------------------------------------------------------------------
+// cos and sin of 2 pi k / 512, 62 fraction bits, evaluated by the compiler: the Taylor series
+// of the angle's distance to the nearest axis, at most pi / 4, in 62-bit fixed point (a few
+// units of 2^-62).
+constexpr int kTrigBits = 9, kTrigSize = 1 << kTrigBits;
+
+struct TrigTable {
+    long long cs[kTrigSize][2];
+};
+
+constexpr long long trig_mul(long long a, long long b) { return (long long)(((__int128)a * b + ((__int128)1 << 61)) >> 62); }
+
+constexpr TrigTable make_trig_table() {
+    TrigTable t{};
+    const long long one = 1LL << 62;
+    const __int128 pi60 = 3622009729038561421LL;  // pi 2^60
+    for (int k = 0; k <= kTrigSize / 8; k++) {
+        const long long x = (long long)((pi60 * k * 4 + kTrigSize / 4) / (kTrigSize / 2));  // 2 pi k / 512
+        const long long x2 = trig_mul(x, x);
+        long long s = 0, c = 0;  // Horner: 1 - x^2/(n (n-1)) (1 - ...)
+        for (int n = 24; n >= 2; n -= 2) {
+            c = one - trig_mul(x2, (n == 24 ? one : c)) / (n * (n - 1));
+            s = one - trig_mul(x2, (n == 24 ? one : s)) / (n * (n + 1));
+        }
+        s = trig_mul(x, s);
+        if (k == 0) {
+            c = one;
+            s = 0;
+        }
+        const int q = kTrigSize / 4;
+        // the eight octants
+        t.cs[k][0] = c, t.cs[k][1] = s;
+        t.cs[q - k][0] = s, t.cs[q - k][1] = c;
+        t.cs[q + k][0] = -s, t.cs[q + k][1] = c;
+        t.cs[2 * q - k][0] = -c, t.cs[2 * q - k][1] = s;
+        t.cs[2 * q + k][0] = -c, t.cs[2 * q + k][1] = -s;
+        t.cs[3 * q - k][0] = -s, t.cs[3 * q - k][1] = -c;
+        t.cs[3 * q + k][0] = s, t.cs[3 * q + k][1] = -c;
+        t.cs[(4 * q - k) % kTrigSize][0] = c, t.cs[(4 * q - k) % kTrigSize][1] = -s;
+    }
+    t.cs[0][1] = 0;
+    return t;
+}
+
+// A phase of t = w L turns: table index (t in 512ths, any integer multiple of 512 away) and the
+// remaining angle in radians, 58 fraction bits, |x| <= pi / 512.
+struct FxAngle {
+    int k;
+    long long x;
+};
+
+// w L is rounded to a multiple of 1/512 by adding 1.5 2^43 (whose last place that is); the FMA
+// leaves the remainder of the exact product with one rounding, 2^-63, and another FMA takes it
+// to radians in the last places of 1.5 2^-6.  `bad` collects the exponents: bits above 19 come
+// up where w L is not finite or beyond 2^42 turns, and the caller takes the FP64 path then.
+CP3_HD FxAngle fx_angle(double w, double L, unsigned int& bad) {
+    constexpr double kRound = 13194139533312.0;  // 1.5 2^43
+    constexpr double kPlace = 0.0234375;         // 1.5 2^-6
+    const double q = fma(w, L, kRound);
+    const double n = q - kRound;
+    const double r = fma(w, L, -n);
+    const double u = fma(r, 6.283185307179586477, kPlace);
+    const long long qb = fx_bits(q), ub = fx_bits(u);
+    bad |= (unsigned int)(qb >> 32) ^ 0x42A00000u;
+    bad |= (unsigned int)(ub >> 32) ^ 0x3F900000u;
+    return FxAngle{(int)qb, ub - 0x3F98000000000000LL};
+}
+
+// cos and sin of an angle: the table's entry T rotated by the remaining x, with
+// sin x = x (1 - p), p = x^2/6 (1 - x^2/20), and cos x - 1 = -x^2/2 (1 - s),
+// s = x^2/12 (1 - x^2/30); |x| <= 0.0062, so p and s need one word.  x, sin x and cos x - 1 are
+// held times 2^7.  Error about 2^-56 (an FP64 sincos rounds at 2^-54).
+CP3_HD void fx_sincos(FxAngle a, const longlong2* trig, fx& c, fx& s) {
+    const longlong2 T = trig[a.k & (kTrigSize - 1)];
+    const fx tc = fx_split(T.x), ts = fx_split(T.y), nts = fx_neg(ts);
+    const long long X = a.x << 11;
+    const fx x = fx_split(X);
+    const long long w = (long long)x.h * x.h * 4 + (((long long)x.h * x.l) >> 29);  // x^2 2^14
+    const int w31 = (int)(w >> 31);                                                 // 31 fraction bits
+    const int d = (int)(((long long)w31 * 8738) >> 32);                             // (4/3) 2^30 x^2/20
+    const int p48 = (int)(((long long)w31 * (1431655765 - d)) >> 30);               // p 2^48
+    const unsigned int s48 = (unsigned int)(((unsigned long long)(unsigned int)w31 * (2863311531u - (unsigned int)(d + (d >> 2)))) >> 32);
+    const long long xp = (long long)x.h * p48 + (((long long)x.l * p48) >> 32);
+    const fx sn = fx_split(X - (xp >> 16));
+    const fx cm = fx_split((((long long)w31 * (int)s48) >> 25) - (w >> 8));
+    fxacc ac, as;
+    fx_mac(ac, tc, cm);
+    fx_mac(ac, nts, sn);
+    fx_mac(as, ts, cm);
+    fx_mac(as, tc, sn);
+    c = fx_split(T.x + (ac.hh >> 5) + (ac.x >> 37));
+    s = fx_split(T.y + (as.hh >> 5) + (as.x >> 37));
+}
+
+// e^{-i phi} of one phase; k and x add up to the determinant's phase.
+CP3_HD cfx fx_unit(FxAngle a, const longlong2* trig) {
+    cfx e;
+    fx_sincos(a, trig, e.re, e.im);
+    e.im = fx_neg(e.im);
+    return e;
+}
+
+// ---- a bin ------------------------------------------------------------------------------
+// One energy column of the table.
+struct FxColumn {
+    const int2* tab;   // at this energy: field f of class c at tab[c * cls_stride + f * stride]
+    const int2* ext;   // extra field f at ext[f * stride]
+    size_t stride, cls_stride;
+    CP3_HD int2 load(const int2* p) const {
+#ifdef __CUDA_ARCH__
+        return __ldg(p);
+#else
+        return *p;
+#endif
+    }
+    CP3_HD fx rot(int c, int f) const { return fx_of(load(tab + c * cls_stride + f * stride)); }
+    CP3_HD fx extra(int f) const { return fx_of(load(ext + f * stride)); }
+    CP3_HD double rate(int c, int k) const {
+        const int2 v = load(tab + c * cls_stride + (kFxRates + k) * stride);
+        return fx_bits_to_double((long long)(((unsigned long long)(unsigned int)v.y << 32) | (unsigned int)v.x));
+    }
+};
+
+CP3_HD void fx_layer(const FxColumn& t, int c, double L, const longlong2* trig, cfx e[2], unsigned int& bad) {
+#pragma unroll
+    for (int k = 0; k < 2; k++) e[k] = fx_unit(fx_angle(t.rate(c, k), L, bad), trig);
+}
+
+CP3_HD void fx_load_rotation(const FxColumn& t, int c, fx R[9]) {
+#pragma unroll
+    for (int f = 0; f < 9; f++) R[f] = t.rot(c, f);
+}
+
+// v <- R v
+CP3_HD void fx_rotate(const fx R[9], cfx v[3]) {
+    cfx o[3];
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        fxacc r, m;
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            fx_mac(r, R[i * 3 + k], v[k].re);
+            fx_mac(m, R[i * 3 + k], v[k].im);
+        }
+        o[i] = cfx{fx_res(r), fx_res(m)};
+    }
+#pragma unroll
+    for (int i = 0; i < 3; i++) v[i] = o[i];
+}
+
+// sum_k a_k b_k over three complex products
+CP3_HD cfx fx_cdot(cfx a0, cfx b0, cfx a1, cfx b1, cfx a2, cfx b2) {
+    fxacc2 r, m;
+    fx_mac(r, a0.re, b0.re), fx_mac(r, fx_neg(a0.im), b0.im), fx_mac(m, a0.re, b0.im), fx_mac(m, a0.im, b0.re);
+    fx_mac(r, a1.re, b1.re), fx_mac(r, fx_neg(a1.im), b1.im), fx_mac(m, a1.re, b1.im), fx_mac(m, a1.im, b1.re);
+    fx_mac(r, a2.re, b2.re), fx_mac(r, fx_neg(a2.im), b2.im), fx_mac(m, a2.re, b2.im), fx_mac(m, a2.im, b2.re);
+    return cfx{fx_res(r), fx_res(m)};
+}
+
+// conj(a x b)_i for entries j, k = i + 1, i + 2
+CP3_HD cfx fx_cross(cfx aj, cfx ak, cfx bj, cfx bk) {
+    fxacc2 r, m;
+    fx_mac(r, aj.re, bk.re), fx_mac(r, fx_neg(aj.im), bk.im), fx_mac(r, fx_neg(ak.re), bj.re), fx_mac(r, ak.im, bj.im);
+    const fx njr = fx_neg(aj.re), nji = fx_neg(aj.im);
+    fx_mac(m, njr, bk.im), fx_mac(m, nji, bk.re), fx_mac(m, ak.re, bj.im), fx_mac(m, ak.im, bj.re);
+    return cfx{fx_res(r), fx_res(m)};
+}
+
+CP3_HD long long fx_norm(cfx a) {
+    fxacc s;
+    fx_mac(s, a.re, a.re);
+    fx_mac(s, a.im, a.im);
+    return fx_sum(s);
+}
+
+// The four probabilities e->e, e->mu, mu->e, mu->mu (62 fraction bits) of one bin over M + 1
+// segments (lengths len[0..M] in km; segment l is class l); the other five follow from
+// unitarity.  Returns false where a phase left the reduction's range.
+//
+// With U_l the eigenvectors of layer l (columns, det = 1), D_l = diag(1, e1, e2) its phases and
+// R_l = U_{l+1}^T U_l, the amplitude W (S_1..S_{M-1}) S_M (S_{M-1}..S_1) S_0 W^+ of
+// S_l = U_l D_l U_l^T is
+//   A = (W U_1) Y^T D_M Y R_0 D_0 (W U_0)^+,   Y = R_{M-1} D_{M-1} ... R_1 D_1,
+// so a layer costs two complex multiplications and one real rotation per column of Y.  Y is
+// unitary with determinant e^{-i sum of the phases}: two of its columns are carried, 52
+// multiplications a layer (two rank-1 updates of three columns took 96), and the third is
+// det Y conj(y0 x y1) at the end.  Only the columns e and mu of A, and of these the rows e and
+// mu, are formed.
+CP3_HD bool fx_bin(const FxColumn& t, const double* len, int M, const longlong2* trig, long long P[4]) {
+    unsigned int bad = 0;
+    cfx e[2];
+    if (M == 0) {
+        // P = P0 + sum_k d_k cos D_k for the two survivals, and for the pair the same plus or
+        // minus J (sin D10 - sin D20 + sin D21)
+        fx_layer(t, 0, len[0], trig, e, bad);
+        fxacc a, b;
+        fx_mac(a, e[0].re, e[1].re), fx_mac(a, e[0].im, e[1].im);  // cos D21
+        fx_mac(b, e[0].im, e[1].re), fx_mac(b, fx_neg(e[0].re), e[1].im);  // sin D21 (e.im = -sin)
+        const fx c3 = fx_res(a);
+        const long long sines = (fx_value(e[1].im) >> 1) - (fx_value(e[0].im) >> 1) + (fx_sum(b) >> 1);
+        long long v[3];
+#pragma unroll
+        for (int q = 0; q < 3; q++) {
+            fxacc2 s;
+            fx_mac(s, t.extra(kFxVac + 4 * q + 1), e[0].re);
+            fx_mac(s, t.extra(kFxVac + 4 * q + 2), e[1].re);
+            fx_mac(s, t.extra(kFxVac + 4 * q + 3), c3);
+            v[q] = fx_value(t.extra(kFxVac + 4 * q)) + fx_sum(s);
+        }
+        fxacc j;
+        fx_mac(j, t.extra(kFxVac + 12), fx_split(sines));
+        const long long jt = fx_sum(j);
+        P[0] = v[0];
+        P[1] = v[2] + jt;
+        P[2] = v[2] - jt;
+        P[3] = v[1];
+        return (bad >> 20) == 0;
+    }
+    cfx y[3][3];
+    if (M > 1) {
+        int ks = 0;
+        long long xs = 0;
+        auto phases = [&](int l) {
+#pragma unroll
+            for (int k = 0; k < 2; k++) {
+                const FxAngle a = fx_angle(t.rate(l, k), len[l], bad);
+                ks += a.k;
+                xs += a.x;
+                e[k] = fx_unit(a, trig);
+            }
+        };
+        phases(1);
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+            const fx a = t.rot(1, 3 * i), b = t.rot(1, 3 * i + 1);
+            fxacc r, m;
+            fx_mac(r, b, e[0].re);
+            fx_mac(m, b, e[0].im);
+            y[0][i] = cfx{a, fx{0, 0}};
+            y[1][i] = cfx{fx_res(r), fx_res(m)};
+        }
+#pragma unroll 1
+        for (int l = 2; l < M; l++) {
+            fx R[9];
+            fx_load_rotation(t, l, R);
+            phases(l);
+#pragma unroll
+            for (int j = 0; j < 2; j++) {
+                y[j][1] = fx_cmul(e[0], y[j][1]);
+                y[j][2] = fx_cmul(e[1], y[j][2]);
+                fx_rotate(R, y[j]);
+            }
+        }
+        // the determinant's phase: 2 pi ks / 512 + xs, the second brought back below pi / 512
+        const double x = (double)xs * 3.469446951953614189e-18;  // 2^-58
+        const double m = rint(x * 81.48733086305041);            // 512 / (2 pi)
+        FxAngle d;
+        d.k = ks + (int)m;
+        d.x = xs - (long long)(int)m * 3537118876014220LL;  // (2 pi / 512) 2^58
+        const cfx det = fx_unit(d, trig);
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+            const int j = (i + 1) % 3, k = (i + 2) % 3;
+            y[2][i] = fx_cmul(det, fx_cross(y[0][j], y[0][k], y[1][j], y[1][k]));
+        }
+    }
+    cfx e0[2];
+    fx_layer(t, 0, len[0], trig, e0, bad);
+    fx_layer(t, M, len[M], trig, e, bad);
+    fx R0[9];
+    fx_load_rotation(t, 0, R0);
+#pragma unroll 1
+    for (int j = 0; j < 2; j++) {  // initial flavours e, mu
+        cfx k[3];
+        // D_0 (W U_0)^+ column j
+#pragma unroll
+        for (int i = 0; i < 3; i++)
+            k[i] = j == 0 ? cfx{t.extra(kFxV0 + i), fx{0, 0}}
+                          : cfx{t.extra(kFxV0 + 3 + i), fx_neg(t.extra(kFxV0 + 6 + i))};
+        k[1] = fx_cmul(e0[0], k[1]);
+        k[2] = fx_cmul(e0[1], k[2]);
+        fx_rotate(R0, k);
+        if (M > 1) {
+            cfx m[3];
+#pragma unroll
+            for (int i = 0; i < 3; i++) m[i] = fx_cdot(y[0][i], k[0], y[1][i], k[1], y[2][i], k[2]);
+            m[1] = fx_cmul(e[0], m[1]);
+            m[2] = fx_cmul(e[1], m[2]);
+#pragma unroll
+            for (int i = 0; i < 3; i++) k[i] = fx_cdot(y[i][0], m[0], y[i][1], m[1], y[i][2], m[2]);
+        } else {
+            k[1] = fx_cmul(e[0], k[1]);
+            k[2] = fx_cmul(e[1], k[2]);
+        }
+        cfx ae, am;
+        {
+            fxacc r, m;
+#pragma unroll
+            for (int i = 0; i < 3; i++) {
+                const fx v = t.extra(kFxV1 + i);
+                fx_mac(r, v, k[i].re);
+                fx_mac(m, v, k[i].im);
+            }
+            ae = cfx{fx_res(r), fx_res(m)};
+        }
+        am = fx_cdot(cfx{t.extra(kFxV1 + 3), t.extra(kFxV1 + 6)}, k[0], cfx{t.extra(kFxV1 + 4), t.extra(kFxV1 + 7)}, k[1],
+                     cfx{t.extra(kFxV1 + 5), t.extra(kFxV1 + 8)}, k[2]);
+        P[2 * j] = fx_norm(ae);
+        P[2 * j + 1] = fx_norm(am);
+    }
+    return (bad >> 20) == 0;
+}
+
+// All nine from the four: channel a*3+b at out[ch * plane].
+CP3_HD void fx_store(const long long P[4], double* __restrict__ out, size_t plane) {
+    const long long one = 1LL << 62;
+    const long long et = one - P[0] - P[1], mt = one - P[2] - P[3];
+    out[0] = fx_to_double(P[0]);
+    out[plane] = fx_to_double(P[1]);
+    out[2 * plane] = fx_to_double(et);
+    out[3 * plane] = fx_to_double(P[2]);
+    out[4 * plane] = fx_to_double(P[3]);
+    out[5 * plane] = fx_to_double(mt);
+    out[6 * plane] = fx_to_double(one - P[0] - P[2]);
+    out[7 * plane] = fx_to_double(one - P[1] - P[3]);
+    out[8 * plane] = fx_to_double(one - et - mt);
+}
+
+// ---- the table of one energy ------------------------------------------------------------
+// One class: U as nine fixed-point numbers (u[k] the eigenvectors 1, 2; u0 = u1 x u2) and the
+// phase rates 2.534 (m_k - m_0) / (2 pi E), each rounded once.  NaN rates where the vectors are
+// not finite or far from orthonormal, so that the bins take the FP64 path.
+//   U comes in orthonormal to FP64 rounding and is made so to the last places of the fixed-point
+// numbers by one Newton-Schulz step, U <- U - U (U^T U - 1) / 2.  A layer is U D U^T: where its
+// phases are small it is near 1 whatever the rotation U, but only if U U^T = 1.  Without the
+// step the rounding of U entered every layer (59 shells at 100 GeV: 1.4e-14 instead of 1e-15).
+struct FxClass {
+    fx U[3][3];  // [component][eigenstate]
+    double rate[2];
+};
+
+CP3_HD bool fx_entry_ok(double v) { return (unsigned int)((fx_bits(v) >> 32) & 0x7fffffff) <= 0x3FF00010u; }
+
+CP3_HD void fx_class(const double u[2][3], const double dmv[3], double E, FxClass& o, double u0[3]) {
+    u0[0] = u[0][1] * u[1][2] - u[0][2] * u[1][1];
+    u0[1] = u[0][2] * u[1][0] - u[0][0] * u[1][2];
+    u0[2] = u[0][0] * u[1][1] - u[0][1] * u[1][0];
+    bool ok = true;
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        ok = ok && fx_entry_ok(u0[i]) && fx_entry_ok(u[0][i]) && fx_entry_ok(u[1][i]);
+        o.U[i][0] = fx_split(fx_from_double(u0[i]));
+        o.U[i][1] = fx_split(fx_from_double(u[0][i]));
+        o.U[i][2] = fx_split(fx_from_double(u[1][i]));
+    }
+    long long C[6];
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+#pragma unroll
+        for (int j = i; j < 3; j++) {
+            fxacc s;
+#pragma unroll
+            for (int k = 0; k < 3; k++) fx_mac(s, o.U[k][i], o.U[k][j]);
+            const long long v = fx_sum(s) - (i == j ? 1LL << 62 : 0);
+            C[sidx(i, j)] = v;
+            ok = ok && v == (int)v;  // within 2^-31 of orthonormal
+        }
+    fx V[3][3];
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+#pragma unroll
+        for (int j = 0; j < 3; j++) {
+            long long s = 0;
+#pragma unroll
+            for (int k = 0; k < 3; k++) s += (long long)o.U[i][k].h * (int)C[sidx(k, j)];
+            V[i][j] = fx_split(fx_value(o.U[i][j]) - (s >> 31));
+        }
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+#pragma unroll
+        for (int j = 0; j < 3; j++) o.U[i][j] = V[i][j];
+    // 2.534 / (2 pi) = kA + kB
+    constexpr double kA = 0.40329862579486275, kB = -2.5640811661172617e-18;
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        const double d = dmv[k + 1] - dmv[0];
+        const double q = d * kA, e = fma(d, kA, -q) + d * kB;
+        const double w = q / E;
+        o.rate[k] = ok ? w + (fma(-w, E, q) + e) / E : fx_bits_to_double(0x7ff8000000000000LL);
+    }
+}
+
+// R = B^T A
+CP3_HD void fx_rotation(const fx B[3][3], const fx A[3][3], fx R[3][3]) {
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+#pragma unroll
+        for (int j = 0; j < 3; j++) {
+            fxacc s;
+#pragma unroll
+            for (int k = 0; k < 3; k++) fx_mac(s, B[k][i], A[k][j]);
+            R[i][j] = fx_res(s);
+        }
+}
+
+// The electron and muon rows of W U: U_e (real), and c u_1 + s e^{i d} u_2 as three real and
+// three imaginary parts; w = {c23, s23, cos d, sin d}.
+CP3_HD void fx_rows(const double u0[3], const double u[2][3], const double* w, fx row[9]) {
+    const double* v[3] = {u0, u[0], u[1]};
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        row[k] = fx_split(fx_from_double(v[k][0]));
+        row[3 + k] = fx_split(fx_from_double(w[0] * v[k][1] + w[1] * w[2] * v[k][2]));
+        row[6 + k] = fx_split(fx_from_double(w[1] * w[3] * v[k][2]));
+    }
+}
+
+// The coefficients of a bin that crosses no shell (the expansion of layer_coefficients64 in
+// cos D_jk itself): for e->e, mu->mu and the mean of e->mu and mu->e a constant and the factors
+// of cos D10, cos D20, cos D21; then twice the factor 2 J of the sines.
+CP3_HD void fx_vacuum(const double u[2][3], const double* w, fx v[13]) {
+    const double cc = w[0] * w[0], ss = w[1] * w[1], cs2 = 2.0 * w[0] * w[1];
+    double m[2][3];  // |U_ek|^2, |U_mu,k|^2
+#pragma unroll
+    for (int k = 1; k < 3; k++) {
+        const double* x = u[k - 1];
+        m[0][k] = x[0] * x[0];
+        m[1][k] = cc * x[1] * x[1] + ss * x[2] * x[2] + cs2 * w[2] * x[1] * x[2];
+    }
+    m[0][0] = 1.0 - m[0][1] - m[0][2];
+    m[1][0] = 1.0 - m[1][1] - m[1][2];
+    auto put = [&](int q, double c0, double a, double b, double c) {
+        v[4 * q] = fx_split(fx_from_double(c0 - a - b - c));
+        v[4 * q + 1] = fx_split(fx_from_double(a));
+        v[4 * q + 2] = fx_split(fx_from_double(b));
+        v[4 * q + 3] = fx_split(fx_from_double(c));
+    };
+#pragma unroll
+    for (int q = 0; q < 2; q++)
+        put(q, 1.0, 2.0 * m[q][0] * m[q][1], 2.0 * m[q][0] * m[q][2], 2.0 * m[q][1] * m[q][2]);
+    const double W0 = m[0][0] * m[1][0], W1 = m[0][1] * m[1][1], W2 = m[0][2] * m[1][2], S = W0 + W1 + W2;
+    put(2, 0.0, 2.0 * W2 - S, 2.0 * W1 - S, 2.0 * W0 - S);
+    v[12] = fx_split(fx_from_double(2.0 * cs2 * w[3] * (u[0][0] * u[1][0]) * (u[0][1] * u[1][2] - u[0][2] * u[1][1])));
+}
+
+}  // namespace cp3

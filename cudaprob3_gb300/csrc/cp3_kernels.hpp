@@ -27,6 +27,11 @@ cudaError_t launch_table_mixed(const OscParams& p, const double* energies, int n
 cudaError_t launch_table_mixed(const OscParams& p, const float2* energies, int ne,
                                const float2* cls_rho, int ncls, float* table, cudaStream_t s);
 
+// The table of the fixed-point FP64 bins (cp3_fixed.cuh), table_fx_words(ncls, ne) word pairs.
+size_t table_fx_words(int ncls, int ne);
+cudaError_t launch_table_fx(const OscParams& p, const double* energies, int ne,
+                            const double* cls_rho, int ncls, int2* table, cudaStream_t s);
+
 // Loads the mixed table kernel (the double-input instance) and the mixed per-bin kernel
 // into the current device's context, as their first launch would.  With lazy module
 // loading that first load may allocate device memory; a caller that must not allocate
@@ -55,6 +60,13 @@ cudaError_t launch_atmos_f64(const OscParams& p, const double* energies, int ne,
                              const double* table, const int* seg_off, const double* seg_len,
                              int n_cosines, const AvgArrays& avg, double* out,
                              cudaStream_t s, RowRange rr = RowRange{});
+// FP64 bins from the fixed-point table, constant densities and a fixed production height.
+// Bins whose table entries or phases are out of its range take the FP64 path, from the class
+// densities.
+cudaError_t launch_atmos_fx(const OscParams& p, const double* energies, int ne, const int2* table,
+                            const double* cls_rho, int ncls, const int* seg_off,
+                            const double* seg_len, int n_cosines, double* out, cudaStream_t s,
+                            RowRange rr = RowRange{});
 cudaError_t launch_atmos_mixed(const OscParams& p, const float* table, int ne,
                                const int* seg_off, const float2* seg_len, int n_cosines,
                                float* out, cudaStream_t s,

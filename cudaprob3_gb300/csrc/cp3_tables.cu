@@ -6,8 +6,11 @@
 // multiply and add separately rounded reproduces the reference's x86 results to the last
 // bits where the eigen-system is ill-conditioned.  The table work is O(classes x energies),
 // amortised over every cosine, so the missing contraction costs nothing that matters.
+#include <algorithm>
+
 #include "cp3_device.cuh"
 #include "cp3_f64.cuh"
+#include "cp3_fixed.cuh"
 #include "cp3_mixed.cuh"
 #include "cp3_kernels.hpp"
 
@@ -36,6 +39,60 @@ __global__ void __launch_bounds__(kTableBlock)
     t[2] = make_double2(u[1][1], u[1][2]);
     t[3] = make_double2(dmv[0], dmv[1]);
     t[4] = make_double2(dmv[2], 0.0);
+}
+
+// The table of the fixed-point FP64 bins (cp3_fixed.cuh): for each class the rotation to the
+// next class's eigenbasis and the phase rates, and once per energy the flavour rows and the
+// vacuum coefficients.  A block is 32 energies by a run of kFxRun classes, one class a warp;
+// the extra warp solves the class after the run, for the last rotation.
+constexpr int kFxRun = 8;
+
+__global__ void __launch_bounds__(32 * (kFxRun + 1))
+    table_fx_kernel(const __grid_constant__ OscParams p, const double* __restrict__ energies,
+                    int ne, int ne_pad, const double* __restrict__ cls_rho, int ncls,
+                    int2* __restrict__ table) {
+    __shared__ int2 s_u[kFxRun + 1][9][32];
+    const int lane = threadIdx.x & 31, wv = threadIdx.x >> 5;
+    const int ie = blockIdx.x * 32 + lane, c = blockIdx.y * kFxRun + wv;
+    const bool on = c < ncls && ie < ne;
+    FxClass k;
+    if (on) {
+        double u[2][3], dmv[3], u0[3];
+        const double E = energies[ie];
+        rotated_layer_f64(&p, E, cls_rho[c], u, dmv);
+        fx_class(u, dmv, E, k, u0);
+#pragma unroll
+        for (int f = 0; f < 9; f++) s_u[wv][f][lane] = make_int2(k.U[f / 3][f % 3].h, k.U[f / 3][f % 3].l);
+        int2* ext = table + (size_t)ncls * kFxFields * ne_pad + ie;
+        if (c < 2 && wv < 2) {  // (class 1 is wv 1 of the first run only)
+            fx row[9];
+            fx_rows(u0, u, p.w, row);
+#pragma unroll
+            for (int f = 0; f < 9; f++)
+                ext[(size_t)((c == 0 ? kFxV0 : kFxV1) + f) * ne_pad] = make_int2(row[f].h, row[f].l);
+        }
+        if (c == 0) {
+            fx v[13];
+            fx_vacuum(u, p.w, v);
+#pragma unroll
+            for (int f = 0; f < 13; f++) ext[(size_t)(kFxVac + f) * ne_pad] = make_int2(v[f].h, v[f].l);
+        }
+    }
+    __syncthreads();
+    if (!on || wv == kFxRun) return;  // (with fewer classes than a run there is no class after it)
+    int2* t = table + (size_t)c * kFxFields * ne_pad + ie;
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+        const long long b = fx_bits(k.rate[q]);
+        t[(size_t)(kFxRates + q) * ne_pad] = make_int2((int)b, (int)(b >> 32));
+    }
+    if (c + 1 == ncls) return;
+    fx B[3][3], R[3][3];
+#pragma unroll
+    for (int f = 0; f < 9; f++) B[f / 3][f % 3] = fx_of(s_u[wv + 1][f][lane]);
+    fx_rotation(B, k.U, R);
+#pragma unroll
+    for (int f = 0; f < 9; f++) t[(size_t)f * ne_pad] = make_int2(R[f / 3][f % 3].h, R[f / 3][f % 3].l);
 }
 
 // Mixed table: real unit eigenvectors u1, u2 of H0 + V e0 e0^T (P_k = u_k u_k^T) and the
@@ -84,6 +141,19 @@ cudaError_t launch_table_f64(const OscParams& p, const double* energies, int ne,
     if (ne <= 0 || ncls <= 0) return cudaSuccess;
     dim3 grid((ne + kTableBlock - 1) / kTableBlock, ncls);
     table_f64_kernel<<<grid, kTableBlock, 0, s>>>(p, energies, ne, pad_energies(ne), cls_rho, table);
+    return cudaGetLastError();
+}
+
+size_t table_fx_words(int ncls, int ne) {
+    return ((size_t)ncls * kFxFields + kFxExtra) * pad_energies(ne);
+}
+
+cudaError_t launch_table_fx(const OscParams& p, const double* energies, int ne,
+                            const double* cls_rho, int ncls, int2* table, cudaStream_t s) {
+    if (ne <= 0 || ncls <= 0) return cudaSuccess;
+    dim3 grid((ne + 31) / 32, (ncls + kFxRun - 1) / kFxRun);
+    table_fx_kernel<<<grid, 32 * (std::min(ncls, kFxRun) + 1), 0, s>>>(p, energies, ne, pad_energies(ne),
+                                                                       cls_rho, ncls, table);
     return cudaGetLastError();
 }
 

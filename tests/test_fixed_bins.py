@@ -1,0 +1,114 @@
+"""The FP64 atmospheric bins in fixed point: on the CPU (the same source built for the host)
+against the oracle over Earth models and parameter sets, with the range test that hands a bin
+to the FP64 path; on the GPU at the edges of its launch and of its table kernel."""
+import ctypes as C
+import os
+import shutil
+import subprocess
+
+import numpy as np
+import pytest
+
+from cudaprob3_gb300 import earth
+from oracle.oracle import Mixing as OMix
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+SRC = os.path.join(os.path.dirname(HERE), "cudaprob3_gb300", "csrc")
+dp = C.POINTER(C.c_double)
+
+
+@pytest.fixture(scope="module")
+def host(tmp_path_factory):
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    if not os.path.exists(nvcc):
+        pytest.skip("nvcc not found")
+    so = str(tmp_path_factory.mktemp("fixed") / "libfixed.so")
+    r = subprocess.run([nvcc, "-gencode", "arch=compute_103a,code=sm_103a", "-std=c++17", "-O2", "-shared",
+                        "-Xcompiler", "-fPIC,-ffp-contract=off", "-I", SRC,
+                        "-I", os.path.join(os.path.dirname(HERE), "include"),
+                        os.path.join(HERE, "cpp", "fixed_bins.cu"), os.path.join(SRC, "cp3_host.cpp"), "-o", so],
+                       capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr[-2000:]
+    return C.CDLL(so)
+
+
+def host_bins(lib, m, anti, cz, en, model, h):
+    a = [np.ascontiguousarray(x, dtype=np.float64)
+         for x in ([m.theta12, m.theta13, m.theta23, m.dcp, m.dm12sq, m.dm23sq], cz, en, *model)]
+    p = [x.ctypes.data_as(dp) for x in a]
+    out = np.empty((9, len(cz), len(en)))
+    n = lib.fixed_atmos(p[0], -1 if anti else 1, int(anti), p[1], len(cz), p[2], len(en), p[3], p[4], p[5],
+                        len(a[3]), C.c_double(h), out.ctypes.data_as(dp))
+    return np.transpose(out, (1, 2, 0)), n
+
+
+def omix(m, anti):
+    return OMix(m.theta12, m.theta13, m.theta23, m.dcp, m.dm12sq, m.dm23sq, -1 if anti else 1)
+
+
+def test_trig_table(host):
+    t = np.zeros((512, 2), dtype=np.int64)
+    host.fixed_trig(t.ctypes.data_as(C.c_void_p))
+    a = 2 * np.longdouble("3.14159265358979323846264") * np.arange(512) / 512
+    # 2^-53 of the double functions compared with
+    assert np.abs(t[:, 0] * 2.0 ** -62 - np.cos(a)).max() <= 4e-16
+    assert np.abs(t[:, 1] * 2.0 ** -62 - np.sin(a)).max() <= 4e-16
+
+
+@pytest.mark.parametrize("shells,h", [(1, 22.0), (2, 0.0), (3, 15.0), (12, 22.0), (59, 100.0), (128, 22.0)])
+def test_host_bins_against_oracle(host, oracle, shells, h):
+    """Both orderings, nu and nubar, vacuum-only rows, vertical and shell-grazing rows, at the
+    FP64 parity bar; every bin inside the fixed-point range."""
+    model = earth.synthetic_shells(shells)
+    cz = np.concatenate([np.linspace(-1, 1, 23), [-1e-9, -0.5]])
+    en = np.logspace(-1, 3, 17)
+    for m in earth.gaussian_sets(4, seed=7)[1:3]:
+        for anti in (False, True):
+            got, outside = host_bins(host, m, anti, cz, en, model, h)
+            assert outside == 0
+            ref = oracle.atmos(omix(m, anti), anti, cz, en, *model, h, layer_limit=128)
+            assert np.abs(got - ref).max() <= 1e-12
+
+
+def test_out_of_range_bins_ask_for_the_fp64_path(host):
+    """Energies that are not finite or zero, and phases past 2^42 turns (13 000 km at 1e-13 GeV
+    and below); the neighbouring energies stay inside."""
+    cz = np.array([-0.9, 0.5])
+    en = np.array([1.0, np.nan, 0.0, np.inf, 1e-16, 5.0])
+    with np.errstate(all="ignore"):
+        for i in range(len(en)):
+            _, outside = host_bins(host, earth.NOMINAL, False, cz, en[i:i + 1], earth.PREM_4LAYER, 22.0)
+            assert outside == (0 if i in (0, 5) else len(cz)), en[i]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shells,nc,ne", [(1, 1, 1), (1, 5, 33), (7, 4, 32), (8, 3, 31), (9, 6, 64), (16, 9, 65), (128, 13, 40)])
+def test_gpu_bins_at_the_edges_of_the_launch(oracle, shells, nc, ne):
+    """Rows and energies around a block's four warps of 32, class counts around the table
+    kernel's runs of eight, up to the largest model."""
+    from tests.gpu_helpers import run_atmos
+    model = earth.synthetic_shells(shells)
+    cz, en = np.linspace(-1, 0.4, nc), earth.log_energy_grid(ne)
+    m = earth.gaussian_sets(2, seed=8)[1]
+    mix6 = [m.theta12, m.theta13, m.theta23, m.dcp, m.dm12sq, m.dm23sq]
+    for anti in (False, True):
+        got = run_atmos("fp64", mix6, -1 if anti else 1, anti, cz, en, *model, 22.0)
+        assert np.abs(got - oracle.atmos(omix(m, anti), anti, cz, en, *model, 22.0, layer_limit=128)).max() <= 1e-12
+
+
+@pytest.mark.gpu
+def test_gpu_out_of_range_bins():
+    """A NaN energy gives NaN in its own column and leaves the others as they are.  An energy too
+    low for the fixed-point reduction takes the FP64 path: its phases (1e18 rad) have lost every
+    digit there, so the values only have to be finite."""
+    from tests.gpu_helpers import run_atmos
+    m = earth.NOMINAL
+    mix6 = [m.theta12, m.theta13, m.theta23, m.dcp, m.dm12sq, m.dm23sq]
+    cz, en = np.linspace(-1, 0.4, 7), earth.log_energy_grid(40)
+    ok = run_atmos("fp64", mix6, 1, False, cz, en, *earth.PREM_4LAYER, 22.0)
+    en[5], en[37] = np.nan, 1e-16
+    got = run_atmos("fp64", mix6, 1, False, cz, en, *earth.PREM_4LAYER, 22.0)
+    keep = [i for i in range(40) if i not in (5, 37)]
+    assert np.array_equal(got[:, keep], ok[:, keep])
+    assert np.isnan(got[:, 5]).all()
+    assert np.isfinite(got[:, 37]).all()
