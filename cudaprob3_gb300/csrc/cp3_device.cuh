@@ -421,10 +421,12 @@ __host__ __device__ __noinline__ inline void eigen_fallback_f64(const OscParams*
 // chains, whose vector errors add up over the layers); else in FP32 (the beam's one layer
 // per baseline).
 // The common path; false where the FP64 fallback has to take over (one call site for it,
-// below, so that no live range of the common path has to survive a call).
+// below, so that no live range of the common path has to survive a call).  With `pairs` the
+// double-float vectors themselves are returned (lane x: u_1, lane y: u_2) and P is not written.
 template <bool kDf>
 __device__ __forceinline__ bool rotated_eigen_mixed_try(const OscParams* __restrict__ p, df Ed,
-                                                        df rhod, float P[2][3], float om[2][2]) {
+                                                        df rhod, float P[2][3], float om[2][2],
+                                                        df2* pairs = nullptr) {
     // V = -fac of getMfast: +2 sqrt2 G_F N_e E for neutrinos, minus for antineutrinos.
     // (2 sqrt2 G_F) N_e comes first: constant over a beam's energies, the batched kernel
     // forms it once per tile (C3 1.2 % faster).
@@ -554,6 +556,10 @@ __device__ __forceinline__ bool rotated_eigen_mixed_try(const OscParams* __restr
 #pragma unroll
         for (int i = 0; i < 3; i++) {
             const df2 v = df2_mul(uu[i], rn);
+            if (pairs) {
+                pairs[i] = v;
+                continue;
+            }
             const float2 f = __fadd2_rn(v.hi, v.lo);
             P[0][i] = f.x;
             P[1][i] = f.y;

@@ -30,7 +30,7 @@ constexpr int kFxRates = 9;
 constexpr int kFxFields = 11;
 // After the classes, once per energy: the electron and muon rows of W U_1 and of W U_0 (three
 // real, three complex numbers each; U_c = [u0 u1 u2] of class c, class 0 the air), and the
-// vacuum coefficients of a bin that crosses no shell.
+// coefficients of a bin that crosses no shell.
 constexpr int kFxV1 = 0, kFxV0 = 9, kFxVac = 18, kFxExtra = 31;
 
 struct fx {
@@ -292,6 +292,33 @@ CP3_HD long long fx_norm(cfx a) {
     return fx_sum(s);
 }
 
+// The four probabilities of a single layer from its coefficients (fx_coefficients) and phases:
+// P = P0 + sum_k d_k cos D_k for the two survivals, and for the pair the same plus or minus
+// J (sin D10 - sin D20 + sin D21).
+CP3_HD void fx_one_layer(const fx v[13], const cfx e[2], long long P[4]) {
+    fxacc a, b;
+    fx_mac(a, e[0].re, e[1].re), fx_mac(a, e[0].im, e[1].im);          // cos D21
+    fx_mac(b, e[0].im, e[1].re), fx_mac(b, fx_neg(e[0].re), e[1].im);  // sin D21 (e.im = -sin)
+    const fx c3 = fx_res(a);
+    const long long sines = (fx_value(e[1].im) >> 1) - (fx_value(e[0].im) >> 1) + (fx_sum(b) >> 1);
+    long long r[3];
+#pragma unroll
+    for (int q = 0; q < 3; q++) {
+        fxacc2 s;
+        fx_mac(s, v[4 * q + 1], e[0].re);
+        fx_mac(s, v[4 * q + 2], e[1].re);
+        fx_mac(s, v[4 * q + 3], c3);
+        r[q] = fx_value(v[4 * q]) + fx_sum(s);
+    }
+    fxacc j;
+    fx_mac(j, v[12], fx_split(sines));
+    const long long jt = fx_sum(j);
+    P[0] = r[0];
+    P[1] = r[2] + jt;
+    P[2] = r[2] - jt;
+    P[3] = r[1];
+}
+
 // The four probabilities e->e, e->mu, mu->e, mu->mu (62 fraction bits) of one bin over M + 1
 // segments (lengths len[0..M] in km; segment l is class l); the other five follow from
 // unitarity.  Returns false where a phase left the reduction's range.
@@ -309,30 +336,11 @@ CP3_HD bool fx_bin(const FxColumn& t, const double* len, int M, const longlong2*
     unsigned int bad = 0;
     cfx e[2];
     if (M == 0) {
-        // P = P0 + sum_k d_k cos D_k for the two survivals, and for the pair the same plus or
-        // minus J (sin D10 - sin D20 + sin D21)
         fx_layer(t, 0, len[0], trig, e, bad);
-        fxacc a, b;
-        fx_mac(a, e[0].re, e[1].re), fx_mac(a, e[0].im, e[1].im);  // cos D21
-        fx_mac(b, e[0].im, e[1].re), fx_mac(b, fx_neg(e[0].re), e[1].im);  // sin D21 (e.im = -sin)
-        const fx c3 = fx_res(a);
-        const long long sines = (fx_value(e[1].im) >> 1) - (fx_value(e[0].im) >> 1) + (fx_sum(b) >> 1);
-        long long v[3];
+        fx v[13];
 #pragma unroll
-        for (int q = 0; q < 3; q++) {
-            fxacc2 s;
-            fx_mac(s, t.extra(kFxVac + 4 * q + 1), e[0].re);
-            fx_mac(s, t.extra(kFxVac + 4 * q + 2), e[1].re);
-            fx_mac(s, t.extra(kFxVac + 4 * q + 3), c3);
-            v[q] = fx_value(t.extra(kFxVac + 4 * q)) + fx_sum(s);
-        }
-        fxacc j;
-        fx_mac(j, t.extra(kFxVac + 12), fx_split(sines));
-        const long long jt = fx_sum(j);
-        P[0] = v[0];
-        P[1] = v[2] + jt;
-        P[2] = v[2] - jt;
-        P[3] = v[1];
+        for (int f = 0; f < 13; f++) v[f] = t.extra(kFxVac + f);
+        fx_one_layer(v, e, P);
         return (bad >> 20) == 0;
     }
     cfx y[3][3];
@@ -445,69 +453,245 @@ CP3_HD void fx_store(const long long P[4], double* __restrict__ out, size_t plan
     out[8 * plane] = fx_to_double(one - et - mt);
 }
 
-// ---- the table of one energy ------------------------------------------------------------
-// One class: U as nine fixed-point numbers (u[k] the eigenvectors 1, 2; u0 = u1 x u2) and the
-// phase rates 2.534 (m_k - m_0) / (2 pi E), each rounded once.  NaN rates where the vectors are
-// not finite or far from orthonormal, so that the bins take the FP64 path.
-//   U comes in orthonormal to FP64 rounding and is made so to the last places of the fixed-point
-// numbers by one Newton-Schulz step, U <- U - U (U^T U - 1) / 2.  A layer is U D U^T: where its
-// phases are small it is near 1 whatever the rotation U, but only if U U^T = 1.  Without the
-// step the rounding of U entered every layer (59 shells at 100 GeV: 1.4e-14 instead of 1e-15).
+// ---- eigen-systems ----------------------------------------------------------------------
+// One layer: U as nine fixed-point numbers (columns u0, u1, u2, det = 1) and the phase rates
+// 2.534 (m_k - m_0) / (2 pi E), k = 1, 2, in turns per km.  NaN rates mark a layer whose bins
+// take the FP64 path.
 struct FxClass {
     fx U[3][3];  // [component][eigenstate]
     double rate[2];
 };
 
-CP3_HD bool fx_entry_ok(double v) { return (unsigned int)((fx_bits(v) >> 32) & 0x7fffffff) <= 0x3FF00010u; }
+constexpr double kFxTurns = 0.40329862579486275;  // 2.534 / (2 pi)
 
-CP3_HD void fx_class(const double u[2][3], const double dmv[3], double E, FxClass& o, double u0[3]) {
-    u0[0] = u[0][1] * u[1][2] - u[0][2] * u[1][1];
-    u0[1] = u[0][2] * u[1][0] - u[0][0] * u[1][2];
-    u0[2] = u[0][0] * u[1][1] - u[0][1] * u[1][0];
-    bool ok = true;
+// v / 2^(kexp - 1023), |v| below that power of two, from the bits (truncated at 2^-62); kexp is
+// a biased double exponent.
+CP3_HD long long fx_scaled(double v, int kexp) {
+    const long long b = fx_bits(v);
+    const int e = (int)((b >> 52) & 0x7ff);
+    const long long m = (long long)(((unsigned long long)b & 0xfffffffffffffull) | 0x10000000000000ull) << 10;
+    const int sh = kexp - e;
+    const long long r = e == 0 || sh > 62 ? 0 : m >> sh;
+    return b < 0 ? -r : r;
+}
+CP3_HD int fx_exponent(double v) { return (int)((fx_bits(v) >> 52) & 0x7ff); }
+
+// u0 = u1 x u2
+CP3_HD void fx_third(fx U[3][3]) {
 #pragma unroll
     for (int i = 0; i < 3; i++) {
-        ok = ok && fx_entry_ok(u0[i]) && fx_entry_ok(u[0][i]) && fx_entry_ok(u[1][i]);
-        o.U[i][0] = fx_split(fx_from_double(u0[i]));
-        o.U[i][1] = fx_split(fx_from_double(u[0][i]));
-        o.U[i][2] = fx_split(fx_from_double(u[1][i]));
+        const int j = (i + 1) % 3, k = (i + 2) % 3;
+        fxacc s;
+        fx_mac(s, U[j][1], U[k][2]);
+        fx_mac(s, fx_neg(U[k][1]), U[j][2]);
+        U[i][0] = fx_res(s);
     }
-    long long C[6];
+}
+
+// C = U^T U - 1 (upper triangle); false unless within 2^-31 of orthonormal
+CP3_HD bool fx_overlap(const fx U[3][3], int C[6]) {
+    bool ok = true;
 #pragma unroll
     for (int i = 0; i < 3; i++)
 #pragma unroll
         for (int j = i; j < 3; j++) {
             fxacc s;
 #pragma unroll
-            for (int k = 0; k < 3; k++) fx_mac(s, o.U[k][i], o.U[k][j]);
+            for (int k = 0; k < 3; k++) fx_mac(s, U[k][i], U[k][j]);
             const long long v = fx_sum(s) - (i == j ? 1LL << 62 : 0);
-            C[sidx(i, j)] = v;
-            ok = ok && v == (int)v;  // within 2^-31 of orthonormal
+            C[sidx(i, j)] = (int)v;
+            ok = ok && v == (int)v;
         }
-    fx V[3][3];
+    return ok;
+}
+
+// U <- U + U X, X small, in units of 2^-62
+CP3_HD void fx_adjust(fx U[3][3], const int X[3][3]) {
 #pragma unroll
-    for (int i = 0; i < 3; i++)
+    for (int i = 0; i < 3; i++) {
+        fx r[3];
 #pragma unroll
         for (int j = 0; j < 3; j++) {
             long long s = 0;
 #pragma unroll
-            for (int k = 0; k < 3; k++) s += (long long)o.U[i][k].h * (int)C[sidx(k, j)];
-            V[i][j] = fx_split(fx_value(o.U[i][j]) - (s >> 31));
+            for (int k = 0; k < 3; k++) s += (long long)U[i][k].h * X[k][j];
+            r[j] = fx_split(fx_value(U[i][j]) + (s >> 30));
         }
+#pragma unroll
+        for (int j = 0; j < 3; j++) U[i][j] = r[j];
+    }
+}
+
+// From a nearly exact U to the eigen-system of H0 + V e0 e0^T in the last places of the
+// fixed-point numbers.  With M = U^T H U (H scaled below 1 by a power of two) and
+// C = U^T U - 1, the eigenvalues are M_ii - C_ii M_ii and the vectors U (1 + K - C / 2) with
+// K_ij = (M_ij - C_ij (M_ii + M_jj) / 2) / (m_j - m_i): first-order perturbation theory on top
+// of a start that is off by 1e-12 at most, so what is left is below 2^-62 (tested: K and C
+// within 2^-32 and 2^-31).  The phase rates come from the refined eigenvalues.
+//   C / 2 is the Newton-Schulz step to the nearest orthonormal U.  It is not optional: a layer
+// is U D U^T, near 1 whatever the rotation U where its phases are small, but only if
+// U U^T = 1.  With U orthonormal to FP64 rounding alone that rounding entered every layer
+// (59 shells at 100 GeV: 1.4e-14 instead of 1e-15).
+//   The same FP64 work -- the cubic's roots by the trigonometric formula, projectors, their
+// vectors -- took about 400 FP64 instructions (64 cycles each); this takes about 220 integer
+// multiply-adds (4.5 cycles) and 15 FP64 instructions.
+CP3_HD bool fx_refine(const OscParams* __restrict__ p, double E, double rE, double rho, FxClass& o) {
+    const double V = p->anti ? -(kTwoRtTwoGf * E * rho) : kTwoRtTwoGf * E * rho;
+    int kexp = fx_exponent(V);
+    const int k1 = fx_exponent(p->dm[3]), k2 = fx_exponent(p->dm[6]);
+    kexp = kexp > k1 ? kexp : k1;
+    kexp = (kexp > k2 ? kexp : k2) + 3;  // |V| + max |mu| < 2^(kexp - 1023) / 2
+    fx H[6];
+#pragma unroll
+    for (int q = 0; q < 6; q++) {
+        const long long h = fx_scaled(p->h0[q], kexp);
+        H[q] = fx_split(q == 0 ? h + fx_scaled(V, kexp) : h);
+    }
+    int C[6];
+    bool ok = fx_overlap(o.U, C);
+    long long M[6];
+#pragma unroll
+    for (int j = 0; j < 3; j++) {
+        fx g[3];
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+            fxacc s;
+#pragma unroll
+            for (int k = 0; k < 3; k++) fx_mac(s, H[sidx(i, k)], o.U[k][j]);
+            g[i] = fx_res(s);
+        }
+#pragma unroll
+        for (int i = 0; i <= j; i++) {
+            fxacc s;
+#pragma unroll
+            for (int k = 0; k < 3; k++) fx_mac(s, o.U[k][i], g[k]);
+            M[sidx(i, j)] = fx_sum(s);
+        }
+    }
+    long long m[3];
+    int mh[3];
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        const long long d = M[sidx(i, i)];
+        mh[i] = (int)(d >> 32);  // 30 fraction bits
+        m[i] = d - (((long long)mh[i] * C[sidx(i, i)]) >> 30);
+    }
+    int X[3][3];
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        X[i][i] = -(C[sidx(i, i)] >> 1);
+#pragma unroll
+        for (int j = i + 1; j < 3; j++) {
+            const int c = C[sidx(i, j)];
+            const long long off = M[sidx(i, j)] - (((long long)((mh[i] + mh[j]) >> 1) * c) >> 30);
+            // (float of the difference of the leading words is enough: K is a correction)
+            const float k = (float)off / ((float)(m[j] - m[i]) * 2.168404344971009e-19f);  // 2^-62
+            ok = ok && fabsf(k) < 1073741824.0f;
+            const int ki = ok ? (int)k : 0;
+            X[i][j] = ki - (c >> 1);
+            X[j][i] = -ki - (c >> 1);
+        }
+    }
+    fx_adjust(o.U, X);
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        const long long d = m[k + 1] - m[0];
+        // the difference in eV^2
+        const double dm = d == 0 ? 0.0 : fx_bits_to_double(fx_bits((double)d) + ((long long)(kexp - 1023 - 62) << 52));
+        o.rate[k] = ok ? dm * kFxTurns * rE : fx_bits_to_double(0x7ff8000000000000LL);
+    }
+    return ok;
+}
+
+// The layer from FP64 vectors and masses (rotated_layer_f64): where the fast solver declines.
+CP3_HD bool fx_entry_ok(double v) { return (unsigned int)((fx_bits(v) >> 32) & 0x7fffffff) <= 0x3FF00010u; }
+
+CP3_HD void fx_class_f64(const double u[2][3], const double dmv[3], double E, FxClass& o) {
+    bool ok = true;
 #pragma unroll
     for (int i = 0; i < 3; i++)
 #pragma unroll
-        for (int j = 0; j < 3; j++) o.U[i][j] = V[i][j];
-    // 2.534 / (2 pi) = kA + kB
-    constexpr double kA = 0.40329862579486275, kB = -2.5640811661172617e-18;
+        for (int k = 0; k < 2; k++) {
+            ok = ok && fx_entry_ok(u[k][i]);
+            o.U[i][k + 1] = fx_split(fx_from_double(u[k][i]));
+        }
+    fx_third(o.U);
+    int C[6], X[3][3];
+    ok = ok && fx_overlap(o.U, C);
 #pragma unroll
-    for (int k = 0; k < 2; k++) {
-        const double d = dmv[k + 1] - dmv[0];
-        const double q = d * kA, e = fma(d, kA, -q) + d * kB;
-        const double w = q / E;
-        o.rate[k] = ok ? w + (fma(-w, E, q) + e) / E : fx_bits_to_double(0x7ff8000000000000LL);
+    for (int i = 0; i < 3; i++)
+#pragma unroll
+        for (int j = 0; j < 3; j++) X[i][j] = -(C[sidx(i, j)] >> 1);
+    fx_adjust(o.U, X);
+#pragma unroll
+    for (int k = 0; k < 2; k++)
+        o.rate[k] = ok ? (dmv[k + 1] - dmv[0]) * kFxTurns / E : fx_bits_to_double(0x7ff8000000000000LL);
+}
+
+#ifdef __CUDACC__
+// x as a float pair, from its bits (conversions between double and float take the FP64 pipe).
+__device__ __forceinline__ bool fx_float_pair(double x, df& o) {
+    const long long b = __double_as_longlong(x);
+    const int e = (int)((b >> 52) & 0x7ff);
+    if ((b << 1) == 0) {
+        o = df{0.0f, 0.0f};
+        return true;
+    }
+    if (e < 1023 - 60 || e > 1023 + 60) return false;
+    const unsigned int sign = (unsigned int)(b >> 63) << 31;
+    const float hi = __uint_as_float(sign | ((unsigned int)(e - 896) << 23) | ((unsigned int)(b >> 29) & 0x7fffffu));
+    const float lo = (float)(unsigned int)(b & 0x1fffffff) * __uint_as_float(sign | ((unsigned int)(e - 948) << 23));
+    o = df_fast2sum(hi, lo);
+    return true;
+}
+__device__ __forceinline__ double fx_to_f64(float x) {  // normal or zero (zero: 1e-38)
+    const unsigned int b = __float_as_uint(x);
+    return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + 0x38000000u)), (int)(b << 29));
+}
+__device__ __forceinline__ fx fx_from_pair(float hi, float lo) {  // |hi + lo| <= 1
+    const int i = __float2int_rn(hi * 1073741824.0f);
+    const float rest = fmaf(-(float)i, 9.31322574615478515625e-10f, hi) + lo;  // 2^-30
+    return fx_split(((long long)i << 32) + __float2ll_rn(rest * 4611686018427387904.0f));
+}
+
+// 1 / E, rounded once but for a last-place error of the correction
+__device__ __forceinline__ double fx_reciprocal(double E, df Ed) {
+    const df r = df_recip(Ed);
+    const double r0 = fx_to_f64(r.hi) + fx_to_f64(r.lo);
+    return fma(fma(-E, r0, 1.0), r0, r0);
+}
+
+static __device__ __noinline__ void fx_solve_f64(const OscParams* __restrict__ p, double E, double rho, FxClass* o) {
+    double u[2][3], dmv[3];
+    rotated_layer_f64(p, E, rho, u, dmv);
+    fx_class_f64(u, dmv, E, *o);
+}
+
+// The layer of one (energy, electron density): double-float roots and vectors on the FP32 pipe
+// (rotated_eigen_mixed_try, 1e-14), refined in fixed point; the FP64 formulas where two levels
+// nearly meet or the vectors' formula has no content.
+__device__ __forceinline__ void fx_solve(const OscParams* __restrict__ p, double E, double rho, FxClass& o) {
+    df Ed, rd;
+    df2 v[3];
+    float none[2][3], om[2][2];
+    bool ok = fx_float_pair(E, Ed) && fx_float_pair(rho, rd) &&
+              rotated_eigen_mixed_try<true>(p, Ed, rd, none, om, v);
+    if (ok) {
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+            o.U[i][1] = fx_from_pair(v[i].hi.x, v[i].lo.x);
+            o.U[i][2] = fx_from_pair(v[i].hi.y, v[i].lo.y);
+        }
+        fx_third(o.U);
+        ok = fx_refine(p, E, fx_reciprocal(E, Ed), rho, o);
+    }
+    if (!ok) {
+        FxClass t;  // (its own storage: taking o's address would put it in local memory)
+        fx_solve_f64(p, E, rho, &t);
+        o = t;
     }
 }
+#endif
 
 // R = B^T A
 CP3_HD void fx_rotation(const fx B[3][3], const fx A[3][3], fx R[3][3]) {
@@ -524,42 +708,61 @@ CP3_HD void fx_rotation(const fx B[3][3], const fx A[3][3], fx R[3][3]) {
 
 // The electron and muon rows of W U: U_e (real), and c u_1 + s e^{i d} u_2 as three real and
 // three imaginary parts; w = {c23, s23, cos d, sin d}.
-CP3_HD void fx_rows(const double u0[3], const double u[2][3], const double* w, fx row[9]) {
-    const double* v[3] = {u0, u[0], u[1]};
+CP3_HD void fx_rows(const fx U[3][3], const double* w, fx row[9]) {
+    const fx c = fx_split(fx_from_double(w[0])), sr = fx_split(fx_from_double(w[1] * w[2])),
+             si = fx_split(fx_from_double(w[1] * w[3]));
 #pragma unroll
     for (int k = 0; k < 3; k++) {
-        row[k] = fx_split(fx_from_double(v[k][0]));
-        row[3 + k] = fx_split(fx_from_double(w[0] * v[k][1] + w[1] * w[2] * v[k][2]));
-        row[6 + k] = fx_split(fx_from_double(w[1] * w[3] * v[k][2]));
+        fxacc r, m;
+        fx_mac(r, c, U[1][k]);
+        fx_mac(r, sr, U[2][k]);
+        fx_mac(m, si, U[2][k]);
+        row[k] = U[0][k];
+        row[3 + k] = fx_res(r);
+        row[6 + k] = fx_res(m);
     }
 }
 
-// The coefficients of a bin that crosses no shell (the expansion of layer_coefficients64 in
-// cos D_jk itself): for e->e, mu->mu and the mean of e->mu and mu->e a constant and the factors
-// of cos D10, cos D20, cos D21; then twice the factor 2 J of the sines.
-CP3_HD void fx_vacuum(const double u[2][3], const double* w, fx v[13]) {
-    const double cc = w[0] * w[0], ss = w[1] * w[1], cs2 = 2.0 * w[0] * w[1];
-    double m[2][3];  // |U_ek|^2, |U_mu,k|^2
+// The coefficients of a single layer (a bin that crosses no shell, a beam) from its flavour
+// rows: the expansion of layer_coefficients64 in cos D_jk itself.  For e->e, mu->mu and the mean
+// of e->mu and mu->e a constant and the factors of cos D10, cos D20, cos D21; then 2 J of the
+// sines, doubled.
+CP3_HD void fx_coefficients(const fx row[9], fx v[13]) {
+    fx m[2][3];
+    long long mv[2][3];
 #pragma unroll
-    for (int k = 1; k < 3; k++) {
-        const double* x = u[k - 1];
-        m[0][k] = x[0] * x[0];
-        m[1][k] = cc * x[1] * x[1] + ss * x[2] * x[2] + cs2 * w[2] * x[1] * x[2];
+    for (int k = 0; k < 3; k++) {
+        fxacc a, b;
+        fx_mac(a, row[k], row[k]);
+        fx_mac(b, row[3 + k], row[3 + k]);
+        fx_mac(b, row[6 + k], row[6 + k]);
+        mv[0][k] = fx_sum(a);
+        mv[1][k] = fx_sum(b);
+        m[0][k] = fx_split(mv[0][k]);
+        m[1][k] = fx_split(mv[1][k]);
     }
-    m[0][0] = 1.0 - m[0][1] - m[0][2];
-    m[1][0] = 1.0 - m[1][1] - m[1][2];
-    auto put = [&](int q, double c0, double a, double b, double c) {
-        v[4 * q] = fx_split(fx_from_double(c0 - a - b - c));
-        v[4 * q + 1] = fx_split(fx_from_double(a));
-        v[4 * q + 2] = fx_split(fx_from_double(b));
-        v[4 * q + 3] = fx_split(fx_from_double(c));
+    auto mul = [](fx a, fx b) {
+        fxacc s;
+        fx_mac(s, a, b);
+        return fx_sum(s);
+    };
+    auto put = [&](int q, long long c0, long long a, long long b, long long c) {
+        v[4 * q] = fx_split(c0 - a - b - c);
+        v[4 * q + 1] = fx_split(a);
+        v[4 * q + 2] = fx_split(b);
+        v[4 * q + 3] = fx_split(c);
     };
 #pragma unroll
     for (int q = 0; q < 2; q++)
-        put(q, 1.0, 2.0 * m[q][0] * m[q][1], 2.0 * m[q][0] * m[q][2], 2.0 * m[q][1] * m[q][2]);
-    const double W0 = m[0][0] * m[1][0], W1 = m[0][1] * m[1][1], W2 = m[0][2] * m[1][2], S = W0 + W1 + W2;
-    put(2, 0.0, 2.0 * W2 - S, 2.0 * W1 - S, 2.0 * W0 - S);
-    v[12] = fx_split(fx_from_double(2.0 * cs2 * w[3] * (u[0][0] * u[1][0]) * (u[0][1] * u[1][2] - u[0][2] * u[1][1])));
+        put(q, 1LL << 62, 2 * mul(m[q][0], m[q][1]), 2 * mul(m[q][0], m[q][2]), 2 * mul(m[q][1], m[q][2]));
+    const long long W0 = mul(m[0][0], m[1][0]), W1 = mul(m[0][1], m[1][1]), W2 = mul(m[0][2], m[1][2]);
+    const long long S = W0 + W1 + W2;
+    put(2, 0, 2 * W2 - S, 2 * W1 - S, 2 * W0 - S);
+    // J = Im(w_2 conj(w_1)), w_k = U_mu,k U_ek: U_e1 U_e2 (im_2 re_1 - re_2 im_1)
+    fxacc j;
+    fx_mac(j, row[8], row[4]);
+    fx_mac(j, fx_neg(row[5]), row[7]);
+    v[12] = fx_split(4 * mul(fx_res(j), fx_split(mul(row[1], row[2]))));
 }
 
 }  // namespace cp3

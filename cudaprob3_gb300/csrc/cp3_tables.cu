@@ -1,11 +1,10 @@
-// cp3_tables.cu -- FP64 eigen work: the per-(density class, energy) tables of the
-// atmospheric kernels and the per-bin FP64 beam kernel.
+// cp3_tables.cu -- eigen work: the per-(density class, energy) tables of the atmospheric
+// kernels and the per-bin FP64 beam kernel.
 //
-// This translation unit is compiled with -fmad=false: its arithmetic is the reference's
-// (physics.hpp getMfast / get_product / getC / getA) in the reference's order, and keeping
+// This translation unit is compiled with -fmad=false: where two levels nearly meet, its FP64
+// arithmetic is the reference's (physics.hpp getMfast) in the reference's order, and keeping
 // multiply and add separately rounded reproduces the reference's x86 results to the last
-// bits where the eigen-system is ill-conditioned.  The table work is O(classes x energies),
-// amortised over every cosine, so the missing contraction costs nothing that matters.
+// bits where the eigen-system is ill-conditioned.
 #include <algorithm>
 
 #include "cp3_device.cuh"
@@ -44,7 +43,9 @@ __global__ void __launch_bounds__(kTableBlock)
 // The table of the fixed-point FP64 bins (cp3_fixed.cuh): for each class the rotation to the
 // next class's eigenbasis and the phase rates, and once per energy the flavour rows and the
 // vacuum coefficients.  A block is 32 energies by a run of kFxRun classes, one class a warp;
-// the extra warp solves the class after the run, for the last rotation.
+// the extra warp solves the class after the run, for the last rotation.  59 shells x 2000
+// energies take 24 us (130 with the FP64 formulas), PREM-4 x 400 energies 11 us (31): one wave,
+// its latency.
 constexpr int kFxRun = 8;
 
 __global__ void __launch_bounds__(32 * (kFxRun + 1))
@@ -57,25 +58,22 @@ __global__ void __launch_bounds__(32 * (kFxRun + 1))
     const bool on = c < ncls && ie < ne;
     FxClass k;
     if (on) {
-        double u[2][3], dmv[3], u0[3];
-        const double E = energies[ie];
-        rotated_layer_f64(&p, E, cls_rho[c], u, dmv);
-        fx_class(u, dmv, E, k, u0);
+        fx_solve(&p, energies[ie], cls_rho[c], k);
 #pragma unroll
         for (int f = 0; f < 9; f++) s_u[wv][f][lane] = make_int2(k.U[f / 3][f % 3].h, k.U[f / 3][f % 3].l);
         int2* ext = table + (size_t)ncls * kFxFields * ne_pad + ie;
-        if (c < 2 && wv < 2) {  // (class 1 is wv 1 of the first run only)
+        if (c < 2) {
             fx row[9];
-            fx_rows(u0, u, p.w, row);
+            fx_rows(k.U, p.w, row);
 #pragma unroll
             for (int f = 0; f < 9; f++)
                 ext[(size_t)((c == 0 ? kFxV0 : kFxV1) + f) * ne_pad] = make_int2(row[f].h, row[f].l);
-        }
-        if (c == 0) {
-            fx v[13];
-            fx_vacuum(u, p.w, v);
+            if (c == 0) {
+                fx v[13];
+                fx_coefficients(row, v);
 #pragma unroll
-            for (int f = 0; f < 13; f++) ext[(size_t)(kFxVac + f) * ne_pad] = make_int2(v[f].h, v[f].l);
+                for (int f = 0; f < 13; f++) ext[(size_t)(kFxVac + f) * ne_pad] = make_int2(v[f].h, v[f].l);
+            }
         }
     }
     __syncthreads();
@@ -114,24 +112,46 @@ __global__ void __launch_bounds__(kTableBlock)
     store_table_entry(table + ((size_t)c * ne_pad + ie) * kMixFields, u, om);
 }
 
-// physics::calculate_beam (physics.hpp:1153-1260), one thread per energy; result [9][ne].
-// The FP64 atmospheric kernels' algebra with one segment: the reference's matter masses
-// (getMfast, in this unit's uncontracted arithmetic), the rotated-basis unit eigenvectors,
-// the reference's phases -2.534 dmMatVac[k][0] L / E (getA, physics.hpp:547-551) as relative
-// phases, S = 1 + z1 u1 u1^T + z2 u2 u2^T and A = W S W^+.  The reference instead sums
-// e^{i arg_k} times its spectral products (get_product: 18 divisions) and rotates them with
-// AXFAC (getA); the two agree to rounding.
+// physics::calculate_beam (physics.hpp:1153-1260), one thread per energy; result [9][ne]: the
+// fixed-point layer of the energy (fx_solve) and the one-layer expansion of its probabilities.
+// 1e5 energies: 22.7 us (135 us in FP64 arithmetic, 582 FP64 instructions an energy).
+__device__ const TrigTable g_trig = make_trig_table();
+
+// A phase out of the fixed-point range: the FP64 formulas.
+__device__ __noinline__ void beam_out_of_range(const OscParams* p, double E, double rho_e, double L,
+                                               double* out, size_t plane) {
+    Layer64 f;
+    double dmv[3], arg[3];
+    rotated_layer_f64(p, E, rho_e, f.u, dmv);
+    layer64_phases(dmv, L, E, 1.0 / E, f, arg);
+    layer_store64(layer_coefficients64(f.u, p->w), f.z, out, plane);
+}
+
 __global__ void __launch_bounds__(kTableBlock)
     beam_f64_kernel(const __grid_constant__ OscParams p, const double* __restrict__ energies,
                     int ne, double rho_e, double L, double* __restrict__ out) {
+    __shared__ longlong2 s_trig[kTrigSize];
+    for (int i = threadIdx.x; i < kTrigSize; i += kTableBlock)
+        s_trig[i] = make_longlong2(g_trig.cs[i][0], g_trig.cs[i][1]);
+    __syncthreads();
     const int ie = blockIdx.x * kTableBlock + threadIdx.x;
     if (ie >= ne) return;
-    const double E = energies[ie];
-    Layer64 f;
-    double dmv[3], arg[3];
-    rotated_layer_f64(&p, E, rho_e, f.u, dmv);
-    layer64_phases(dmv, L, E, 1.0 / E, f, arg);
-    layer_store64(layer_coefficients64(f.u, p.w), f.z, out + ie, (size_t)ne);
+    FxClass k;
+    fx_solve(&p, energies[ie], rho_e, k);
+    unsigned int bad = 0;
+    cfx e[2];
+#pragma unroll
+    for (int q = 0; q < 2; q++) e[q] = fx_unit(fx_angle(k.rate[q], L, bad), s_trig);
+    if ((bad >> 20) != 0) {
+        beam_out_of_range(&p, energies[ie], rho_e, L, out + ie, (size_t)ne);
+        return;
+    }
+    fx row[9], v[13];
+    fx_rows(k.U, p.w, row);
+    fx_coefficients(row, v);
+    long long P[4];
+    fx_one_layer(v, e, P);
+    fx_store(P, out + ie, (size_t)ne);
 }
 
 }  // namespace

@@ -14,7 +14,7 @@ extern "C" void fixed_trig(long long* out) { std::memcpy(out, &kTable, sizeof kT
 
 extern "C" int fixed_atmos(const double* mix, int knutype, int anti, const double* cz, int nc,
                            const double* en, int ne, const double* radii, const double* rho,
-                           const double* ye, int n, double height_km, double* out) {
+                           const double* ye, int n, double height_km, int refine, double* out) {
     OscParams p;
     build_osc_params(MixingInput{mix[0], mix[1], mix[2], mix[3], knutype, mix[4], mix[5]}, anti, &p);
     EarthModel model;
@@ -30,16 +30,25 @@ extern "C" int fixed_atmos(const double* mix, int knutype, int anti, const doubl
     std::vector<FxClass> cls(ncls);
     for (int ie = 0; ie < ne; ie++) {
         for (int c = 0; c < ncls; c++) {
-            double u[2][3], dmv[3], u0[3];
-            rotated_layer_f64(&p, en[ie], c ? model.rho[c - 1] * model.ye[c - 1] : 0.0, u, dmv);
-            fx_class(u, dmv, en[ie], cls[c], u0);
-            fx v[13];
+            // the FP64 vectors stand for the device's double-float ones, rounded as those are
+            double u[2][3], dmv[3];
+            const double E = en[ie], rho_e = c ? model.rho[c - 1] * model.ye[c - 1] : 0.0;
+            rotated_layer_f64(&p, E, rho_e, u, dmv);
+            fx_class_f64(u, dmv, E, cls[c]);
+            if (refine) {
+                for (int i = 0; i < 3; i++)
+                    for (int k = 1; k < 3; k++)
+                        cls[c].U[i][k] = fx_split((fx_from_double(u[k - 1][i]) >> 16) * 65536);  // 2^-46
+                fx_third(cls[c].U);
+                if (!fx_refine(&p, E, 1.0 / E, rho_e, cls[c])) fx_class_f64(u, dmv, E, cls[c]);
+            }
+            fx v[13], row[9];
             if (c < 2) {
-                fx_rows(u0, u, p.w, v);
-                for (int f = 0; f < 9; f++) ext[(c ? kFxV1 : kFxV0) + f] = make_int2(v[f].h, v[f].l);
+                fx_rows(cls[c].U, p.w, row);
+                for (int f = 0; f < 9; f++) ext[(c ? kFxV1 : kFxV0) + f] = make_int2(row[f].h, row[f].l);
             }
             if (c == 0) {
-                fx_vacuum(u, p.w, v);
+                fx_coefficients(row, v);
                 for (int f = 0; f < 13; f++) ext[kFxVac + f] = make_int2(v[f].h, v[f].l);
             }
         }

@@ -32,13 +32,13 @@ def host(tmp_path_factory):
     return C.CDLL(so)
 
 
-def host_bins(lib, m, anti, cz, en, model, h):
+def host_bins(lib, m, anti, cz, en, model, h, refine=1):
     a = [np.ascontiguousarray(x, dtype=np.float64)
          for x in ([m.theta12, m.theta13, m.theta23, m.dcp, m.dm12sq, m.dm23sq], cz, en, *model)]
     p = [x.ctypes.data_as(dp) for x in a]
     out = np.empty((9, len(cz), len(en)))
     n = lib.fixed_atmos(p[0], -1 if anti else 1, int(anti), p[1], len(cz), p[2], len(en), p[3], p[4], p[5],
-                        len(a[3]), C.c_double(h), out.ctypes.data_as(dp))
+                        len(a[3]), C.c_double(h), refine, out.ctypes.data_as(dp))
     return np.transpose(out, (1, 2, 0)), n
 
 
@@ -58,16 +58,18 @@ def test_trig_table(host):
 @pytest.mark.parametrize("shells,h", [(1, 22.0), (2, 0.0), (3, 15.0), (12, 22.0), (59, 100.0), (128, 22.0)])
 def test_host_bins_against_oracle(host, oracle, shells, h):
     """Both orderings, nu and nubar, vacuum-only rows, vertical and shell-grazing rows, at the
-    FP64 parity bar; every bin inside the fixed-point range."""
+    FP64 parity bar; every bin inside the fixed-point range.  With the eigen-systems from the
+    FP64 formulas, and refined in fixed point from vectors cut at 2^-46."""
     model = earth.synthetic_shells(shells)
     cz = np.concatenate([np.linspace(-1, 1, 23), [-1e-9, -0.5]])
     en = np.logspace(-1, 3, 17)
     for m in earth.gaussian_sets(4, seed=7)[1:3]:
         for anti in (False, True):
-            got, outside = host_bins(host, m, anti, cz, en, model, h)
-            assert outside == 0
             ref = oracle.atmos(omix(m, anti), anti, cz, en, *model, h, layer_limit=128)
-            assert np.abs(got - ref).max() <= 1e-12
+            for refine in (0, 1):
+                got, outside = host_bins(host, m, anti, cz, en, model, h, refine)
+                assert outside == 0
+                assert np.abs(got - ref).max() <= 1e-12
 
 
 def test_out_of_range_bins_ask_for_the_fp64_path(host):
