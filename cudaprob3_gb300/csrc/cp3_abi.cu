@@ -78,13 +78,12 @@ struct cp3_propagator {
     DevBuf<float2> d_energies_df, d_cls_rho_df;  // mixed kernels: (hi, lo) pairs split here
     DevBuf<int> d_seg_off;
     DevBuf<double> d_seg_len, d_cls_rho, d_seg_rho;
-    DevBuf<double> d_ph_prob, d_ph_shift, d_air_cm;  // production-height averaging (FP64)
-    DevBuf<float> d_ph_prob_f, d_ph_hw;              // ... and its float form (mixed)
+    DevBuf<double> d_ph_prob, d_ph_mid, d_ph_wid;  // production-height averaging (FP64)
+    DevBuf<float> d_ph_prob_f, d_ph_hw;            // ... and its float form (mixed)
     DevBuf<float2> d_ph_hm;
     bool avg_dirty = true;
     DevBuf<float2> d_seg_len_df;
-    DevBuf<double> d_table64;   // FP64 with production-height averaging
-    DevBuf<int2> d_table_fx;    // FP64 without
+    DevBuf<int2> d_table_fx;
     DevBuf<double> d_plane;  // getProbabilityArr: one channel, transposed on the device
     DevBuf<float> d_table32;
     DevBuf<char> d_result;
@@ -288,6 +287,11 @@ int prepare_atmos(cp3_propagator* h) {
         CP3_CUDA(h, h->d_seg_rho.reserve(nseg), "allocate trajectories");
         CP3_CUDA(h, cudaMemcpy(h->d_seg_rho.ptr, t.rho_e.data(), sizeof(double) * nseg,
                                cudaMemcpyHostToDevice), "upload trajectories");
+        if (h->precision == CP3_FP64) {  // the air's class, for its table
+            const double air = 0.0;
+            CP3_CUDA(h, h->d_cls_rho.reserve(1), "allocate classes");
+            CP3_CUDA(h, cudaMemcpy(h->d_cls_rho.ptr, &air, sizeof air, cudaMemcpyHostToDevice), "upload classes");
+        }
         h->traj_dirty = false;
         return CP3_OK;
     }
@@ -311,68 +315,66 @@ int prepare_atmos(cp3_propagator* h) {
     return CP3_OK;
 }
 
-// Averaging inputs: the client's probabilities and, per cosine, the path-length shifts at the
-// bin edges and the air segment in cm (the reference's `dist` of layer 0).
+// Averaging inputs: the client's probabilities [2][3][ne][nc][bins], transposed on the device so
+// that consecutive energies are contiguous (the kernels' warps run over energies), and per
+// (cosine, bin) the mid path-length shift and the width in km; zero where the air segment is
+// zero, as the reference's d0 = 0 there (physics.hpp:1030-1034).
 int prepare_averaging(cp3_propagator* h, AvgArrays* av, AvgMixed* avm) {
     if (h->avg_bins == 0) return CP3_OK;
-    if (h->avg_dirty)
+    const bool mixed = h->precision == CP3_MIXED;
+    const int nb = h->avg_bins;
+    if (h->avg_dirty) {
         if (int rc = wait_last_compute(h)) return rc;
-    if (h->avg_dirty && h->precision == CP3_MIXED) {
-        // float probabilities; per (cosine, bin) the mid shift as a float pair and the width,
-        // both in km (the phase rates are per km); zero where the air segment is zero, as the
-        // reference's d0 = 0 there (physics.hpp:1030-1034)
         std::vector<double> shifts;
-        production_height_shifts(h->cosines.data(), h->nc, h->height_cm, h->avg_edges.data(),
-                                  h->avg_bins, &shifts);
-        const int nb = h->avg_bins;
-        std::vector<float> prob(h->avg_prob.begin(), h->avg_prob.end()), hw((size_t)h->nc * nb);
-        std::vector<float2> hm((size_t)h->nc * nb);
+        production_height_shifts(h->cosines.data(), h->nc, h->height_cm, h->avg_edges.data(), nb, &shifts);
+        const size_t cells = (size_t)h->nc * nb;
+        std::vector<double> mid(cells), wid(cells);
         for (int ic = 0; ic < h->nc; ic++)
             for (int b = 0; b < nb; b++) {
                 const double h0 = shifts[(size_t)ic * (nb + 1) + b], h1 = shifts[(size_t)ic * (nb + 1) + b + 1];
                 const bool zero = h->traj.air_cm[ic] == 0.0;
-                const double mid_km = zero ? 0.0 : 0.5 * (h1 + h0) / kKm2Cm;
-                const float mh = (float)mid_km;
-                hm[(size_t)ic * nb + b] = make_float2(mh, (float)(mid_km - (double)mh));
-                hw[(size_t)ic * nb + b] = zero ? 0.0f : (float)((h1 - h0) / kKm2Cm);
+                mid[(size_t)ic * nb + b] = zero ? 0.0 : 0.5 * (h1 + h0) / kKm2Cm;
+                wid[(size_t)ic * nb + b] = zero ? 0.0 : (h1 - h0) / kKm2Cm;
             }
-        CP3_CUDA(h, h->d_ph_prob_f.reserve(prob.size()), "allocate averaging");
-        CP3_CUDA(h, h->d_ph_hm.reserve(hm.size()), "allocate averaging");
-        CP3_CUDA(h, h->d_ph_hw.reserve(hw.size()), "allocate averaging");
-        CP3_CUDA(h, cudaMemcpy(h->d_ph_prob_f.ptr, prob.data(), sizeof(float) * prob.size(),
-                               cudaMemcpyHostToDevice), "upload averaging");
-        CP3_CUDA(h, cudaMemcpy(h->d_ph_hm.ptr, hm.data(), sizeof(float2) * hm.size(),
-                               cudaMemcpyHostToDevice), "upload averaging");
-        CP3_CUDA(h, cudaMemcpy(h->d_ph_hw.ptr, hw.data(), sizeof(float) * hw.size(),
-                               cudaMemcpyHostToDevice), "upload averaging");
+        if (mixed) {
+            const std::vector<float2> hm = split_pairs(mid.data(), cells);
+            const std::vector<float> hw(wid.begin(), wid.end());
+            CP3_CUDA(h, h->d_ph_hm.reserve(cells), "allocate averaging");
+            CP3_CUDA(h, h->d_ph_hw.reserve(cells), "allocate averaging");
+            CP3_CUDA(h, cudaMemcpy(h->d_ph_hm.ptr, hm.data(), sizeof(float2) * cells, cudaMemcpyHostToDevice), "upload averaging");
+            CP3_CUDA(h, cudaMemcpy(h->d_ph_hw.ptr, hw.data(), sizeof(float) * cells, cudaMemcpyHostToDevice), "upload averaging");
+            CP3_CUDA(h, h->d_ph_prob_f.reserve(h->avg_prob.size()), "allocate averaging");
+        } else {
+            CP3_CUDA(h, h->d_ph_mid.reserve(cells), "allocate averaging");
+            CP3_CUDA(h, h->d_ph_wid.reserve(cells), "allocate averaging");
+            CP3_CUDA(h, cudaMemcpy(h->d_ph_mid.ptr, mid.data(), sizeof(double) * cells, cudaMemcpyHostToDevice), "upload averaging");
+            CP3_CUDA(h, cudaMemcpy(h->d_ph_wid.ptr, wid.data(), sizeof(double) * cells, cudaMemcpyHostToDevice), "upload averaging");
+            CP3_CUDA(h, h->d_ph_prob.reserve(h->avg_prob.size()), "allocate averaging");
+        }
+        // one (type, flavour) slab [ne][nc bins] at a time, through a buffer freed at the end
+        DevBuf<double> raw;
+        const size_t slab = cells * h->ne;
+        CP3_CUDA(h, raw.reserve(slab), "allocate averaging");
+        for (int k = 0; k < 6; k++) {
+            CP3_CUDA(h, cudaMemcpyAsync(raw.ptr, h->avg_prob.data() + k * slab, sizeof(double) * slab,
+                                        cudaMemcpyHostToDevice, h->stream), "upload averaging");
+            void* dst = mixed ? (void*)(h->d_ph_prob_f.ptr + k * slab) : (void*)(h->d_ph_prob.ptr + k * slab);
+            CP3_CUDA(h, launch_weights_transpose(raw.ptr, h->ne, (long long)cells, dst, mixed, h->stream), "transpose averaging");
+        }
+        CP3_CUDA(h, cudaStreamSynchronize(h->stream), "upload averaging");
         h->avg_dirty = false;
     }
-    if (h->precision == CP3_MIXED) {
+    if (mixed) {
         avm->prob = h->d_ph_prob_f.ptr;
         avm->hm = h->d_ph_hm.ptr;
         avm->hw = h->d_ph_hw.ptr;
-        avm->nb = h->avg_bins;
+        avm->nb = nb;
         return CP3_OK;
     }
-    if (h->avg_dirty) {
-        std::vector<double> shifts;
-        production_height_shifts(h->cosines.data(), h->nc, h->height_cm, h->avg_edges.data(),
-                                 h->avg_bins, &shifts);
-        CP3_CUDA(h, h->d_ph_prob.reserve(h->avg_prob.size()), "allocate averaging");
-        CP3_CUDA(h, h->d_ph_shift.reserve(shifts.size()), "allocate averaging");
-        CP3_CUDA(h, h->d_air_cm.reserve(h->nc), "allocate averaging");
-        CP3_CUDA(h, cudaMemcpy(h->d_ph_prob.ptr, h->avg_prob.data(), sizeof(double) * h->avg_prob.size(),
-                               cudaMemcpyHostToDevice), "upload averaging");
-        CP3_CUDA(h, cudaMemcpy(h->d_ph_shift.ptr, shifts.data(), sizeof(double) * shifts.size(),
-                               cudaMemcpyHostToDevice), "upload averaging");
-        CP3_CUDA(h, cudaMemcpy(h->d_air_cm.ptr, h->traj.air_cm.data(), sizeof(double) * h->nc,
-                               cudaMemcpyHostToDevice), "upload averaging");
-        h->avg_dirty = false;
-    }
     av->prob = h->d_ph_prob.ptr;
-    av->shift = h->d_ph_shift.ptr;
-    av->air_cm = h->d_air_cm.ptr;
-    av->n_bins = h->avg_bins;
+    av->mid = h->d_ph_mid.ptr;
+    av->wid = h->d_ph_wid.ptr;
+    av->n_bins = nb;
     return CP3_OK;
 }
 
@@ -420,37 +422,29 @@ int launch(cp3_propagator* h, int type, cudaStream_t s, void* host_dst = nullptr
         rc = prepare_averaging(h, &av, &avm);
         if (rc) return rc;
         const bool mixed = h->precision == CP3_MIXED;
-        // FP64 with constant densities: the averaging reads the FP64 table, everything else
-        // the fixed-point one
+        // FP64: constant densities come from the fixed-point table; quadratic densities and the
+        // averaging solve their layers in place and read only the air's class
         const bool fx = !mixed && !h->model.poly && av.n_bins == 0;
-        if (fx)
-            CP3_CUDA(h, h->d_table_fx.reserve(table_fx_words(h->ncls_used, h->ne)), "allocate eigen table");
-        else if (!mixed && !h->model.poly)
-            CP3_CUDA(h, h->d_table64.reserve((size_t)h->ncls_used * pad_energies(h->ne) * kF64Fields),
-                     "allocate eigen table");
+        const int fx_classes = fx ? h->ncls_used : 1;
+        if (!mixed)
+            CP3_CUDA(h, h->d_table_fx.reserve(table_fx_words(fx_classes, h->ne)), "allocate eigen table");
         mark(0);
-        if (!h->model.poly) {
-            if (fx)
-                e = launch_table_fx(p, h->d_energies.ptr, h->ne, h->d_cls_rho.ptr, h->ncls_used,
-                                    h->d_table_fx.ptr, s);
-            else if (mixed)
-                e = launch_table_mixed(p, h->d_energies_df.ptr, h->ne, h->d_cls_rho_df.ptr,
-                                       h->ncls_used, h->d_table32.ptr, s);
-            else
-                e = launch_table_f64(p, h->d_energies.ptr, h->ne, h->d_cls_rho.ptr, h->ncls_used,
-                                     h->d_table64.ptr, s);
-        }
+        if (!mixed)
+            e = launch_table_fx(p, h->d_energies.ptr, h->ne, h->d_cls_rho.ptr, fx_classes,
+                                h->d_table_fx.ptr, s);
+        else if (!h->model.poly)
+            e = launch_table_mixed(p, h->d_energies_df.ptr, h->ne, h->d_cls_rho_df.ptr,
+                                   h->ncls_used, h->d_table32.ptr, s);
         mark(1);
         auto bins = [&](RowRange rr) {
             if (h->model.poly && mixed && avm.nb > 0)
                 return launch_atmos_mixed_inline_avg(p, h->d_energies.ptr, h->ne, h->d_seg_off.ptr,
                                                      h->d_seg_len_df.ptr, h->d_seg_rho.ptr, h->nc,
                                                      avm, (float*)h->d_result.ptr, s, rr);
-            if (h->model.poly)
-                return launch_atmos_inline(p, mixed, h->d_energies.ptr, h->ne, h->d_seg_off.ptr,
-                                           mixed ? (const void*)h->d_seg_len_df.ptr
-                                                 : (const void*)h->d_seg_len.ptr,
-                                           h->d_seg_rho.ptr, h->nc, av, h->d_result.ptr, s, rr);
+            if (h->model.poly && mixed)
+                return launch_atmos_mixed_inline(p, h->d_energies.ptr, h->ne, h->d_seg_off.ptr,
+                                                 h->d_seg_len_df.ptr, h->d_seg_rho.ptr, h->nc,
+                                                 (float*)h->d_result.ptr, s, rr);
             if (mixed && avm.nb > 0)
                 return launch_atmos_mixed_avg(p, h->d_table32.ptr, h->ne, h->d_seg_off.ptr,
                                               h->d_seg_len_df.ptr, h->nc, avm,
@@ -463,9 +457,10 @@ int launch(cp3_propagator* h, int type, cudaStream_t s, void* host_dst = nullptr
                 return launch_atmos_fx(p, h->d_energies.ptr, h->ne, h->d_table_fx.ptr,
                                        h->d_cls_rho.ptr, h->ncls_used, h->d_seg_off.ptr,
                                        h->d_seg_len.ptr, h->nc, (double*)h->d_result.ptr, s, rr);
-            return launch_atmos_f64(p, h->d_energies.ptr, h->ne, h->d_table64.ptr,
-                                    h->d_seg_off.ptr, h->d_seg_len.ptr, h->nc,
-                                    av, (double*)h->d_result.ptr, s, rr);
+            return launch_atmos_fx_inline(p, h->d_energies.ptr, h->ne, h->d_table_fx.ptr,
+                                          h->d_seg_off.ptr, h->d_seg_len.ptr,
+                                          h->model.poly ? h->d_seg_rho.ptr : h->d_cls_rho.ptr,
+                                          !h->model.poly, h->nc, av, (double*)h->d_result.ptr, s, rr);
         };
         if (!host_dst) {
             if (e == cudaSuccess) e = bins(RowRange{});

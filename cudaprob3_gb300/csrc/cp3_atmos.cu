@@ -37,23 +37,6 @@ constexpr int kMaxGridY = 65535;
 // complex 3x3 products.  The phases are formed exactly as the reference forms them, so
 // their roundings -- which matter over ~120 layers of up to ~800 rad -- are the reference's.
 
-// Table entry (10 doubles, five 16-byte words): u1, u2, dmMatVac[0..2][0], 1 unused.
-__device__ __forceinline__ void layer64_from_table(const double* __restrict__ t, double L,
-                                                   double E, double rE, Layer64& f,
-                                                   double arg[3]) {
-    const double2* t2 = reinterpret_cast<const double2*>(t);
-    const double2 a = __ldg(t2), b = __ldg(t2 + 1), c = __ldg(t2 + 2), d = __ldg(t2 + 3),
-                  e = __ldg(t2 + 4);
-    f.u[0][0] = a.x;
-    f.u[0][1] = a.y;
-    f.u[0][2] = b.x;
-    f.u[1][0] = b.y;
-    f.u[1][1] = c.x;
-    f.u[1][2] = c.y;
-    const double dmv[3] = {d.x, d.y, e.x};
-    layer64_phases(dmv, L, E, rE, f, arg);
-}
-
 // G <- S G
 __device__ __forceinline__ void apply_left64(const Layer64& f, cm3& G) {
 #pragma unroll
@@ -102,9 +85,9 @@ struct WParams64 {
 };
 
 struct AvgInput {
-    const double* prob;    // [2][3][ne][nc][nb]
-    const double* shift;   // [nc][nb + 1] path-length shifts at the bin edges, cm
-    const double* air_cm;  // [nc] segment 0 length, cm
+    const double* prob;  // [2][3][nc][nb][ne]
+    const double* mid;   // [nc][nb] mid path-length shift of a height bin, km (0 without an air segment)
+    const double* wid;   // [nc][nb] its width, km (0 likewise)
     int nb, type;
 };
 
@@ -116,8 +99,7 @@ __device__ __forceinline__ double sinc_reference(double x) {
 }
 
 __device__ __forceinline__ void avg_shift_factors(const AvgInput& av, int ic, int nc, int ie, int ne,
-                                                  const double arg0[3], cd sf[3][3]) {
-    const double dist = av.air_cm[ic];
+                                                  double dist, const double arg0[3], cd sf[3][3]) {
     double d0[3];
 #pragma unroll
     for (int k = 0; k < 3; k++) d0[k] = dist == 0. ? 0. : arg0[k] / dist;
@@ -126,10 +108,8 @@ __device__ __forceinline__ void avg_shift_factors(const AvgInput& av, int ic, in
 #pragma unroll
         for (int f = 0; f < 3; f++) sf[q][f] = cd{0.0, 0.0};
     const int pa[3] = {1, 2, 2}, pb[3] = {0, 0, 1};
-    const double* sh = av.shift + (size_t)ic * (av.nb + 1);
     for (int p = 0; p < av.nb; p++) {
-        const double h0 = sh[p], h1 = sh[p + 1];
-        const double hm = (h1 + h0) / 2., hw = (h1 - h0);
+        const double hm = av.mid[(size_t)ic * av.nb + p], hw = av.wid[(size_t)ic * av.nb + p];
 #pragma unroll
         for (int q = 0; q < 3; q++) {
             const double d = d0[pa[q]] - d0[pb[q]];
@@ -138,7 +118,7 @@ __device__ __forceinline__ void avg_shift_factors(const AvgInput& av, int ic, in
             const double fim = sinc_reference(sarg) * sin(d * hm);
 #pragma unroll
             for (int f = 0; f < 3; f++) {
-                const size_t idx = (((size_t)(av.type * 3 + f) * ne + ie) * nc + ic) * av.nb + p;
+                const size_t idx = (((size_t)(av.type * 3 + f) * nc + ic) * av.nb + p) * ne + ie;
                 const double w = av.prob[idx];
                 sf[q][f].re += w * fre;
                 sf[q][f].im += w * fim;
@@ -199,7 +179,7 @@ __device__ __noinline__ void finish_averaged64(const cm3& G, const Layer64& F0, 
 
 // One FP64 bin over M+1 layers; seg(l, F, arg) fills layer l (0 = air) and its phases.
 template <class SegFn>
-__device__ __forceinline__ void atmos_bin_f64(SegFn seg, int M, const double* w,
+__device__ __forceinline__ void atmos_bin_f64(SegFn seg, int M, const double* w, double air_km,
                                               const AvgInput& av, int ic, int nc, int ie, int ne,
                                               double* __restrict__ out, size_t plane) {
     cm3 G;
@@ -246,7 +226,7 @@ __device__ __forceinline__ void atmos_bin_f64(SegFn seg, int M, const double* w,
     }
     if (av.nb > 0) {
         cd sf[3][3];
-        avg_shift_factors(av, ic, nc, ie, ne, arg, sf);
+        avg_shift_factors(av, ic, nc, ie, ne, air_km, arg, sf);
         finish_averaged64(G, F, w, sf, out, plane);
         return;
     }
@@ -258,58 +238,6 @@ __device__ __forceinline__ void atmos_bin_f64(SegFn seg, int M, const double* w,
 #pragma unroll
         for (int j = 0; j < 3; j++)
             out[(size_t)(j * 3 + i) * plane] = A.a[i][j].re * A.a[i][j].re + A.a[i][j].im * A.a[i][j].im;
-}
-
-// FP64 atmospheric bins, quadratic density: every segment carries its own density, so its
-// eigen-system is solved per segment (the reference's getMfast, then the rotated projectors).
-__global__ void __launch_bounds__(kBlock)
-    atmos_f64_inline_kernel(const __grid_constant__ OscParams p, const double* __restrict__ energies,
-                            int ne, const int* __restrict__ seg_off,
-                            const double* __restrict__ seg_len, const double* __restrict__ seg_rho,
-                            int ic0, int nc, AvgInput av, double* __restrict__ out) {
-    __shared__ double s_len[kMaxSegments];
-    __shared__ double s_rho[kMaxSegments];
-    const int ic = ic0 + blockIdx.y;
-    const int s0 = seg_off[ic];
-    const int nseg = seg_off[ic + 1] - s0;
-    for (int i = threadIdx.x; i < nseg; i += kBlock) {
-        s_len[i] = seg_len[s0 + i];
-        s_rho[i] = seg_rho[s0 + i];
-    }
-    __syncthreads();
-    const int ie = blockIdx.x * kBlock + threadIdx.x;
-    if (ie >= ne) return;
-    const double E = energies[ie], rE = 1.0 / E;
-    atmos_bin_f64(
-        [&](int l, Layer64& F, double arg[3]) {
-            double dmv[3];
-            rotated_layer_f64(&p, E, s_rho[l], F.u, dmv);
-            layer64_phases(dmv, s_len[l], E, rE, F, arg);
-        },
-        nseg - 1, p.w, av, ic, nc, ie, ne, out + (size_t)ic * ne + ie, (size_t)nc * ne);
-}
-
-__global__ void __launch_bounds__(kBlock)
-    atmos_f64_kernel(const double* __restrict__ energies, int ne, int ne_pad,
-                     const double* __restrict__ table, const int* __restrict__ seg_off,
-                     const double* __restrict__ seg_len, int ic0, int nc,
-                     const __grid_constant__ WParams64 w, AvgInput av, double* __restrict__ out) {
-    __shared__ double s_len[kMaxSegments];
-    const int ic = ic0 + blockIdx.y;
-    const int s0 = seg_off[ic];
-    const int nseg = seg_off[ic + 1] - s0;
-    for (int i = threadIdx.x; i < nseg; i += kBlock) s_len[i] = seg_len[s0 + i];
-    __syncthreads();
-    const int ie = blockIdx.x * kBlock + threadIdx.x;
-    if (ie >= ne) return;
-    const double E = energies[ie], rE = 1.0 / E;
-    const size_t cls_stride = (size_t)kF64Fields * ne_pad;
-    const double* tab = table + (size_t)ie * kF64Fields;
-    atmos_bin_f64(
-        [&](int l, Layer64& F, double arg[3]) {
-            layer64_from_table(tab + l * cls_stride, s_len[l], E, rE, F, arg);  // class l
-        },
-        nseg - 1, w.w, av, ic, nc, ie, ne, out + (size_t)ic * ne + ie, (size_t)nc * ne);
 }
 
 // FP64 bins in fixed point (cp3_fixed.cuh).  One warp is one cosine row x 32 energies; a block's
@@ -324,16 +252,16 @@ __device__ const TrigTable g_trig = make_trig_table();
 // A bin out of the fixed-point range (a phase beyond 2^42 turns, or one that is not finite): the
 // FP64 layers solved in place.
 __device__ __noinline__ void atmos_bin_out_of_range(const OscParams* p, double E, const double* len,
-                                                    const double* cls_rho, int M, double* out,
-                                                    size_t plane) {
+                                                    const double* rho, int M, const AvgInput& av,
+                                                    int ic, int nc, int ie, int ne, double* out) {
     const double rE = 1.0 / E;
     atmos_bin_f64(
         [&](int l, Layer64& F, double arg[3]) {
             double dmv[3];
-            rotated_layer_f64(p, E, cls_rho[l], F.u, dmv);
+            rotated_layer_f64(p, E, rho[l], F.u, dmv);
             layer64_phases(dmv, len[l], E, rE, F, arg);
         },
-        M, p->w, AvgInput{}, 0, 0, 0, 0, out, plane);
+        M, p->w, len[0], av, ic, nc, ie, ne, out, (size_t)nc * ne);
 }
 
 __global__ void __launch_bounds__(32 * kFxWarps, 4)
@@ -364,7 +292,147 @@ __global__ void __launch_bounds__(32 * kFxWarps, 4)
     if (fx_bin(col, s_len[wv], nseg - 1, s_trig, P))
         fx_store(P, o, plane);
     else
-        atmos_bin_out_of_range(&p, energies[ie], s_len[wv], cls_rho, nseg - 1, o, plane);
+        atmos_bin_out_of_range(&p, energies[ie], s_len[wv], cls_rho, nseg - 1, AvgInput{}, ic, nc, ie, ne, o);
+}
+
+// FP64 bins in fixed point whose layers are solved in place, the air layer from a table of one
+// class.  (Solved by a block's first warp instead, its latency held the other three up: 96 us
+// instead of 73 + 8 for the grid below.)
+
+__device__ __forceinline__ FxAir load_air(const int2* table, int ne_pad, int ie, bool coef) {
+    const FxColumn col{table + ie, table + (size_t)kFxFields * ne_pad + ie, (size_t)ne_pad, 0};
+    FxAir air;
+#pragma unroll
+    for (int f = 0; f < 9; f++) {
+        air.U[f / 3][f % 3] = col.extra(kFxV1 + f);
+        air.row[f] = col.extra(kFxV0 + f);
+    }
+    if (coef)
+#pragma unroll
+        for (int f = 0; f < 13; f++) air.coef[f] = col.extra(kFxVac + f);
+    air.rate[0] = col.rate(0, 0);
+    air.rate[1] = col.rate(0, 1);
+    return air;
+}
+
+// Quadratic densities: an eigen-system for every segment of every bin.  Blocks as above.  PREM's
+// quadratic model, 500 x 500: 73 us (481 in FP64 arithmetic).
+__global__ void __launch_bounds__(32 * kFxWarps, 3)
+    atmos_fx_inline_kernel(const __grid_constant__ OscParams p, const double* __restrict__ energies,
+                           int ne, int ne_pad, const int2* __restrict__ table, const int* __restrict__ seg_off,
+                           const double* __restrict__ seg_len, const double* __restrict__ seg_rho, int ic0,
+                           int ic1, int nc, double* __restrict__ out) {
+    __shared__ longlong2 s_trig[kTrigSize];
+    __shared__ double s_len[kFxWarps][kMaxSegments], s_rho[kFxWarps][kMaxSegments];
+    for (int i = threadIdx.x; i < kTrigSize; i += 32 * kFxWarps)
+        s_trig[i] = make_longlong2(g_trig.cs[i][0], g_trig.cs[i][1]);
+    const int lane = threadIdx.x & 31, wv = threadIdx.x >> 5;
+    const int ic = ic0 + blockIdx.y * kFxWarps + wv, ie = blockIdx.x * 32 + lane;
+    int nseg = 0;
+    if (ic < ic1) {
+        const int s0 = seg_off[ic];
+        nseg = seg_off[ic + 1] - s0;
+        for (int i = lane; i < nseg; i += 32) {
+            s_len[wv][i] = seg_len[s0 + i];
+            s_rho[wv][i] = seg_rho[s0 + i];
+        }
+    }
+    __syncthreads();
+    if (ic >= ic1 || ie >= ne) return;
+    const double E = energies[ie];
+    const FxAir air = load_air(table, ne_pad, ie, nseg == 1);
+    double* o = out + (size_t)ic * ne + ie;
+    auto solve = [&](int l, FxClass& k) { fx_solve(&p, E, s_rho[wv][l], k); };
+    long long P[4];
+    if (fx_bin_inline(solve, air, fx_w(p.w), s_len[wv], nseg - 1, s_trig, P))
+        fx_store(P, o, (size_t)nc * ne);
+    else
+        atmos_bin_out_of_range(&p, E, s_len[wv], s_rho[wv], nseg - 1, AvgInput{}, ic, nc, ie, ne, o);
+}
+
+// Production-height averaging (rho per segment or, per_class, per class).  A block is one row x
+// 32 energies: its first warp runs the chain of layers while the others sum the shift factors of
+// the height bins, a third each (on a row that crosses no shell all four take a quarter) -- the
+// two are independent, and a grid of a few hundred rows and energies leaves the chip half empty
+// with one warp a bin.  PREM-4, 200 x 150, 20 heights:
+// 70 us (688 in FP64 arithmetic with the weights read across energies; 96 with one warp a bin).
+__global__ void __launch_bounds__(32 * kFxWarps, 4)
+    atmos_fx_avg_kernel(const __grid_constant__ OscParams p, const double* __restrict__ energies, int ne,
+                        int ne_pad, const int2* __restrict__ table, const int* __restrict__ seg_off,
+                        const double* __restrict__ seg_len, const double* __restrict__ rho, bool per_class,
+                        int ic0, int nc, AvgInput av, double* __restrict__ out) {
+    __shared__ longlong2 s_trig[kTrigSize];
+    __shared__ double s_len[kMaxSegments], s_rho[kMaxSegments];
+    __shared__ long long s_sum[kFxWarps][21][32];
+    __shared__ unsigned int s_bad[kFxWarps][32];
+    for (int i = threadIdx.x; i < kTrigSize; i += 32 * kFxWarps)
+        s_trig[i] = make_longlong2(g_trig.cs[i][0], g_trig.cs[i][1]);
+    const int lane = threadIdx.x & 31, wv = threadIdx.x >> 5;
+    const int ic = ic0 + blockIdx.y, ie = blockIdx.x * 32 + lane;
+    const int s0 = seg_off[ic], nseg = seg_off[ic + 1] - s0;
+    for (int i = threadIdx.x; i < nseg; i += 32 * kFxWarps) {
+        s_len[i] = seg_len[s0 + i];
+        s_rho[i] = rho[per_class ? i : s0 + i];
+    }
+    __syncthreads();
+    const bool on = ie < ne;
+    unsigned int bad = 0;
+    const int first = nseg > 1 ? 1 : 0;  // of the warps that sum
+    if (wv >= first && on) {
+        const FxColumn col{table + ie, nullptr, (size_t)ne_pad, 0};
+        const double rate[2] = {col.rate(0, 0), col.rate(0, 1)};
+        const size_t cell = (size_t)ic * av.nb;
+        FxShift sum;
+        fx_shift_sums(rate, wv - first, kFxWarps - first, av.nb, av.prob + ((size_t)av.type * 3 * nc * av.nb + cell) * ne + ie,
+                      (size_t)nc * av.nb * ne, (size_t)ne, av.mid + cell, av.wid + cell, s_trig, bad, sum);
+#pragma unroll
+        for (int f = 0; f < 3; f++) {
+            s_sum[wv][18 + f][lane] = (long long)sum.total[f];
+#pragma unroll
+            for (int q = 0; q < 6; q++) s_sum[wv][6 * f + q][lane] = sum.value(q >> 1, f, q & 1);
+        }
+        s_bad[wv][lane] = bad;
+    }
+    double E = 0.0;
+    cfx a[2][3];
+    if (wv == 0 && on) {
+        E = energies[ie];
+        const FxAir air = load_air(table, ne_pad, ie, false);
+        auto solve = [&](int l, FxClass& k) { fx_solve(&p, E, s_rho[l], k); };
+        fx_air_rows(solve, air, fx_w(p.w), s_len, nseg - 1, s_trig, bad, a);
+    }
+    __syncthreads();
+    if (wv > 0 || !on) return;
+    long long sum[3][3][2] = {};
+    unsigned long long total[3] = {};
+#pragma unroll
+    for (int k = 0; k < kFxWarps; k++) {
+        if (k < first) continue;
+        bad |= s_bad[k][lane];
+#pragma unroll
+        for (int f = 0; f < 3; f++) {
+            total[f] += (unsigned long long)s_sum[k][18 + f][lane];
+#pragma unroll
+            for (int q = 0; q < 6; q++) sum[q >> 1][f][q & 1] += s_sum[k][6 * f + q][lane];
+        }
+    }
+    cfx t[3][3];
+    fx_shift_factors(sum, total, bad, t);
+    const FxAir air = load_air(table, ne_pad, ie, false);
+    long long P[3][2];
+    fx_average(a, air, fx_w(p.w), s_len[0], s_trig, t, bad, P);
+    double* o = out + (size_t)ic * ne + ie;
+    const size_t plane = (size_t)nc * ne;
+    if ((bad >> 20) == 0) {
+#pragma unroll
+        for (int j = 0; j < 3; j++) {
+            o[(size_t)(3 * j) * plane] = fx_to_double(P[j][0]);
+            o[(size_t)(3 * j + 1) * plane] = fx_to_double(P[j][1]);
+            o[(size_t)(3 * j + 2) * plane] = fx_to_double((1LL << 62) - P[j][0] - P[j][1]);
+        }
+    } else {
+        atmos_bin_out_of_range(&p, E, s_len, s_rho, nseg - 1, av, ic, nc, ie, ne, o);
+    }
 }
 
 // Mixed atmospheric bins (the physics of calculate_atmos rearranged for FP32: see
@@ -422,20 +490,24 @@ __global__ void __launch_bounds__(kBlock)
 
 }  // namespace
 
-cudaError_t launch_atmos_f64(const OscParams& p, const double* energies, int ne,
-                             const double* table, const int* seg_off, const double* seg_len,
-                             int n_cosines, const AvgArrays& avg, double* out,
-                             cudaStream_t s, RowRange rr) {
+cudaError_t launch_atmos_fx_inline(const OscParams& p, const double* energies, int ne,
+                                   const int2* table, const int* seg_off, const double* seg_len, const double* rho,
+                                   bool per_class, int n_cosines, const AvgArrays& avg, double* out,
+                                   cudaStream_t s, RowRange rr) {
     if (ne <= 0 || n_cosines <= 0) return cudaSuccess;
-    const int ne_pad = pad_energies(ne);
-    const AvgInput av{avg.prob, avg.shift, avg.air_cm, avg.n_bins, p.anti};
-    const WParams64 w{{p.w[0], p.w[1], p.w[2], p.w[3]}};
-    const int end = rr.end < 0 ? n_cosines : rr.end;
-    for (int ic0 = rr.begin; ic0 < end; ic0 += kMaxGridY) {
-        const int rows = end - ic0 < kMaxGridY ? end - ic0 : kMaxGridY;
-        dim3 grid((ne + kBlock - 1) / kBlock, rows);
-        atmos_f64_kernel<<<grid, kBlock, 0, s>>>(energies, ne, ne_pad, table, seg_off, seg_len,
-                                                 ic0, n_cosines, w, av, out);
+    const AvgInput av{avg.prob, avg.mid, avg.wid, avg.n_bins, p.anti};
+    const bool averaged = avg.n_bins > 0;
+    const int rows = averaged ? 1 : kFxWarps;  // of a block
+    const int end = rr.end < 0 ? n_cosines : rr.end, step = kMaxGridY * rows;
+    for (int ic0 = rr.begin; ic0 < end; ic0 += step) {
+        const int ic1 = end - ic0 < step ? end : ic0 + step;
+        dim3 grid((ne + 31) / 32, (ic1 - ic0 + rows - 1) / rows);
+        if (averaged)
+            atmos_fx_avg_kernel<<<grid, 32 * kFxWarps, 0, s>>>(p, energies, ne, pad_energies(ne), table, seg_off,
+                                                               seg_len, rho, per_class, ic0, n_cosines, av, out);
+        else
+            atmos_fx_inline_kernel<<<grid, 32 * kFxWarps, 0, s>>>(p, energies, ne, pad_energies(ne), table, seg_off,
+                                                                  seg_len, rho, ic0, ic1, n_cosines, out);
     }
     return cudaGetLastError();
 }
@@ -476,24 +548,17 @@ cudaError_t preload_atmos_mixed() {
     return cudaFuncGetAttributes(&a, atmos_mixed_kernel);
 }
 
-cudaError_t launch_atmos_inline(const OscParams& p, bool mixed, const double* energies, int ne,
-                                const int* seg_off, const void* seg_len, const double* seg_rho,
-                                int n_cosines, const AvgArrays& avg, void* out, cudaStream_t s,
-                                RowRange rr) {
+cudaError_t launch_atmos_mixed_inline(const OscParams& p, const double* energies, int ne,
+                                      const int* seg_off, const float2* seg_len,
+                                      const double* seg_rho, int n_cosines, float* out,
+                                      cudaStream_t s, RowRange rr) {
     if (ne <= 0 || n_cosines <= 0) return cudaSuccess;
-    const AvgInput av{avg.prob, avg.shift, avg.air_cm, avg.n_bins, p.anti};
     const int end = rr.end < 0 ? n_cosines : rr.end;
     for (int ic0 = rr.begin; ic0 < end; ic0 += kMaxGridY) {
         const int rows = end - ic0 < kMaxGridY ? end - ic0 : kMaxGridY;
         dim3 grid((ne + kBlock - 1) / kBlock, rows);
-        if (mixed)
-            atmos_mixed_inline_kernel<<<grid, kBlock, 0, s>>>(p, wparams(p), energies, ne, seg_off,
-                                                              (const float2*)seg_len, seg_rho, ic0,
-                                                              n_cosines, (float*)out);
-        else
-            atmos_f64_inline_kernel<<<grid, kBlock, 0, s>>>(p, energies, ne, seg_off,
-                                                            (const double*)seg_len, seg_rho, ic0,
-                                                            n_cosines, av, (double*)out);
+        atmos_mixed_inline_kernel<<<grid, kBlock, 0, s>>>(p, wparams(p), energies, ne, seg_off,
+                                                          seg_len, seg_rho, ic0, n_cosines, out);
     }
     return cudaGetLastError();
 }
@@ -564,7 +629,7 @@ __device__ __forceinline__ void atmos_bin_mixed_avg(SegFn seg, int M, const Laye
         float pr[3];
 #pragma unroll
         for (int f = 0; f < 3; f++)
-            pr[f] = av.prob[((((size_t)av.type * 3 + f) * ne + ie) * nc + ic) * av.nb + b];
+            pr[f] = av.prob[((((size_t)av.type * 3 + f) * nc + ic) * av.nb + b) * ne + ie];
 #pragma unroll
         for (int q = 0; q < 3; q++) {
             float lo;
@@ -747,6 +812,34 @@ cudaError_t launch_plane_transpose(const void* src, bool is_float, int nc, int n
         plane_transpose_kernel<float><<<grid, block, 0, s>>>((const float*)src, nc, ne, dst);
     else
         plane_transpose_kernel<double><<<grid, block, 0, s>>>((const double*)src, nc, ne, dst);
+    return cudaGetLastError();
+}
+
+// A matrix [rows][cols] of doubles transposed to [cols][rows] (as T): 32 x 32 tiles, one a block.
+template <class T>
+__global__ void __launch_bounds__(32 * 8)
+    weights_transpose_kernel(const double* __restrict__ src, int rows, long long cols, T* __restrict__ dst) {
+    __shared__ double tile[32][33];
+    const int tiles = (rows + 31) / 32;
+    const int r0 = (int)(blockIdx.x % tiles) * 32;
+    const long long c0 = (long long)(blockIdx.x / tiles) * 32;
+    for (int k = threadIdx.y; k < 32; k += 8)
+        if (r0 + k < rows && c0 + threadIdx.x < cols) tile[k][threadIdx.x] = src[(size_t)(r0 + k) * cols + c0 + threadIdx.x];
+    __syncthreads();
+    for (int k = threadIdx.y; k < 32; k += 8)
+        if (c0 + k < cols && r0 + (int)threadIdx.x < rows) dst[(size_t)(c0 + k) * rows + r0 + threadIdx.x] = (T)tile[threadIdx.x][k];
+}
+
+cudaError_t launch_weights_transpose(const double* src, int rows, long long cols, void* dst,
+                                     bool to_float, cudaStream_t s) {
+    if (rows <= 0 || cols <= 0) return cudaSuccess;
+    const long long blocks = (long long)((rows + 31) / 32) * ((cols + 31) / 32);
+    if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
+    const dim3 block(32, 8);
+    if (to_float)
+        weights_transpose_kernel<float><<<(unsigned)blocks, block, 0, s>>>(src, rows, cols, (float*)dst);
+    else
+        weights_transpose_kernel<double><<<(unsigned)blocks, block, 0, s>>>(src, rows, cols, (double*)dst);
     return cudaGetLastError();
 }
 

@@ -30,7 +30,8 @@ constexpr int kFxRates = 9;
 constexpr int kFxFields = 11;
 // After the classes, once per energy: the electron and muon rows of W U_1 and of W U_0 (three
 // real, three complex numbers each; U_c = [u0 u1 u2] of class c, class 0 the air), and the
-// coefficients of a bin that crosses no shell.
+// coefficients of a bin that crosses no shell.  A table of the air alone holds U_0 in the place
+// of the rows of W U_1.
 constexpr int kFxV1 = 0, kFxV0 = 9, kFxVac = 18, kFxExtra = 31;
 
 struct fx {
@@ -75,9 +76,10 @@ CP3_HD double fx_bits_to_double(long long b) {
 #endif
 }
 
-// A fixed-point number in [0, 2) as a double (below 0, by the last bits of its sums: 0).
+// A fixed-point number as a double.  A probability that the rounding of its sums left within
+// 2^-50 below zero is zero.
 CP3_HD double fx_to_double(long long v) {
-    if (v <= 0) return 0.0;
+    if (v <= 0 && v > -4096) return 0.0;
     return fx_bits_to_double(fx_bits((double)v) - (62LL << 52));
 }
 
@@ -240,11 +242,6 @@ struct FxColumn {
     }
 };
 
-CP3_HD void fx_layer(const FxColumn& t, int c, double L, const longlong2* trig, cfx e[2], unsigned int& bad) {
-#pragma unroll
-    for (int k = 0; k < 2; k++) e[k] = fx_unit(fx_angle(t.rate(c, k), L, bad), trig);
-}
-
 CP3_HD void fx_load_rotation(const FxColumn& t, int c, fx R[9]) {
 #pragma unroll
     for (int f = 0; f < 9; f++) R[f] = t.rot(c, f);
@@ -292,6 +289,58 @@ CP3_HD long long fx_norm(cfx a) {
     return fx_sum(s);
 }
 
+// y <- D y for the phases e of one layer
+CP3_HD void fx_phase(const cfx e[2], cfx y[3]) {
+    y[1] = fx_cmul(e[0], y[1]);
+    y[2] = fx_cmul(e[1], y[2]);
+}
+
+// The sum of the layers' phases: e^{-i (sum)} is the determinant of their product.
+struct FxDet {
+    int k = 0;
+    long long x = 0;
+};
+
+// The two phases of one layer; `det` collects them where given.
+CP3_HD void fx_layer(const double rate[2], double L, const longlong2* trig, cfx e[2], unsigned int& bad,
+                     FxDet* det = nullptr) {
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        const FxAngle a = fx_angle(rate[k], L, bad);
+        if (det) {
+            det->k += a.k;
+            det->x += a.x;
+        }
+        e[k] = fx_unit(a, trig);
+    }
+}
+
+// The third column of a unitary matrix from two: det conj(y0 x y1).
+CP3_HD void fx_third_column(const FxDet& s, const longlong2* trig, cfx y[3][3]) {
+    // the phase is 2 pi k / 512 + x; x is brought back below pi / 512
+    const double x = (double)s.x * 3.469446951953614189e-18;  // 2^-58
+    const double m = rint(x * 81.48733086305041);             // 512 / (2 pi)
+    FxAngle d;
+    d.k = s.k + (int)m;
+    d.x = s.x - (long long)(int)m * 3537118876014220LL;  // (2 pi / 512) 2^58
+    const cfx det = fx_unit(d, trig);
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        const int j = (i + 1) % 3, k = (i + 2) % 3;
+        y[2][i] = fx_cmul(det, fx_cross(y[0][j], y[0][k], y[1][j], y[1][k]));
+    }
+}
+
+// k <- Y^T D Y k for Y with columns y[0..2]
+CP3_HD void fx_palindrome(const cfx y[3][3], const cfx e[2], cfx k[3]) {
+    cfx m[3];
+#pragma unroll
+    for (int i = 0; i < 3; i++) m[i] = fx_cdot(y[0][i], k[0], y[1][i], k[1], y[2][i], k[2]);
+    fx_phase(e, m);
+#pragma unroll
+    for (int i = 0; i < 3; i++) k[i] = fx_cdot(y[i][0], m[0], y[i][1], m[1], y[i][2], m[2]);
+}
+
 // The four probabilities of a single layer from its coefficients (fx_coefficients) and phases:
 // P = P0 + sum_k d_k cos D_k for the two survivals, and for the pair the same plus or minus
 // J (sin D10 - sin D20 + sin D21).
@@ -335,8 +384,12 @@ CP3_HD void fx_one_layer(const fx v[13], const cfx e[2], long long P[4]) {
 CP3_HD bool fx_bin(const FxColumn& t, const double* len, int M, const longlong2* trig, long long P[4]) {
     unsigned int bad = 0;
     cfx e[2];
+    auto layer = [&](int l, cfx* f, FxDet* det) {
+        const double rate[2] = {t.rate(l, 0), t.rate(l, 1)};
+        fx_layer(rate, len[l], trig, f, bad, det);
+    };
     if (M == 0) {
-        fx_layer(t, 0, len[0], trig, e, bad);
+        layer(0, e, nullptr);
         fx v[13];
 #pragma unroll
         for (int f = 0; f < 13; f++) v[f] = t.extra(kFxVac + f);
@@ -345,18 +398,8 @@ CP3_HD bool fx_bin(const FxColumn& t, const double* len, int M, const longlong2*
     }
     cfx y[3][3];
     if (M > 1) {
-        int ks = 0;
-        long long xs = 0;
-        auto phases = [&](int l) {
-#pragma unroll
-            for (int k = 0; k < 2; k++) {
-                const FxAngle a = fx_angle(t.rate(l, k), len[l], bad);
-                ks += a.k;
-                xs += a.x;
-                e[k] = fx_unit(a, trig);
-            }
-        };
-        phases(1);
+        FxDet det;
+        layer(1, e, &det);
 #pragma unroll
         for (int i = 0; i < 3; i++) {
             const fx a = t.rot(1, 3 * i), b = t.rot(1, 3 * i + 1);
@@ -370,30 +413,18 @@ CP3_HD bool fx_bin(const FxColumn& t, const double* len, int M, const longlong2*
         for (int l = 2; l < M; l++) {
             fx R[9];
             fx_load_rotation(t, l, R);
-            phases(l);
+            layer(l, e, &det);
 #pragma unroll
             for (int j = 0; j < 2; j++) {
-                y[j][1] = fx_cmul(e[0], y[j][1]);
-                y[j][2] = fx_cmul(e[1], y[j][2]);
+                fx_phase(e, y[j]);
                 fx_rotate(R, y[j]);
             }
         }
-        // the determinant's phase: 2 pi ks / 512 + xs, the second brought back below pi / 512
-        const double x = (double)xs * 3.469446951953614189e-18;  // 2^-58
-        const double m = rint(x * 81.48733086305041);            // 512 / (2 pi)
-        FxAngle d;
-        d.k = ks + (int)m;
-        d.x = xs - (long long)(int)m * 3537118876014220LL;  // (2 pi / 512) 2^58
-        const cfx det = fx_unit(d, trig);
-#pragma unroll
-        for (int i = 0; i < 3; i++) {
-            const int j = (i + 1) % 3, k = (i + 2) % 3;
-            y[2][i] = fx_cmul(det, fx_cross(y[0][j], y[0][k], y[1][j], y[1][k]));
-        }
+        fx_third_column(det, trig, y);
     }
     cfx e0[2];
-    fx_layer(t, 0, len[0], trig, e0, bad);
-    fx_layer(t, M, len[M], trig, e, bad);
+    layer(0, e0, nullptr);
+    layer(M, e, nullptr);
     fx R0[9];
     fx_load_rotation(t, 0, R0);
 #pragma unroll 1
@@ -404,21 +435,12 @@ CP3_HD bool fx_bin(const FxColumn& t, const double* len, int M, const longlong2*
         for (int i = 0; i < 3; i++)
             k[i] = j == 0 ? cfx{t.extra(kFxV0 + i), fx{0, 0}}
                           : cfx{t.extra(kFxV0 + 3 + i), fx_neg(t.extra(kFxV0 + 6 + i))};
-        k[1] = fx_cmul(e0[0], k[1]);
-        k[2] = fx_cmul(e0[1], k[2]);
+        fx_phase(e0, k);
         fx_rotate(R0, k);
-        if (M > 1) {
-            cfx m[3];
-#pragma unroll
-            for (int i = 0; i < 3; i++) m[i] = fx_cdot(y[0][i], k[0], y[1][i], k[1], y[2][i], k[2]);
-            m[1] = fx_cmul(e[0], m[1]);
-            m[2] = fx_cmul(e[1], m[2]);
-#pragma unroll
-            for (int i = 0; i < 3; i++) k[i] = fx_cdot(y[i][0], m[0], y[i][1], m[1], y[i][2], m[2]);
-        } else {
-            k[1] = fx_cmul(e[0], k[1]);
-            k[2] = fx_cmul(e[1], k[2]);
-        }
+        if (M > 1)
+            fx_palindrome(y, e, k);
+        else
+            fx_phase(e, k);
         cfx ae, am;
         {
             fxacc r, m;
@@ -763,6 +785,288 @@ CP3_HD void fx_coefficients(const fx row[9], fx v[13]) {
     fx_mac(j, row[8], row[4]);
     fx_mac(j, fx_neg(row[5]), row[7]);
     v[12] = fx_split(4 * mul(fx_res(j), fx_split(mul(row[1], row[2]))));
+}
+
+// ---- bins whose layers are solved in place ------------------------------------------------
+// (quadratic densities, where every segment has its own, and production-height averaging)
+
+// What the bins of one energy share: the air layer and W's entries.
+struct FxAir {
+    fx U[3][3];     // eigenvectors of the air layer
+    fx row[9];      // its flavour rows (fx_rows)
+    fx coef[13];    // fx_coefficients
+    double rate[2];
+};
+struct FxW {
+    fx c, s, cr, ci, sr, si;  // cos, sin of theta23; the same times e^{i delta}
+};
+CP3_HD FxW fx_w(const double* w) {
+    return FxW{fx_split(fx_from_double(w[0])),        fx_split(fx_from_double(w[1])),
+               fx_split(fx_from_double(w[0] * w[2])), fx_split(fx_from_double(w[0] * w[3])),
+               fx_split(fx_from_double(w[1] * w[2])), fx_split(fx_from_double(w[1] * w[3]))};
+}
+
+// a x + (b + i c) y: a row of W on entries x, y of a vector in the rotated basis
+CP3_HD cfx fx_flavour(fx a, fx b, fx c, cfx x, cfx y) {
+    fxacc2 r, m;
+    fx_mac(r, a, x.re), fx_mac(r, b, y.re), fx_mac(r, fx_neg(c), y.im);
+    fx_mac(m, a, x.im), fx_mac(m, b, y.im), fx_mac(m, c, y.re);
+    return cfx{fx_res(r), fx_res(m)};
+}
+
+// U v and U^T v, U real
+CP3_HD void fx_apply(const fx U[3][3], cfx v[3]) {
+    const fx R[9] = {U[0][0], U[0][1], U[0][2], U[1][0], U[1][1], U[1][2], U[2][0], U[2][1], U[2][2]};
+    fx_rotate(R, v);
+}
+CP3_HD void fx_apply_transposed(const fx U[3][3], cfx v[3]) {
+    const fx R[9] = {U[0][0], U[1][0], U[2][0], U[0][1], U[1][1], U[2][1], U[0][2], U[1][2], U[2][2]};
+    fx_rotate(R, v);
+}
+
+// The amplitude of the segments 1..M in the rotated basis, G = B^T S_M B with B = S_{M-1}..S_1
+// (G = 1 for M = 0), ready to be applied to vectors: Y = U_M^T B, whose columns start from the
+// rows of U_1.  solve(l, k) gives segment l's layer.
+struct FxAmplitude {
+    cfx y[3][3];
+    cfx e[2];
+    fx U1[3][3];
+    int M;
+    CP3_HD void apply(cfx k[3]) const {
+        if (M == 0) return;
+        if (M == 1) {
+            fx_apply_transposed(U1, k);
+            fx_phase(e, k);
+            fx_apply(U1, k);
+        } else {
+            fx_palindrome(y, e, k);
+        }
+    }
+};
+
+template <class Solve>
+CP3_HD void fx_chain(Solve solve, const double* len, int M, const longlong2* trig, unsigned int& bad, FxAmplitude& g) {
+    g.M = M;
+    FxDet det;
+    fx U[3][3];
+#pragma unroll 1
+    for (int l = 1; l <= M; l++) {
+        FxClass n;
+        solve(l, n);
+        if (l == 1) {
+#pragma unroll
+            for (int j = 0; j < 2; j++)
+#pragma unroll
+                for (int i = 0; i < 3; i++) g.y[j][i] = cfx{n.U[j][i], fx{0, 0}};
+        } else {
+            fx R[3][3];
+            fx_rotation(n.U, U, R);
+#pragma unroll
+            for (int j = 0; j < 2; j++) {
+                fx_phase(g.e, g.y[j]);
+                fx_apply(R, g.y[j]);
+            }
+        }
+        fx_layer(n.rate, len[l], trig, g.e, bad, l < M ? &det : nullptr);
+#pragma unroll
+        for (int i = 0; i < 3; i++)
+#pragma unroll
+            for (int k = 0; k < 3; k++) U[i][k] = n.U[i][k];
+    }
+    if (M == 1) {
+#pragma unroll
+        for (int i = 0; i < 3; i++)
+#pragma unroll
+            for (int k = 0; k < 3; k++) g.U1[i][k] = U[i][k];
+    } else if (M > 1) {
+        fx_third_column(det, trig, g.y);
+    }
+}
+
+// One bin; false where it needs the FP64 path.
+template <class Solve>
+CP3_HD bool fx_bin_inline(Solve solve, const FxAir& air, const FxW& w, const double* len, int M,
+                          const longlong2* trig, long long P[4]) {
+    unsigned int bad = 0;
+    cfx e0[2];
+    fx_layer(air.rate, len[0], trig, e0, bad);
+    if (M == 0) {
+        fx_one_layer(air.coef, e0, P);
+        return (bad >> 20) == 0;
+    }
+    FxAmplitude g;
+    fx_chain(solve, len, M, trig, bad, g);
+#pragma unroll 1
+    for (int j = 0; j < 2; j++) {  // initial flavours e, mu: S_0 W^+ column j
+        cfx k[3];
+#pragma unroll
+        for (int i = 0; i < 3; i++)
+            k[i] = j == 0 ? cfx{air.row[i], fx{0, 0}} : cfx{air.row[3 + i], fx_neg(air.row[6 + i])};
+        fx_phase(e0, k);
+        fx_apply(air.U, k);
+        g.apply(k);
+        P[2 * j] = fx_norm(k[0]);
+        P[2 * j + 1] = fx_norm(fx_flavour(w.c, w.sr, w.si, k[1], k[2]));
+    }
+    return (bad >> 20) == 0;
+}
+
+// ---- production-height averaging ----------------------------------------------------------
+// physics.hpp:997-1130: with the amplitude split over the air layer's eigenstates,
+// A = sum_k e_k a_k b_k^+ (a_k = W G u_k, b_k = W u_k), each cross term of a probability is
+// weighted by t_kq = sum over height bins of prob sinc(d w / 2) e^{i d m}, d = -(omega_k -
+// omega_q), m and w the mid shift and the width of the bin's path lengths:
+//   P(j -> i) = sum_k |a_ki|^2 |b_kj|^2
+//               + 2 sum_{q<k} Re[conj(a_qi) a_ki  e_k conj(e_q) b_qj conj(b_kj) t_kq,j].
+// The a_k are orthonormal, so the sum over i is 1 whatever the weights, and the rows e and mu
+// are enough.
+
+// math::defined_sinc (math.hpp:49-55) as the reference evaluates it (its abs() is the int one:
+// the series branch for every |x| < 1).
+CP3_HD fx fx_sinc(double x) {
+    if (!(fabs(x) < 1.0)) return fx_split(fx_from_double(sin(x) / x));
+    const fx X = fx_split(fx_scaled(x, 1023));
+    fxacc a;
+    fx_mac(a, X, X);
+    const fx x2 = fx_res(a);
+    fxacc b, c;
+    fx_mac(b, x2, fx_split(38430716820228232LL));  // 1 / 120
+    fx_mac(c, x2, fx_split(768614336404564651LL - fx_sum(b)));  // 1 / 6 - x^2 / 120
+    return fx_split((1LL << 62) - fx_sum(c));
+}
+
+// The sums t over some of a bin's heights (b0, b0 + step, ...), and the sums of the weights'
+// magnitudes (54 fraction bits).  The products' leading and cross terms accumulate over the
+// heights as they are, with the low words cut to 27 bits (2^-57): the cross terms of 20 heights
+// stay below 2^63 and no sum is formed per height.
+struct FxShift {
+    long long hh[3][3][2] = {}, x[3][3][2] = {};  // [pair][initial flavour][re, im]
+    unsigned long long total[3] = {};
+    CP3_HD long long value(int q, int f, int c) const { return hh[q][f][c] * 4 + (x[q][f][c] >> 25); }
+};
+
+// prob, mid, wid: the height bins' probabilities of the three initial flavours (b-th at
+// prob[f * flavour + b * stride]), their mid shifts and widths in km.
+CP3_HD void fx_shift_sums(const double rate[2], int b0, int step, int nb, const double* prob, size_t flavour,
+                          size_t stride, const double* mid, const double* wid, const longlong2* trig,
+                          unsigned int& bad, FxShift& o) {
+    const double pr[2] = {rate[0] * M_PI, rate[1] * M_PI};
+#pragma unroll 1
+    for (int b = b0; b < nb; b += step) {
+        const double h = -mid[b], w = wid[b];
+        cfx z[3];
+        double x[3];
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+            fx_sincos(fx_angle(rate[q], h, bad), trig, z[q].re, z[q].im);
+            x[q] = pr[q] * w;
+        }
+        x[2] = x[1] - x[0];
+        z[2] = fx_cmul(cfx{z[0].re, fx_neg(z[0].im)}, z[1]);
+#pragma unroll
+        for (int q = 0; q < 3; q++) {
+            const fx s = fx_sinc(x[q]);
+            fxacc r, m;
+            fx_mac(r, s, z[q].re);
+            fx_mac(m, s, z[q].im);
+            z[q] = cfx{fx_res(r), fx_res(m)};
+            z[q].re.l >>= 5;
+            z[q].im.l >>= 5;
+        }
+#pragma unroll
+        for (int f = 0; f < 3; f++) {
+            const double p = prob[f * flavour + b * stride];
+            const long long pb = fx_bits(p) & 0x7fffffffffffffffLL;
+            if (pb > 0x3ff0000000000000LL) bad |= 1u << 20;  // above 1, or not a number
+            const long long pv = pb > 0x3ff0000000000000LL ? 0 : fx_scaled(p, 1023);
+            o.total[f] += (unsigned long long)(pv < 0 ? -pv : pv) >> 8;
+            fx pf = fx_split(pv);
+            pf.l >>= 5;
+#pragma unroll
+            for (int q = 0; q < 3; q++)
+#pragma unroll
+                for (int c = 0; c < 2; c++) {
+                    const fx v = c == 0 ? z[q].re : z[q].im;
+                    o.hh[q][f][c] += (long long)pf.h * v.h;
+                    o.x[q][f][c] += (long long)pf.h * v.l;
+                    o.x[q][f][c] += (long long)pf.l * v.h;
+                }
+        }
+    }
+}
+
+// The factors t from the sums over all heights; weights that add up to more than 5/4 leave the
+// range.
+CP3_HD void fx_shift_factors(const long long sum[3][3][2], const unsigned long long total[3], unsigned int& bad,
+                             cfx t[3][3]) {
+#pragma unroll
+    for (int f = 0; f < 3; f++)
+        if (total[f] > (5ULL << 52)) bad |= 1u << 20;
+#pragma unroll
+    for (int q = 0; q < 3; q++)
+#pragma unroll
+        for (int f = 0; f < 3; f++) t[q][f] = cfx{fx_split(sum[q][f][0]), fx_split(sum[q][f][1])};
+}
+
+// The rows e, mu of a_k = W G u_k.
+template <class Solve>
+CP3_HD void fx_air_rows(Solve solve, const FxAir& air, const FxW& w, const double* len, int M,
+                        const longlong2* trig, unsigned int& bad, cfx a[2][3]) {
+    FxAmplitude g;
+    fx_chain(solve, len, M, trig, bad, g);
+#pragma unroll 1
+    for (int k = 0; k < 3; k++) {
+        cfx v[3];
+#pragma unroll
+        for (int i = 0; i < 3; i++) v[i] = cfx{air.U[i][k], fx{0, 0}};
+        g.apply(v);
+        a[0][k] = v[0];
+        a[1][k] = fx_flavour(w.c, w.sr, w.si, v[1], v[2]);
+    }
+}
+
+// One averaged bin from these rows and its shift factors; P[j][i] the probability of j -> i,
+// i = e, mu.
+CP3_HD void fx_average(const cfx a[2][3], const FxAir& air, const FxW& w, double air_km,
+                       const longlong2* trig, const cfx t[3][3], unsigned int& bad, long long P[3][2]) {
+    cfx e[3];  // e_k conj(e_q) of the pairs (1,0), (2,0), (2,1)
+    fx_layer(air.rate, air_km, trig, e, bad);
+    e[2] = fx_cmul(cfx{e[0].re, fx_neg(e[0].im)}, e[1]);
+    const int hi[3] = {1, 2, 2}, lo[3] = {0, 0, 1};
+    fx n[2][3];
+    cfx d[2][3];  // conj(a_qi) a_ki
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            n[i][k] = fx_split(fx_norm(a[i][k]));
+            const cfx q = a[i][lo[k]];
+            d[i][k] = fx_cmul(cfx{q.re, fx_neg(q.im)}, a[i][hi[k]]);
+        }
+#pragma unroll 1
+    for (int j = 0; j < 3; j++) {
+        cfx b[3];
+#pragma unroll
+        for (int k = 0; k < 3; k++)
+            b[k] = j == 0 ? cfx{air.row[k], fx{0, 0}}
+                   : j == 1 ? cfx{air.row[3 + k], air.row[6 + k]}
+                            : fx_flavour(fx_neg(w.s), w.cr, w.ci, cfx{air.U[1][k], fx{0, 0}}, cfx{air.U[2][k], fx{0, 0}});
+        fxacc2 s[2], x[2];
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            const fx m = fx_split(fx_norm(b[k]));
+            const cfx c = b[hi[k]];
+            const cfx f = fx_cmul(t[k][j], fx_cmul(e[k], fx_cmul(cfx{c.re, fx_neg(c.im)}, b[lo[k]])));
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+                fx_mac(s[i], n[i][k], m);
+                fx_mac(x[i], d[i][k].re, f.re);
+                fx_mac(x[i], fx_neg(d[i][k].im), f.im);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 2; i++) P[j][i] = fx_sum(s[i]) + 2 * fx_sum(x[i]);
+    }
 }
 
 }  // namespace cp3

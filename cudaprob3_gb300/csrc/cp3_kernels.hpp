@@ -8,19 +8,14 @@
 
 namespace cp3 {
 
-// Fields of one (density class, energy) entry of the eigen tables.
-constexpr int kF64Fields = 10;  // u1 (3), u2 (3) rotated-basis unit eigenvectors,
-                                // dmMatVac[k][0] (3), 1 unused (one 80-byte entry)
+// Fields of one (density class, energy) entry of the mixed eigen table.
 constexpr int kMixFields = 12;  // u1 (3), u2 (3) real unit eigenvectors; omega_1, omega_2 in
                                 // turns per km, double-float as (hi1, hi2, lo1, lo2); 2 unused
                                 // (one 48-byte entry per (class, energy))
 
 inline int pad_energies(int ne) { return (ne + 31) / 32 * 32; }
 
-// Eigen tables over (class, energy): FP64 flavour projectors (reference expansion), or the
-// rotated-basis real projectors + double-float phase rates of the mixed kernels.
-cudaError_t launch_table_f64(const OscParams& p, const double* energies, int ne,
-                             const double* cls_rho, int ncls, double* table, cudaStream_t s);
+// The mixed eigen table over (class, energy): real eigenvectors and double-float phase rates.
 cudaError_t launch_table_mixed(const OscParams& p, const double* energies, int ne,
                                const double* cls_rho, int ncls, float* table, cudaStream_t s);
 // The same from float pairs (hi, lo) split on the host: no FP64 instruction on the device.
@@ -41,9 +36,10 @@ cudaError_t preload_atmos_mixed();
 
 // Production-height averaging inputs of the FP64 kernels (n_bins == 0: fixed height).
 struct AvgArrays {
-    const double* prob = nullptr;    // [2][3][ne][nc][n_bins]
-    const double* shift = nullptr;   // [nc][n_bins + 1] path-length shifts at the edges, cm
-    const double* air_cm = nullptr;  // [nc] first (air) segment, cm
+    const double* prob = nullptr;  // [2][3][nc][n_bins][ne]: consecutive energies are contiguous
+    const double* mid = nullptr;   // [nc][n_bins] mid path-length shift of each bin, km (0 where the
+                                   // air segment has zero length)
+    const double* wid = nullptr;   // [nc][n_bins] bin width, km (0 likewise)
     int n_bins = 0;
 };
 
@@ -56,10 +52,6 @@ struct RowRange {
 // trajectory of row i is segments seg_off[i]..seg_off[i+1]-1 (air, then shells inwards); the
 // table class of a row's segment l is l itself (class 0 the air, class l shell l-1, as
 // build_trajectories numbers them), so no class array is read.
-cudaError_t launch_atmos_f64(const OscParams& p, const double* energies, int ne,
-                             const double* table, const int* seg_off, const double* seg_len,
-                             int n_cosines, const AvgArrays& avg, double* out,
-                             cudaStream_t s, RowRange rr = RowRange{});
 // FP64 bins from the fixed-point table, constant densities and a fixed production height.
 // Bins whose table entries or phases are out of its range take the FP64 path, from the class
 // densities.
@@ -74,7 +66,7 @@ cudaError_t launch_atmos_mixed(const OscParams& p, const float* table, int ne,
 
 // Production-height averaging inputs of the mixed kernels (float, from AvgArrays on the host).
 struct AvgMixed {
-    const float* prob = nullptr;  // [2][3][ne][nc][n_bins]
+    const float* prob = nullptr;  // [2][3][nc][n_bins][ne]
     const float2* hm = nullptr;   // [nc][n_bins] mid shift of each bin, km, float pair (0 where the
                                   // air segment has zero length)
     const float* hw = nullptr;    // [nc][n_bins] bin width, km (0 likewise)
@@ -94,12 +86,22 @@ cudaError_t launch_atmos_mixed_inline_avg(const OscParams& p, const double* ener
                                           const AvgMixed& av, float* out, cudaStream_t s,
                                           RowRange rr = RowRange{});
 
-// Atmospheric bins whose segments each carry their own electron density (quadratic model):
-// per-segment eigen-solve.  seg_len: double[] (FP64) or float2[] hi/lo (mixed).
-cudaError_t launch_atmos_inline(const OscParams& p, bool mixed, const double* energies, int ne,
-                                const int* seg_off, const void* seg_len, const double* seg_rho,
-                                int n_cosines, const AvgArrays& avg, void* out, cudaStream_t s,
-                                RowRange rr = RowRange{});
+// Atmospheric bins whose layers are solved in place.  FP64: quadratic densities (rho per
+// segment) and production-height averaging (avg.n_bins > 0; rho per segment, or per class with
+// per_class), with the fixed-point table of the air alone (launch_table_fx, one class); mixed:
+// quadratic densities.
+cudaError_t launch_atmos_fx_inline(const OscParams& p, const double* energies, int ne,
+                                   const int2* table, const int* seg_off, const double* seg_len, const double* rho,
+                                   bool per_class, int n_cosines, const AvgArrays& avg, double* out,
+                                   cudaStream_t s, RowRange rr = RowRange{});
+cudaError_t launch_atmos_mixed_inline(const OscParams& p, const double* energies, int ne,
+                                      const int* seg_off, const float2* seg_len,
+                                      const double* seg_rho, int n_cosines, float* out,
+                                      cudaStream_t s, RowRange rr = RowRange{});
+
+// A matrix [rows][cols] of doubles transposed to [cols][rows], as floats or doubles.
+cudaError_t launch_weights_transpose(const double* src, int rows, long long cols, void* dst,
+                                     bool to_float, cudaStream_t s);
 
 // out[i] = (x[i] rounded to float, the remainder rounded to float), on the device.
 cudaError_t launch_split_pairs(const double* x, int n, float2* out, cudaStream_t s);

@@ -19,27 +19,6 @@ namespace {
 
 constexpr int kTableBlock = 128;
 
-// FP64 table: the rotated-basis unit eigenvectors u1, u2 (from the reference's getMfast
-// masses, physics.hpp:267-340, and the projectors of H0 + V e0 e0^T) and dmMatVac[k][0]
-// (physics.hpp:337-339), from which the bin kernel forms the reference's phases.  AoS: one
-// 80-byte entry per (class c, energy e) at table[(c * ne_pad + e) * 10].
-__global__ void __launch_bounds__(kTableBlock)
-    table_f64_kernel(const __grid_constant__ OscParams p, const double* __restrict__ energies,
-                     int ne, int ne_pad, const double* __restrict__ cls_rho,
-                     double* __restrict__ table) {
-    const int ie = blockIdx.x * kTableBlock + threadIdx.x;
-    const int c = blockIdx.y;
-    if (ie >= ne) return;
-    double u[2][3], dmv[3];
-    rotated_layer_f64(&p, energies[ie], cls_rho[c], u, dmv);
-    double2* t = reinterpret_cast<double2*>(table + ((size_t)c * ne_pad + ie) * kF64Fields);
-    t[0] = make_double2(u[0][0], u[0][1]);
-    t[1] = make_double2(u[0][2], u[1][0]);
-    t[2] = make_double2(u[1][1], u[1][2]);
-    t[3] = make_double2(dmv[0], dmv[1]);
-    t[4] = make_double2(dmv[2], 0.0);
-}
-
 // The table of the fixed-point FP64 bins (cp3_fixed.cuh): for each class the rotation to the
 // next class's eigenbasis and the phase rates, and once per energy the flavour rows and the
 // vacuum coefficients.  A block is 32 energies by a run of kFxRun classes, one class a warp;
@@ -73,6 +52,10 @@ __global__ void __launch_bounds__(32 * (kFxRun + 1))
                 fx_coefficients(row, v);
 #pragma unroll
                 for (int f = 0; f < 13; f++) ext[(size_t)(kFxVac + f) * ne_pad] = make_int2(v[f].h, v[f].l);
+                if (ncls == 1) {
+#pragma unroll
+                    for (int f = 0; f < 9; f++) ext[(size_t)(kFxV1 + f) * ne_pad] = s_u[wv][f][lane];
+                }
             }
         }
     }
@@ -155,14 +138,6 @@ __global__ void __launch_bounds__(kTableBlock)
 }
 
 }  // namespace
-
-cudaError_t launch_table_f64(const OscParams& p, const double* energies, int ne,
-                             const double* cls_rho, int ncls, double* table, cudaStream_t s) {
-    if (ne <= 0 || ncls <= 0) return cudaSuccess;
-    dim3 grid((ne + kTableBlock - 1) / kTableBlock, ncls);
-    table_f64_kernel<<<grid, kTableBlock, 0, s>>>(p, energies, ne, pad_energies(ne), cls_rho, table);
-    return cudaGetLastError();
-}
 
 size_t table_fx_words(int ncls, int ne) {
     return ((size_t)ncls * kFxFields + kFxExtra) * pad_energies(ne);

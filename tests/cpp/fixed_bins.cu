@@ -73,3 +73,81 @@ extern "C" int fixed_atmos(const double* mix, int knutype, int anti, const doubl
     }
     return outside;
 }
+
+// The bins whose layers are solved in place: densities per segment (poly: the quadratic
+// coefficients a, b, c), with nb > 0 production-height averaging (prob [2][3][nc][nb][ne], edges
+// in km).
+extern "C" int fixed_inline(const double* mix, int knutype, int anti, const double* cz, int nc,
+                            const double* en, int ne, const double* radii, const double* a,
+                            const double* b, const double* c, const double* ye, int n, int poly,
+                            double height_km, int nb, const double* prob, const double* edges, double* out) {
+    OscParams p;
+    build_osc_params(MixingInput{mix[0], mix[1], mix[2], mix[3], knutype, mix[4], mix[5]}, anti, &p);
+    EarthModel model;
+    std::string msg;
+    TrajectoryTable t;
+    if (make_earth_model(radii, a, b, c, ye, n, poly != 0, &model, &msg) ||
+        build_trajectories(model, cz, nc, height_km * 1e5, &t, &msg))
+        return -1;
+    std::vector<double> sh;
+    if (nb) production_height_shifts(cz, nc, height_km * 1e5, edges, nb, &sh);
+    const longlong2* trig = reinterpret_cast<const longlong2*>(&kTable);
+    const FxW w = fx_w(p.w);
+    int outside = 0;
+    for (int ie = 0; ie < ne; ie++) {
+        auto layer = [&](double rho_e, FxClass& k) {
+            double u[2][3], dmv[3];
+            rotated_layer_f64(&p, en[ie], rho_e, u, dmv);
+            fx_class_f64(u, dmv, en[ie], k);
+        };
+        FxClass k0;
+        layer(0.0, k0);
+        FxAir air;
+        std::memcpy(air.U, k0.U, sizeof air.U);
+        fx_rows(k0.U, p.w, air.row);
+        fx_coefficients(air.row, air.coef);
+        air.rate[0] = k0.rate[0], air.rate[1] = k0.rate[1];
+        for (int ic = 0; ic < nc; ic++) {
+            const double *len = t.len_km.data() + t.offset[ic], *rho = t.rho_e.data() + t.offset[ic];
+            auto solve = [&](int l, FxClass& k) { layer(rho[l], k); };
+            double* o = out + (size_t)ic * ne + ie;
+            const size_t plane = (size_t)nc * ne;
+            if (nb == 0) {
+                long long P[4];
+                outside += !fx_bin_inline(solve, air, w, len, t.maxlayers[ic], trig, P);
+                fx_store(P, o, plane);
+                continue;
+            }
+            std::vector<double> mid(nb), wid(nb);
+            for (int q = 0; q < nb; q++) {
+                const double h0 = sh[(size_t)ic * (nb + 1) + q], h1 = sh[(size_t)ic * (nb + 1) + q + 1];
+                mid[q] = t.air_cm[ic] == 0.0 ? 0.0 : 0.5 * (h0 + h1) / kKm2Cm;
+                wid[q] = t.air_cm[ic] == 0.0 ? 0.0 : (h1 - h0) / kKm2Cm;
+            }
+            unsigned int bad = 0;
+            long long sum[3][3][2] = {};
+            unsigned long long total[3] = {};
+            for (int part = 0; part < 3; part++) {  // the heights in three shares, as on the device
+                FxShift one;
+                fx_shift_sums(air.rate, part, 3, nb, prob + (((size_t)anti * 3 * nc + ic) * nb) * ne + ie,
+                              (size_t)nc * nb * ne, ne, mid.data(), wid.data(), trig, bad, one);
+                for (int j = 0; j < 3; j++) {
+                    total[j] += one.total[j];
+                    for (int q = 0; q < 6; q++) sum[q >> 1][j][q & 1] += one.value(q >> 1, j, q & 1);
+                }
+            }
+            cfx f[3][3], rows[2][3];
+            long long P[3][2];
+            fx_shift_factors(sum, total, bad, f);
+            fx_air_rows(solve, air, w, len, t.maxlayers[ic], trig, bad, rows);
+            fx_average(rows, air, w, len[0], trig, f, bad, P);
+            outside += (bad >> 20) != 0;
+            for (int j = 0; j < 3; j++) {
+                o[(size_t)(3 * j) * plane] = fx_to_double(P[j][0]);
+                o[(size_t)(3 * j + 1) * plane] = fx_to_double(P[j][1]);
+                o[(size_t)(3 * j + 2) * plane] = fx_to_double((1LL << 62) - P[j][0] - P[j][1]);
+            }
+        }
+    }
+    return outside;
+}

@@ -83,6 +83,36 @@ def test_out_of_range_bins_ask_for_the_fp64_path(host):
             assert outside == (0 if i in (0, 5) else len(cz)), en[i]
 
 
+@pytest.mark.parametrize("poly", [False, True])
+@pytest.mark.parametrize("nb,h", [(0, 22.0), (1, 0.0), (3, 22.0), (20, 15.0)])
+def test_host_bins_solved_in_place_against_oracle(host, oracle, poly, nb, h):
+    """Quadratic densities and production-height averaging: one bin and twenty, wide bins whose
+    sinc leaves its series, an air segment of zero length (h = 0); weights that are not a
+    distribution ask for the FP64 path."""
+    r, abc, ye = ((earth.PREM_4LAYER_QUAD_V2[0], earth.PREM_4LAYER_QUAD_V2[1:4], earth.PREM_4LAYER_QUAD_V2[4]) if poly
+                  else (earth.PREM_12LAYER[0], (earth.PREM_12LAYER[1],) * 3, earth.PREM_12LAYER[2]))
+    cz, en = np.concatenate([np.linspace(-1, 1, 13), [-0.02]]), np.logspace(-1, 2, 11)
+    rng = np.random.default_rng(4)
+    edges = np.linspace(2.0, 80.0, nb + 1)
+    prob = rng.uniform(0.1, 1.0, (2, 3, len(en), len(cz), max(nb, 1)))
+    prob /= prob.sum(axis=-1, keepdims=True)
+    m = earth.gaussian_sets(2, seed=9)[1]
+    for anti in (False, True):
+        ref = oracle.atmos(omix(m, anti), anti, cz, en, r, None if poly else abc[0], ye, h, poly_abc=abc if poly else None,
+                           avg=(nb, prob.ravel(), edges) if nb else None)
+        for scale, want in ((1.0, 0), (2.0, len(cz) * len(en) if nb else 0)):
+            a = [np.ascontiguousarray(x, dtype=np.float64)
+                 for x in ([m.theta12, m.theta13, m.theta23, m.dcp, m.dm12sq, m.dm23sq], cz, en, r, *abc, ye,
+                           np.transpose(scale * prob, (0, 1, 3, 4, 2)), edges)]
+            p = [x.ctypes.data_as(dp) for x in a]
+            out = np.empty((9, len(cz), len(en)))
+            n = host.fixed_inline(p[0], -1 if anti else 1, int(anti), p[1], len(cz), p[2], len(en), p[3], p[4], p[5], p[6],
+                                  p[7], len(r), int(poly), C.c_double(h), nb, p[8], p[9], out.ctypes.data_as(dp))
+            assert n == want
+            if scale == 1.0:
+                assert np.abs(np.transpose(out, (1, 2, 0)) - ref).max() <= 1e-12
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("shells,nc,ne", [(1, 1, 1), (1, 5, 33), (7, 4, 32), (8, 3, 31), (9, 6, 64), (16, 9, 65), (128, 13, 40)])
 def test_gpu_bins_at_the_edges_of_the_launch(oracle, shells, nc, ne):
@@ -96,6 +126,27 @@ def test_gpu_bins_at_the_edges_of_the_launch(oracle, shells, nc, ne):
     for anti in (False, True):
         got = run_atmos("fp64", mix6, -1 if anti else 1, anti, cz, en, *model, 22.0)
         assert np.abs(got - oracle.atmos(omix(m, anti), anti, cz, en, *model, 22.0, layer_limit=128)).max() <= 1e-12
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nb,nc,ne", [(1, 1, 1), (2, 5, 33), (20, 3, 31)])
+def test_gpu_averaged_bins_at_the_edges_and_out_of_range(oracle, nb, nc, ne):
+    """Averaged bins (FP64 and mixed) at the block edges, with weights that do not add up to one:
+    sums up to 1.2 stay in fixed point, sums of 3 take the FP64 path."""
+    from tests.test_gpu_averaging import run_avg
+    r, rho, ye = earth.synthetic_shells(9)
+    cz, en = np.linspace(-1, 0.4, nc), earth.log_energy_grid(ne)
+    prob = np.random.default_rng(6).uniform(0.1, 1.0, (2, 3, ne, nc, nb))
+    prob /= prob.sum(axis=-1, keepdims=True)
+    edges = np.linspace(3.0, 60.0, nb + 1)
+    m = earth.gaussian_sets(2, seed=10)[1]
+    mix6 = [m.theta12, m.theta13, m.theta23, m.dcp, m.dm12sq, m.dm23sq]
+    for scale in (1.0, 1.2, 3.0):
+        w = (scale * prob).ravel()
+        ref = oracle.atmos(omix(m, True), True, cz, en, r, rho, ye, 20.0, avg=(nb, w, edges))
+        for prec, tol in (("fp64", 1e-12), ("mixed", 1e-5)):
+            got = run_avg(prec, mix6, -1, True, cz, en, r, rho, ye, 20.0, nb, w, edges)
+            assert np.abs(got - ref).max() <= tol * max(1.0, scale)
 
 
 @pytest.mark.gpu
