@@ -242,9 +242,10 @@ __device__ __forceinline__ void atmos_bin_f64(SegFn seg, int M, const double* w,
 
 // FP64 bins in fixed point (cp3_fixed.cuh).  One warp is one cosine row x 32 energies; a block's
 // four warps take consecutive rows of the same energies, so that they read the same table lines.
-// Bound by the integer multiply-adds (80 % of the FMA pipe's heavy half; FP64 pipe 31 %).
-// Measured against the FP64 kernel it replaced: 59 shells, 2000 x 2000, 1.48 ms (10.14); PREM-12,
-// 307 x 811, 71 us; PREM-4, 400 x 400, 30 us (140).
+// Bound by the integer multiply-adds and the chain they stand in (72 % of the FMA pipe's heavy
+// half, ALU 46 %, FP64 pipe 40 %; three to five blocks an SM and two to eight warps a block are
+// within 8 %).  Measured against the FP64 kernel it replaced: 59 shells, 2000 x 2000, 1.12 ms
+// (10.14); PREM-12, 307 x 811, 53 us; PREM-4, 400 x 400, 22 us (140).
 constexpr int kFxWarps = 4;
 
 __device__ const TrigTable g_trig = make_trig_table();
@@ -297,7 +298,7 @@ __global__ void __launch_bounds__(32 * kFxWarps, 4)
 
 // FP64 bins in fixed point whose layers are solved in place, the air layer from a table of one
 // class.  (Solved by a block's first warp instead, its latency held the other three up: 96 us
-// instead of 73 + 8 for the grid below.)
+// for the quadratic grid below when this kernel took 73 and the table 8.)
 
 __device__ __forceinline__ FxAir load_air(const int2* table, int ne_pad, int ie, bool coef) {
     const FxColumn col{table + ie, table + (size_t)kFxFields * ne_pad + ie, (size_t)ne_pad, 0};
@@ -316,7 +317,7 @@ __device__ __forceinline__ FxAir load_air(const int2* table, int ne_pad, int ie,
 }
 
 // Quadratic densities: an eigen-system for every segment of every bin.  Blocks as above.  PREM's
-// quadratic model, 500 x 500: 73 us (481 in FP64 arithmetic).
+// quadratic model, 500 x 500: 57 us (481 in FP64 arithmetic).
 __global__ void __launch_bounds__(32 * kFxWarps, 3)
     atmos_fx_inline_kernel(const __grid_constant__ OscParams p, const double* __restrict__ energies,
                            int ne, int ne_pad, const int2* __restrict__ table, const int* __restrict__ seg_off,
@@ -355,7 +356,7 @@ __global__ void __launch_bounds__(32 * kFxWarps, 3)
 // the height bins, a third each (on a row that crosses no shell all four take a quarter) -- the
 // two are independent, and a grid of a few hundred rows and energies leaves the chip half empty
 // with one warp a bin.  PREM-4, 200 x 150, 20 heights:
-// 70 us (688 in FP64 arithmetic with the weights read across energies; 96 with one warp a bin).
+// 59 us (688 in FP64 arithmetic with the weights read across energies).
 __global__ void __launch_bounds__(32 * kFxWarps, 4)
     atmos_fx_avg_kernel(const __grid_constant__ OscParams p, const double* __restrict__ energies, int ne,
                         int ne_pad, const int2* __restrict__ table, const int* __restrict__ seg_off,

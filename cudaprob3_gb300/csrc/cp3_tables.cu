@@ -23,7 +23,7 @@ constexpr int kTableBlock = 128;
 // next class's eigenbasis and the phase rates, and once per energy the flavour rows and the
 // vacuum coefficients.  A block is 32 energies by a run of kFxRun classes, one class a warp;
 // the extra warp solves the class after the run, for the last rotation.  59 shells x 2000
-// energies take 24 us (130 with the FP64 formulas), PREM-4 x 400 energies 11 us (31): one wave,
+// energies take 21 us (130 with the FP64 formulas), PREM-4 x 400 energies 11 us (31): one wave,
 // its latency.
 constexpr int kFxRun = 8;
 
@@ -97,7 +97,7 @@ __global__ void __launch_bounds__(kTableBlock)
 
 // physics::calculate_beam (physics.hpp:1153-1260), one thread per energy; result [9][ne]: the
 // fixed-point layer of the energy (fx_solve) and the one-layer expansion of its probabilities.
-// 1e5 energies: 22.7 us (135 us in FP64 arithmetic, 582 FP64 instructions an energy).
+// 1e5 energies: 20.3 us (135 us in FP64 arithmetic, 582 FP64 instructions an energy).
 __device__ const TrigTable g_trig = make_trig_table();
 
 // A phase out of the fixed-point range: the FP64 formulas.
