@@ -1,5 +1,5 @@
 """Batches: many propagation problems (parameter set x neutrino type x grid) computed by one
-persistent, graph-captured launch (C ABI cp3_batch_*)."""
+persistent launch (C ABI cp3_batch_*)."""
 from __future__ import annotations
 
 import ctypes as C

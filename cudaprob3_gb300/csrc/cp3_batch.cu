@@ -3,7 +3,7 @@
 // A batch holds atmospheric problems (one Earth model and production height for the batch,
 // each problem with its own cosine and energy grid) and beam problems (own energies, density
 // and one or more baselines), each with its own oscillation parameters and neutrino type.
-// One run is one or two launches of a persistent kernel, captured once in a CUDA graph:
+// One run is one or two launches of a persistent kernel:
 //
 //   * the grid is (SMs x resident blocks); every warp pulls tiles from an atomic counter;
 //   * tiles [0, A) build the per-(class, energy) eigen tables of the atmospheric problems,
@@ -16,7 +16,8 @@
 //     warps holding them are running and the wait ends; it is bounded all the same (status
 //     flag on time-out).  The serving loop uses this form;
 //   * everything a run needs -- descriptors, tile prefix sums, parameters -- is in device
-//     memory, so the captured graph replays unchanged while parameters change between runs.
+//     memory, changed parameters by one copy before the launches; the kernel leaves its
+//     counters cleared for the next run and its status word is in host memory.
 //
 // The tile shape (rows_per_tile, blocks per SM, beam_chunk) and the split do not change any
 // bin's arithmetic: results are bit-identical across them, which lets an autotuner pick by
@@ -102,27 +103,29 @@ struct cp3_batch {
     Buf<int> d_astart, d_bstart;
     Buf<Header> d_hdr;
     Buf<OscParams> d_params;
-    Buf<int> d_row_off, d_done, d_status;
+    Buf<int> d_row_off, d_done;
     Buf<float2> d_energies, d_cls_rho, d_seg_len, d_baselines;
     Buf<float> d_tables, d_out;
     Buf<unsigned int> d_counter;
     OscParams* h_params = nullptr;  // pinned staging
+    int* h_status = nullptr;        // the last run's status word, in page-locked memory
     bool params_dirty = true;
+    bool counters_dirty = false;    // the last run did not leave the counters zero
 
     int rows_per_tile = 2, blocks_per_sm = 0, beam_chunk = 4;
     bool split_tables = true;      // tables and bins as two launches (cp3_batch_set_split_tables)
     bool withhold_tables = false;  // testing aid: cp3_batch_debug_withhold_tables
     long long total_a = 0, total_b = 0;
-    cudaGraphExec_t graph = nullptr;
     cudaEvent_t ev_params = nullptr, ev0 = nullptr, ev1 = nullptr;
     bool timed = false;
     bool ran = false;  // ev1 marks the end of a run
 
-    // What a run in pieces (cp3_batch_run_to_host) launches directly: the kernel arguments,
-    // the problem mix, the grids of the table and bin instances, the bin-tile prefix sums;
-    // set by every configure.
+    // What a run launches: the kernel arguments, the problem mix, whether tables and bins are
+    // two launches, the grids of the single launch and of the table and bin instances, the
+    // bin-tile prefix sums; set by every configure.
     Args args{};
-    int kinds = 0, grid_tab = 1, grid_bins = 1;
+    bool split = false;
+    int kinds = 0, grid_all = 1, grid_tab = 1, grid_bins = 1;
     std::vector<int> bstart;
     // The copy stream of a run in pieces, an event per piece, and the end of its copies.
     cudaStream_t copy_stream = nullptr;
@@ -134,11 +137,11 @@ struct cp3_batch {
         cudaSetDevice(device);
         if (stream) cudaStreamSynchronize(stream);
         if (copy_stream) cudaStreamSynchronize(copy_stream);
-        if (graph) cudaGraphExecDestroy(graph);
         for (cudaEvent_t e : {ev_params, ev0, ev1, ev_copied})
             if (e) cudaEventDestroy(e);
         for (cudaEvent_t e : ev_piece) cudaEventDestroy(e);
         if (h_params) cudaFreeHost(h_params);
+        if (h_status) cudaFreeHost(h_status);
         if (copy_stream) cudaStreamDestroy(copy_stream);
         if (stream) cudaStreamDestroy(stream);
     }
@@ -196,7 +199,7 @@ int batch_kinds(const std::vector<Problem>& probs) {
     return launch_kinds(a, b);
 }
 
-// Tile counts for the current shape, the device header and the graph.
+// Tile counts for the current shape, the device header and the launches.
 int configure(cp3_batch* b) {
     const int n = (int)b->probs.size();
     std::vector<long long> a(n + 1, 0), bb(n + 1, 0);
@@ -225,54 +228,26 @@ int configure(cp3_batch* b) {
     const int kinds = batch_kinds(b->probs);
     // (a run in pieces launches the table and bin instances separately, split or not)
     int occ = 0, occ_tab = 0, occ_bins = 0;
-    if (occupancy(kinds, &occ, split ? kPhaseBins : kPhaseAll) || occ < 1 ||
-        occupancy(kinds, &occ_bins, kPhaseBins) || occ_bins < 1 ||
+    if (occupancy(kinds, &occ, kPhaseAll) || occ < 1 || occupancy(kinds, &occ_bins, kPhaseBins) || occ_bins < 1 ||
         (a[n] > 0 && (occupancy(kinds, &occ_tab, kPhaseTables) || occ_tab < 1)))
         return bfail(b, CP3_ERR_CUDA, "occupancy query failed");
-    const int bps = b->blocks_per_sm > 0 ? std::min(b->blocks_per_sm, occ) : occ;
-    const int grid = std::max(1, b->sms * bps);
-    // The table launch needs no more warps than it has tiles.
-    const long long tab_blocks = (a[n] + kBlock / 32 - 1) / (kBlock / 32);
-    const int grid_tab = (int)std::max(1LL, std::min<long long>((long long)b->sms * occ_tab, tab_blocks));
-    Args args{b->d_hdr.ptr, b->d_probs.ptr, b->d_astart.ptr, b->d_bstart.ptr, b->d_params.ptr,
-              b->d_energies.ptr, b->d_row_off.ptr, b->d_seg_len.ptr,
-              b->d_cls_rho.ptr, b->d_baselines.ptr, b->d_tables.ptr, b->d_out.ptr,
-              b->d_done.ptr, b->d_counter.ptr, b->d_status.ptr,
-              (long long)b->d_tables.n, (long long)b->d_out.n, (long long)b->d_seg_len.n,
-              (long long)b->d_energies.n};
-    b->args = args;
+    // No launch needs more warps than it has tiles.
+    auto grid = [&](int resident, long long tiles) {
+        const int bps = b->blocks_per_sm > 0 ? std::min(b->blocks_per_sm, resident) : resident;
+        return (int)std::max(1LL, std::min((long long)b->sms * bps, (tiles + kBlock / 32 - 1) / (kBlock / 32)));
+    };
+    b->args = Args{b->d_hdr.ptr, b->d_probs.ptr, b->d_astart.ptr, b->d_bstart.ptr, b->d_params.ptr,
+                   b->d_energies.ptr, b->d_row_off.ptr, b->d_seg_len.ptr,
+                   b->d_cls_rho.ptr, b->d_baselines.ptr, b->d_tables.ptr, b->d_out.ptr,
+                   b->d_done.ptr, b->d_counter.ptr, b->h_status,
+                   (long long)b->d_tables.n, (long long)b->d_out.n, (long long)b->d_seg_len.n,
+                   (long long)b->d_energies.n};
     b->kinds = kinds;
-    b->grid_tab = grid_tab;
-    b->grid_bins = std::max(1, b->sms * std::min(bps, occ_bins));
+    b->split = split;
+    b->grid_all = grid(occ, h.total_a + (long long)h.total_b);
+    b->grid_tab = (int)std::max(1LL, std::min<long long>((long long)b->sms * occ_tab, (a[n] + kBlock / 32 - 1) / (kBlock / 32)));
+    b->grid_bins = grid(occ_bins, bb[n]);
     b->bstart = bi;
-    if (b->graph) {
-        cudaGraphExecDestroy(b->graph);
-        b->graph = nullptr;
-    }
-    cudaStream_t cs;
-    B_CUDA(b, cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking), "capture stream");
-    cudaGraph_t g;
-    cudaError_t e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
-    if (e == cudaSuccess) e = cudaMemsetAsync(b->d_counter.ptr, 0, 2 * sizeof(unsigned int), cs);
-    if (e == cudaSuccess) e = cudaMemsetAsync(b->d_done.ptr, 0, sizeof(int) * std::max(n, 1), cs);
-    if (e == cudaSuccess) e = cudaMemsetAsync(b->d_status.ptr, 0, sizeof(int), cs);
-    if (e == cudaSuccess && split) {
-        kernel_for(kinds, kPhaseTables)<<<grid_tab, kBlock, 0, cs>>>(args);
-        e = cudaGetLastError();
-        if (e == cudaSuccess) {
-            kernel_for(kinds, kPhaseBins)<<<grid, kBlock, 0, cs>>>(args);
-            e = cudaGetLastError();
-        }
-    } else if (e == cudaSuccess) {
-        kernel_for(kinds)<<<grid, kBlock, 0, cs>>>(args);
-        e = cudaGetLastError();
-    }
-    const cudaError_t e2 = cudaStreamEndCapture(cs, &g);
-    if (e == cudaSuccess) e = e2;
-    if (e == cudaSuccess) e = cudaGraphInstantiate(&b->graph, g, 0);
-    if (e2 == cudaSuccess) cudaGraphDestroy(g);
-    cudaStreamDestroy(cs);
-    if (e != cudaSuccess) return bcuda(b, e, "graph capture");
     return CP3_OK;
 }
 
@@ -348,8 +323,7 @@ int commit(cp3_batch* b) {
     B_CUDA(b, b->d_tables.alloc(tab), "allocate eigen tables");
     B_CUDA(b, b->d_out.alloc(out), "allocate results");
     B_CUDA(b, b->d_done.alloc(n), "allocate");
-    B_CUDA(b, b->d_status.alloc(1), "allocate");
-    B_CUDA(b, b->d_counter.alloc(2), "allocate");
+    B_CUDA(b, b->d_counter.alloc(kCounters), "allocate");
     B_CUDA(b, b->d_probs.upload(b->probs, b->stream), "upload");
     B_CUDA(b, b->d_energies.upload(energies, b->stream), "upload");
     B_CUDA(b, b->d_cls_rho.upload(cls_rho, b->stream), "upload");
@@ -359,20 +333,42 @@ int commit(cp3_batch* b) {
     if (b->h_params) cudaFreeHost(b->h_params);
     b->h_params = nullptr;
     B_CUDA(b, cudaMallocHost(&b->h_params, sizeof(OscParams) * n), "pinned parameters");
+    if (!b->h_status) B_CUDA(b, cudaMallocHost(&b->h_status, sizeof(int)), "pinned status");
+    *b->h_status = 0;
     for (int p = 0; p < n; p++) build_osc_params(b->hp[p].mix, b->hp[p].type, b->h_params + p);
     b->params_dirty = true;
+    B_CUDA(b, cudaMemsetAsync(b->d_counter.ptr, 0, kCounters * sizeof(unsigned int), b->stream), "reset");
+    B_CUDA(b, cudaMemsetAsync(b->d_done.ptr, 0, sizeof(int) * n, b->stream), "reset");
     B_CUDA(b, cudaStreamSynchronize(b->stream), "commit");
     b->committed = true;
     return configure(b);
 }
 
-int upload_params(cp3_batch* b, cudaStream_t s) {
+// The start of a run: the parameters, if they changed, and the status word.  The counters are
+// zero where the last run's launches left them so.
+int begin_run(cp3_batch* b, bool clears, cudaStream_t s) {
     if (b->params_dirty) {
         B_CUDA(b, cudaMemcpyAsync(b->d_params.ptr, b->h_params, sizeof(OscParams) * b->probs.size(),
                                   cudaMemcpyHostToDevice, s), "upload parameters");
         B_CUDA(b, cudaEventRecord(b->ev_params, s), "event");
         b->params_dirty = false;
     }
+    if (b->counters_dirty || !clears) {
+        B_CUDA(b, cudaMemsetAsync(b->d_counter.ptr, 0, kCounters * sizeof(unsigned int), s), "reset");
+        B_CUDA(b, cudaMemsetAsync(b->d_done.ptr, 0, sizeof(int) * b->probs.size(), s), "reset");
+    }
+    b->counters_dirty = true;  // until the run's last launch is queued
+    *(volatile int*)b->h_status = 0;
+    return CP3_OK;
+}
+
+// A run belongs to no capture: its parameters are uploaded as they change, and the next run is
+// ordered after it by its events.
+int refuse_capture(cp3_batch* b, cudaStream_t s) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    B_CUDA(b, cudaStreamIsCapturing(s, &cap), "stream");
+    if (cap != cudaStreamCaptureStatusNone)
+        return bfail(b, CP3_ERR_UNSUPPORTED, "a batch's run cannot be captured");
     return CP3_OK;
 }
 
@@ -388,10 +384,20 @@ int order_after_last_run(cp3_batch* b, cudaStream_t s) {
 int launch(cp3_batch* b, cudaStream_t s) {
     if (!b->committed) return bfail(b, CP3_ERR_NOT_SET, "cp3_batch_commit first");
     B_CUDA(b, cudaSetDevice(b->device), "cudaSetDevice");
+    if (int rc = refuse_capture(b, s)) return rc;
     if (int rc = order_after_last_run(b, s)) return rc;
-    if (int rc = upload_params(b, s)) return rc;
+    const bool clears = b->split || clears_counters(b->kinds, kPhaseAll);
+    if (int rc = begin_run(b, clears, s)) return rc;
     B_CUDA(b, cudaEventRecord(b->ev0, s), "event");
-    B_CUDA(b, cudaGraphLaunch(b->graph, s), "graph launch");
+    if (b->split) {
+        kernel_for(b->kinds, kPhaseTables)<<<b->grid_tab, kBlock, 0, s>>>(b->args);
+        B_CUDA(b, cudaGetLastError(), "table launch");
+        kernel_for(b->kinds, kPhaseBins)<<<b->grid_bins, kBlock, 0, s>>>(b->args);
+    } else {
+        kernel_for(b->kinds)<<<b->grid_all, kBlock, 0, s>>>(b->args);
+    }
+    B_CUDA(b, cudaGetLastError(), "launch");
+    b->counters_dirty = !clears;
     B_CUDA(b, cudaEventRecord(b->ev1, s), "event");
     b->timed = b->ran = true;
     return CP3_OK;
@@ -435,13 +441,10 @@ int run_to_host(cp3_batch* b, float* dst, int n_pieces, cudaStream_t s) {
         if (p < n) cut.push_back(p);
     }
     cut.push_back(n);
+    if (int rc = refuse_capture(b, s)) return rc;
     if (int rc = order_after_last_run(b, s)) return rc;
-    if (int rc = upload_params(b, s)) return rc;
+    if (int rc = begin_run(b, true, s)) return rc;
     B_CUDA(b, cudaEventRecord(b->ev0, s), "event");
-    // the resets the captured run does, then the launches of its split form
-    B_CUDA(b, cudaMemsetAsync(b->d_counter.ptr, 0, 2 * sizeof(unsigned int), s), "reset");
-    B_CUDA(b, cudaMemsetAsync(b->d_done.ptr, 0, sizeof(int) * std::max(n, 1), s), "reset");
-    B_CUDA(b, cudaMemsetAsync(b->d_status.ptr, 0, sizeof(int), s), "reset");
     if (b->total_a > 0) {
         kernel_for(b->kinds, kPhaseTables)<<<b->grid_tab, kBlock, 0, s>>>(b->args);
         B_CUDA(b, cudaGetLastError(), "table launch");
@@ -451,7 +454,6 @@ int run_to_host(cp3_batch* b, float* dst, int n_pieces, cudaStream_t s) {
         Args a = b->args;
         a.bin_lo = b->bstart[p0];
         a.bin_hi = b->bstart[p1];
-        B_CUDA(b, cudaMemsetAsync(b->d_counter.ptr + 1, 0, sizeof(unsigned int), s), "reset");
         kernel_for(b->kinds, kPhaseBins)<<<b->grid_bins, kBlock, 0, s>>>(a);
         B_CUDA(b, cudaGetLastError(), "bin launch");
         B_CUDA(b, cudaEventRecord(b->ev_piece[i], s), "event");
@@ -460,6 +462,7 @@ int run_to_host(cp3_batch* b, float* dst, int n_pieces, cudaStream_t s) {
         B_CUDA(b, cudaMemcpyAsync(dst + lo, b->d_out.ptr + lo, (hi - lo) * sizeof(float), cudaMemcpyDefault,
                                   b->copy_stream), "copy results");
     }
+    b->counters_dirty = false;
     B_CUDA(b, cudaEventRecord(b->ev1, s), "event");
     B_CUDA(b, cudaEventRecord(b->ev_copied, b->copy_stream), "event");
     b->downloads = true;
@@ -590,8 +593,10 @@ int cp3_batch_set_params(cp3_batch* b, int id, double t12, double t13, double t2
     H.type = neutrino_type;
     H.params_set = true;
     if (b->committed) {
-        // the previous upload from the staging area must have left before it is rewritten
-        B_CUDA(b, cudaEventSynchronize(b->ev_params), "event");
+        // the last run's upload from the staging area must have ended before it is rewritten; once
+        // one problem's parameters have been, no other upload can have begun (waiting for the
+        // event again for each of a batch's problems cost 1.5 us a problem)
+        if (!b->params_dirty) B_CUDA(b, cudaEventSynchronize(b->ev_params), "event");
         build_osc_params(H.mix, H.type, b->h_params + id);
         b->params_dirty = true;
     }
@@ -674,8 +679,7 @@ int cp3_batch_synchronize(cp3_batch* b, double* ms) {
         B_CUDA(b, cudaEventElapsedTime(&f, b->ev0, b->ev1), "elapsed");
         *ms = f;
     }
-    int st = 0;
-    B_CUDA(b, cudaMemcpy(&st, b->d_status.ptr, sizeof(int), cudaMemcpyDeviceToHost), "status");
+    const int st = *(volatile int*)b->h_status;
     if (st == kStatusWaitLimit)
         return bfail(b, CP3_ERR_CUDA, "batch kernel: eigen tables did not complete (wait limit)");
     if (st == kStatusBounds)

@@ -63,9 +63,10 @@ struct Args {
     const float2* baselines;
     float* tables;
     float* out;
-    int* done_a;
-    unsigned int* counter;
-    int* status;
+    int* done_a;               // nprob: finished table tiles (kPhaseAll launches; cleared before)
+    unsigned int* counter;     // kCounters: next table / only tile, next bin tile, finished warps
+                               // (zero before a run: see clears_counters)
+    int* status;               // in page-locked host memory
     // Element counts of the arenas, read only by the bounds checks of CP3_DEVICE_CHECKS builds.
     long long n_tables, n_out, n_seg, n_energies;
     // The bin tiles a kPhaseBins launch runs, counted from the first bin tile:
@@ -74,10 +75,15 @@ struct Args {
     int bin_lo = 0, bin_hi = 0x7fffffff;
 };
 
+constexpr int kCounters = 3;
+
 // Status words the kernel can leave: a wait that ran out, a tile of a kind the instance was
 // not built for, and (CP3_DEVICE_CHECKS builds) a tile whose accesses would have left an
 // arena, which is then skipped.
 constexpr int kStatusWaitLimit = 1, kStatusKind = 2, kStatusBounds = 3;
+
+// Rare: a plain store to the host's word (the end of the kernel makes it visible there).
+__device__ __forceinline__ void report(int* status, int code) { *(volatile int*)status = code; }
 
 __device__ __forceinline__ unsigned long long global_timer_ns() {
     unsigned long long t;
@@ -136,6 +142,14 @@ CP3_HD int launch_kinds(bool has_atmos, bool has_beam) {
 // counter 1 kPhaseBins launches.
 constexpr int kPhaseTables = 1, kPhaseBins = 2, kPhaseAll = 3;
 
+// Whether a launch leaves the counters cleared (its last warp does), so that the next run needs
+// no memset before it: the launches that end a run, except the single launch with tables, where
+// the code for it cost spills and 1.5 %; that form is cleared by memsets as it needs for its
+// done-counts anyway.
+CP3_HD constexpr bool clears_counters(int kinds, int phases) {
+    return phases == kPhaseBins || (phases == kPhaseAll && kinds == kBeam);
+}
+
 // 72 registers per thread, 7 blocks per SM: measured 1-2 % faster on the batched atmospheric
 // and beam workloads than 64 registers (8 blocks), which spill more; 6 blocks is slower.  The
 // kPhaseBins instance fits 72 registers without spills; 64 or 56 (8 or 9 blocks) measured
@@ -182,7 +196,7 @@ static __global__ void __launch_bounds__(kBlock, 7) batch_kernel(const Args a) {
 
         if (ph == 0) {
             if (!(kKinds & kAtmos)) {  // cannot happen: the host picks kKinds from the problems
-                if (lane == 0) atomicExch(a.status, kStatusKind);
+                if (lane == 0) report(a.status, kStatusKind);
                 break;
             }
             // ---- eigen-table tile: one class x 32 energies ----------------------------
@@ -193,9 +207,9 @@ static __global__ void __launch_bounds__(kBlock, 7) batch_kernel(const Args a) {
             if (!(c >= 0 && c < P.ncls && span_ok(P.e_off, P.ne, a.n_energies) &&
                   span_ok(P.tab_off, (long long)P.ncls * P.ne_pad * kMixFields, a.n_tables) &&
                   P.ne <= P.ne_pad)) {
-                if (lane == 0) atomicExch(a.status, kStatusBounds);
+                if (lane == 0) report(a.status, kStatusBounds);
                 __syncwarp();
-                if (lane == 0) atomicAdd(a.done_a + p, 1);  // no waiter is left hanging
+                if (kPhases == kPhaseAll && lane == 0) atomicAdd(a.done_a + p, 1);  // no waiter is left hanging
                 t = __shfl_sync(0xffffffffu, next, 0);
                 continue;
             }
@@ -207,12 +221,14 @@ static __global__ void __launch_bounds__(kBlock, 7) batch_kernel(const Args a) {
                 store_table_entry(a.tables + P.tab_off + ((size_t)c * P.ne_pad + e) * kMixFields,
                                   u, om);
             }
-            __threadfence();
-            __syncwarp();
-            if (lane == 0) atomicAdd(a.done_a + p, 1);
+            if (kPhases == kPhaseAll) {
+                __threadfence();
+                __syncwarp();
+                if (lane == 0) atomicAdd(a.done_a + p, 1);
+            }
         } else if (P.kind == 0) {
             if (!(kKinds & kAtmos)) {
-                if (lane == 0) atomicExch(a.status, kStatusKind);
+                if (lane == 0) report(a.status, kStatusKind);
                 break;
             }
             // ---- atmospheric bin tile: rows_per_tile rows x 32 energies ------------------
@@ -227,7 +243,7 @@ static __global__ void __launch_bounds__(kBlock, 7) batch_kernel(const Args a) {
                     while (*done < need) {
                         __nanosleep(256);
                         if (++it > kSpinLimit || global_timer_ns() - t0 > kWaitLimitNs) {
-                            atomicExch(a.status, kStatusWaitLimit);  // tables never completed: report
+                            report(a.status, kStatusWaitLimit);  // tables never completed: report
                             break;
                         }
                     }
@@ -255,7 +271,7 @@ static __global__ void __launch_bounds__(kBlock, 7) batch_kernel(const Args a) {
                 tile_ok = tile_ok && nseg >= 1 && nseg <= kMaxSegments && nseg <= P.ncls &&
                           span_ok(s0, nseg, a.n_seg);
                 if (!tile_ok) {
-                    if (lane == 0) atomicExch(a.status, kStatusBounds);
+                    if (lane == 0) report(a.status, kStatusBounds);
                     break;
                 }
 #endif
@@ -271,7 +287,7 @@ static __global__ void __launch_bounds__(kBlock, 7) batch_kernel(const Args a) {
             }
         } else {
             if (!(kKinds & kBeam)) {
-                if (lane == 0) atomicExch(a.status, kStatusKind);
+                if (lane == 0) report(a.status, kStatusKind);
                 break;
             }
             // ---- beam tile: beam_chunk x 32 energies, every baseline --------------------
@@ -281,7 +297,7 @@ static __global__ void __launch_bounds__(kBlock, 7) batch_kernel(const Args a) {
 #ifdef CP3_DEVICE_CHECKS
             if (!(span_ok(P.out_off, 9LL * P.nrows * P.ne, a.n_out) &&
                   span_ok(P.e_off, P.ne, a.n_energies))) {
-                if (lane == 0) atomicExch(a.status, kStatusBounds);
+                if (lane == 0) report(a.status, kStatusBounds);
                 t = __shfl_sync(0xffffffffu, next, 0);
                 continue;
             }
@@ -296,6 +312,13 @@ static __global__ void __launch_bounds__(kBlock, 7) batch_kernel(const Args a) {
             }
         }
         t = __shfl_sync(0xffffffffu, next, 0);
+    }
+    if (clears_counters(kKinds, kPhases)) {
+        // Every warp that has counted itself here has its last tile index.
+        unsigned int finished = 0;
+        if (lane == 0) finished = atomicAdd(a.counter + 2, 1u);
+        if (__shfl_sync(0xffffffffu, finished, 0) == gridDim.x * kWarps - 1 && (int)lane < kCounters)
+            a.counter[lane] = 0;
     }
 }
 

@@ -10,9 +10,8 @@
 // class densities) are registered once and stay resident; each request's eigen table and
 // result live in a device pool until the client releases the request.  A host callback on the
 // stream stamps the completion time and the status of every request of a launch: the
-// launch's graph clears the kernel's status word first and copies it into page-locked host
-// memory last, so the callback reads it without a CUDA call.  A launch whose CUDA calls fail
-// fails its own requests (cp3_server_wait reports the error, cp3_server_result refuses the
+// kernel's status word is in page-locked host memory, so the callback reads it without a CUDA
+// call.  A launch whose CUDA calls fail fails its own requests (cp3_server_wait reports the error, cp3_server_result refuses the
 // result) and no others.
 #include <cuda_runtime.h>
 
@@ -47,9 +46,6 @@ int64_t now_ns() {
 constexpr size_t kUnit = 64;  // pool granularity in floats (256 bytes)
 constexpr int kServeRows = 2;       // tile shape of the serving launches: cosine rows per tile
 constexpr int kServeBeamChunk = 2;  // and 32-energy groups per beam tile
-// Launches with atmospheric requests run as a table launch and a bin launch (see
-// capture_slot).
-constexpr bool kServeSplitTables = true;
 
 // x as a float pair (hi, lo), hi + lo = x to ~48 bits.
 float2 split_pair(double x) {
@@ -140,23 +136,31 @@ struct Request {
     std::atomic<int> state{kQueued};
 };
 
+// Where the parts of a launch of n requests lie in its stage, in 16-byte words.
+struct StageLayout {
+    size_t a, b, probs, params, words;
+    explicit StageLayout(int n) {
+        auto after = [](size_t at, size_t bytes) { return at + (bytes + 15) / 16; };
+        a = after(0, sizeof(Header));
+        b = after(a, sizeof(int) * ((size_t)n + 1));
+        probs = after(b, sizeof(int) * ((size_t)n + 1));
+        params = after(probs, sizeof(Problem) * (size_t)n);
+        words = after(params, sizeof(OscParams) * (size_t)n);
+    }
+};
+
 struct Slot {
     struct cp3_server* owner = nullptr;
     cudaStream_t stream = nullptr;
-    cudaGraphExec_t graph[4] = {nullptr, nullptr, nullptr, nullptr};  // by launch kinds (1..3)
-    DBuf<Problem> d_probs;
-    DBuf<int> d_a, d_b;
-    DBuf<Header> d_hdr;
-    DBuf<OscParams> d_params;
-    DBuf<int> d_done, d_status;
+    // A launch's header, tile prefix sums, problems and parameters, packed one after the other
+    // (StageLayout) and brought to the device by one copy.
+    HBuf<uint4> h_stage;
+    DBuf<uint4> d_stage;
     DBuf<unsigned int> d_counter;
-    HBuf<Problem> h_probs;
-    HBuf<int> h_a, h_b;
-    HBuf<Header> h_hdr;
-    HBuf<OscParams> h_params;
-    HBuf<int> h_status;  // the launch's status word, copied back by the graph's last node
+    HBuf<int> h_status;  // the launch's status word
     std::vector<std::shared_ptr<Request>> reqs;
     bool busy = false;
+    bool counters_dirty = true;  // the counters are not known to be zero
     std::atomic<int> finished{0};
 };
 
@@ -198,6 +202,7 @@ struct cp3_server {
     bool started = false;
     std::atomic<long long> launches{0}, completed{0};
     std::string launch_error;      // the last failed launch's CUDA error (under mu)
+    int grid_tab[4] = {1, 1, 1, 1}, grid_bins[4] = {1, 1, 1, 1};  // resident blocks by launch kinds
     int debug_fail_launches = 0;   // testing aid: cp3_server_debug_fail_launches (under mu)
 
     // completion queue for cp3_server_poll: ids in completion order, recorded once a client
@@ -253,11 +258,11 @@ void finish_requests(cp3_server* s, const std::vector<std::shared_ptr<Request>>&
 }
 
 // Host callback after a slot's launch: every request of the launch is done, with the status
-// word the launch's graph copied into page-locked memory before this callback (stream order).
+// word the launch left in page-locked memory before this callback (stream order).
 // It takes no lock of the scheduler's: the scheduler may hold cp3_server::mu while it waits.
 void CUDART_CB on_launch_done(void* user) {
     Slot* slot = static_cast<Slot*>(user);
-    finish_requests(slot->owner, slot->reqs, *slot->h_status.ptr);
+    finish_requests(slot->owner, slot->reqs, *(volatile int*)slot->h_status.ptr);
     slot->finished.store(1);
     slot->owner->cv.notify_all();
 }
@@ -269,13 +274,27 @@ const char* status_text(int st) {
                                     : "the launch of this request failed";
 }
 
-// Packs queued requests into one launch on `slot`; caller holds s->mu.  Order: requests
+// The kernels of a launch by the problem kinds it holds: tables where there are atmospheric
+// requests, then the bins (a beam-only launch is the single kernel).
+using ServeKernel = void (*)(Args);
+ServeKernel table_kernel(int kinds) {
+    return kinds == kAtmos ? batch_kernel<kAtmos, kPhaseTables> : batch_kernel<kBoth, kPhaseTables>;
+}
+ServeKernel bin_kernel(int kinds) {
+    return kinds == kBeam    ? batch_kernel<kBeam>
+           : kinds == kAtmos ? batch_kernel<kAtmos, kPhaseBins>
+                             : batch_kernel<kBoth, kPhaseBins>;
+}
+
+// Packs queued requests into one launch on `slot`; the caller holds s->mu through `lk`, which is
+// let go of while the launch's CUDA calls are made (clients submit meanwhile: the slot and its
+// requests, admitted and not done, are the scheduler's alone).  Order: requests
 // older than the aging limit first (arrival order), then the rest smallest-first, so small
 // requests are not stuck behind large ones and large ones cannot starve.  A request is
 // admitted only if its table and result fit in the pool (admission by device memory).
 // Requests of one grid have one size, so when a grid's oldest request does not fit (pool or
 // the launch's bin cap), none of that grid's does, and the grid is passed over.
-void launch_slot(cp3_server* s, Slot& slot) {
+void launch_slot(cp3_server* s, Slot& slot, std::unique_lock<std::mutex>& lk) {
     TraceRange trace("serve_launch");
     slot.reqs.clear();
     const int64_t now = now_ns();
@@ -314,7 +333,14 @@ void launch_slot(cp3_server* s, Slot& slot) {
     if (slot.reqs.empty()) return;
     const int n = (int)slot.reqs.size();
     long long a = 0, b = 0;
-    slot.h_a.ptr[0] = slot.h_b.ptr[0] = 0;
+    const StageLayout L(n);
+    uint4* const stage = slot.h_stage.ptr;
+    int* const h_a = reinterpret_cast<int*>(stage + L.a);
+    int* const h_b = reinterpret_cast<int*>(stage + L.b);
+    Problem* const h_probs = reinterpret_cast<Problem*>(stage + L.probs);
+    OscParams* const h_params = reinterpret_cast<OscParams*>(stage + L.params);
+    h_a[0] = h_b[0] = 0;
+    bool has_atmos = false, has_beam = false;
     const int64_t t0 = now_ns();
     for (int i = 0; i < n; i++) {
         Request& r = *slot.reqs[i];
@@ -333,54 +359,80 @@ void launch_slot(cp3_server* s, Slot& slot) {
         P.out_off = P.tab_off + (long long)T.tab_floats;
         P.rho_e[0] = T.rho_e[0];
         P.rho_e[1] = T.rho_e[1];
-        slot.h_probs.ptr[i] = P;
-        slot.h_params.ptr[i] = r.params;
+        h_probs[i] = P;
+        h_params[i] = r.params;
+        (T.kind == 0 ? has_atmos : has_beam) = true;
         long long na = 0, nb = 0;
         problem_tiles(P, kServeRows, kServeBeamChunk, &na, &nb);
         a += na;
         b += nb;
-        slot.h_a.ptr[i + 1] = (int)a;  // < kMaxTiles: a launch holds at most max_bins bins
-        slot.h_b.ptr[i + 1] = (int)b;  // besides its first request, and requests fit the pool
+        h_a[i + 1] = (int)a;  // < kMaxTiles: a launch holds at most max_bins bins
+        h_b[i + 1] = (int)b;  // besides its first request, and requests fit the pool
         r.t_start = t0;
         r.state.store(kRunning);
     }
-    *slot.h_hdr.ptr = Header{n, kServeRows, kServeBeamChunk, (int)a, (int)b};
+    *reinterpret_cast<Header*>(stage) = Header{n, kServeRows, kServeBeamChunk, (int)a, (int)b};
     cudaStream_t st = slot.stream;
-    bool has_atmos = false, has_beam = false;
-    for (int i = 0; i < n; i++) (slot.h_probs.ptr[i].kind == 0 ? has_atmos : has_beam) = true;
     slot.finished.store(0);
+    *slot.h_status.ptr = 0;
     s->launches++;
     // Every call is checked.  A launch that fails before its host callback is queued fails
     // its own requests here, after its stream has drained (so no kernel of it can still
     // write into pool memory that a release hands to the next request).
     cudaError_t e = cudaSuccess;
     const char* what = "";
-    bool graph_queued = false;
+    bool queued = false;
     if (s->debug_fail_launches > 0) {
         s->debug_fail_launches--;
         e = cudaErrorLaunchFailure;
         what = "injected launch failure (cp3_server_debug_fail_launches)";
     }
+    lk.unlock();
 #define SERVE_STEP(call, name)        \
     if (e == cudaSuccess) {           \
         e = (call);                   \
         if (e != cudaSuccess) what = name; \
     }
-    SERVE_STEP(cudaMemcpyAsync(slot.d_probs.ptr, slot.h_probs.ptr, sizeof(Problem) * n, cudaMemcpyHostToDevice, st), "upload problems")
-    SERVE_STEP(cudaMemcpyAsync(slot.d_params.ptr, slot.h_params.ptr, sizeof(OscParams) * n, cudaMemcpyHostToDevice, st), "upload parameters")
-    SERVE_STEP(cudaMemcpyAsync(slot.d_a.ptr, slot.h_a.ptr, sizeof(int) * (n + 1), cudaMemcpyHostToDevice, st), "upload tile offsets")
-    SERVE_STEP(cudaMemcpyAsync(slot.d_b.ptr, slot.h_b.ptr, sizeof(int) * (n + 1), cudaMemcpyHostToDevice, st), "upload tile offsets")
-    SERVE_STEP(cudaMemcpyAsync(slot.d_hdr.ptr, slot.h_hdr.ptr, sizeof(Header), cudaMemcpyHostToDevice, st), "upload header")
-    SERVE_STEP(cudaGraphLaunch(slot.graph[launch_kinds(has_atmos, has_beam)], st), "graph launch")
-    graph_queued = e == cudaSuccess;
+    // One copy brings the stage over; then the single kernel, or with atmospheric requests a
+    // table launch and a bin launch that reads the finished tables (no wait).  No launch has
+    // more warps than tiles.
+    uint4* const dev = slot.d_stage.ptr;
+    const Args args{reinterpret_cast<const Header*>(dev), reinterpret_cast<const Problem*>(dev + L.probs),
+                    reinterpret_cast<const int*>(dev + L.a), reinterpret_cast<const int*>(dev + L.b),
+                    reinterpret_cast<const OscParams*>(dev + L.params),
+                    s->d_energies.ptr, s->d_row_off.ptr, s->d_seg_len.ptr,
+                    s->d_cls_rho.ptr, s->d_baselines.ptr, s->d_pool.ptr, s->d_pool.ptr,
+                    nullptr, slot.d_counter.ptr, slot.h_status.ptr,
+                    (long long)s->d_pool.n, (long long)s->d_pool.n, (long long)s->d_seg_len.n,
+                    (long long)s->d_energies.n};
+    const int kinds = launch_kinds(has_atmos, has_beam);
+    auto grid = [](int full, long long tiles) {
+        return (int)std::max(1LL, std::min((long long)full, (tiles + kBlock / 32 - 1) / (kBlock / 32)));
+    };
+    if (slot.counters_dirty) {  // the slot's first launch, or one after a failed one
+        SERVE_STEP(cudaMemsetAsync(slot.d_counter.ptr, 0, kCounters * sizeof(unsigned int), st), "reset")
+    }
+    slot.counters_dirty = true;  // until the launch is queued
+    SERVE_STEP(cudaMemcpyAsync(dev, stage, L.words * sizeof(uint4), cudaMemcpyHostToDevice, st), "upload")
+    queued = e == cudaSuccess;
+    auto run = [&](ServeKernel k, int blocks) {
+        k<<<blocks, kBlock, 0, st>>>(args);
+        return cudaGetLastError();
+    };
+    if (has_atmos) SERVE_STEP(run(table_kernel(kinds), grid(s->grid_tab[kinds], a)), "table launch")
+    SERVE_STEP(run(bin_kernel(kinds), grid(s->grid_bins[kinds], b)), "bin launch")
     SERVE_STEP(cudaLaunchHostFunc(st, on_launch_done, &slot), "completion callback")
 #undef SERVE_STEP
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        if (queued) cudaStreamSynchronize(st);
+    }
+    lk.lock();
     if (e == cudaSuccess) {
         slot.busy = true;
+        slot.counters_dirty = false;
         return;
     }
-    cudaGetLastError();
-    if (graph_queued) cudaStreamSynchronize(st);
     s->launch_error = std::string("serve launch: ") + what + ": " + cudaGetErrorString(e);
     finish_requests(s, slot.reqs, kReqLaunchFailed);
     slot.reqs.clear();
@@ -400,7 +452,7 @@ void scheduler(cp3_server* s) {
         bool launched = false;
         for (Slot& sl : s->slots)
             if (!sl.busy && s->queued > 0) {
-                launch_slot(s, sl);
+                launch_slot(s, sl, lk);
                 launched = launched || sl.busy;
             }
         // Nothing launchable (slots busy, queue empty, or the pool full until a release):
@@ -411,71 +463,24 @@ void scheduler(cp3_server* s) {
     }
 }
 
-int capture_slot(cp3_server* s, Slot& sl) {
+int make_slot(cp3_server* s, Slot& sl) {
     const int cap = s->max_batch;
     S_CUDA(s, cudaStreamCreateWithFlags(&sl.stream, cudaStreamNonBlocking), "stream");
-    S_CUDA(s, sl.d_probs.alloc(cap), "allocate");
-    S_CUDA(s, sl.d_a.alloc(cap + 1), "allocate");
-    S_CUDA(s, sl.d_b.alloc(cap + 1), "allocate");
-    S_CUDA(s, sl.d_hdr.alloc(1), "allocate");
-    S_CUDA(s, sl.d_params.alloc(cap), "allocate");
-    S_CUDA(s, sl.d_done.alloc(cap), "allocate");
-    S_CUDA(s, sl.d_status.alloc(1), "allocate");
-    S_CUDA(s, sl.d_counter.alloc(2), "allocate");
-    S_CUDA(s, sl.h_probs.alloc(cap), "pinned");
-    S_CUDA(s, sl.h_a.alloc(cap + 1), "pinned");
-    S_CUDA(s, sl.h_b.alloc(cap + 1), "pinned");
-    S_CUDA(s, sl.h_hdr.alloc(1), "pinned");
-    S_CUDA(s, sl.h_params.alloc(cap), "pinned");
+    S_CUDA(s, sl.d_stage.alloc(StageLayout(cap).words), "allocate");
+    S_CUDA(s, sl.d_counter.alloc(kCounters), "allocate");
+    S_CUDA(s, sl.h_stage.alloc(StageLayout(cap).words), "pinned");
     S_CUDA(s, sl.h_status.alloc(1), "pinned");
     *sl.h_status.ptr = 0;
-    Args args{sl.d_hdr.ptr, sl.d_probs.ptr, sl.d_a.ptr, sl.d_b.ptr, sl.d_params.ptr,
-              s->d_energies.ptr, s->d_row_off.ptr, s->d_seg_len.ptr,
-              s->d_cls_rho.ptr, s->d_baselines.ptr, s->d_pool.ptr, s->d_pool.ptr,
-              sl.d_done.ptr, sl.d_counter.ptr, sl.d_status.ptr,
-              (long long)s->d_pool.n, (long long)s->d_pool.n, (long long)s->d_seg_len.n,
-              (long long)s->d_energies.n};
-    // One graph per set of problem kinds; a launch replays the one for the kinds it holds.
-    // With atmospheric requests it is a table launch, then a bin launch that reads the
-    // finished tables (no wait); a beam-only launch is the single kernel.  The table launch
-    // has a full grid: the number of table tiles changes from launch to launch, and warps
-    // without a tile return at once.  Each graph clears the status word first and copies it
-    // to the slot's page-locked word last, where the completion callback reads it.
+    return CP3_OK;
+}
+
+int resident_grids(cp3_server* s) {
     for (int kinds = 1; kinds <= 3; kinds++) {
-        using Kern = void (*)(Args);
-        const bool split = kServeSplitTables && (kinds & kAtmos);
-        const Kern tab = kinds == kAtmos ? batch_kernel<kAtmos, kPhaseTables> : batch_kernel<kBoth, kPhaseTables>;
-        const Kern kern = !split ? (kinds == kBeam ? batch_kernel<kBeam> : kinds == kAtmos ? batch_kernel<kAtmos>
-                                                                                           : batch_kernel<kBoth>)
-                                 : (kinds == kAtmos ? batch_kernel<kAtmos, kPhaseBins> : batch_kernel<kBoth, kPhaseBins>);
-        int occ = 0, occ_tab = 0;
-        S_CUDA(s, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kBlock, 0), "occupancy");
-        if (split) S_CUDA(s, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_tab, tab, kBlock, 0), "occupancy");
-        const int grid = std::max(1, s->sms * std::max(occ, 1));
-        const int grid_tab = std::max(1, s->sms * std::max(occ_tab, 1));
-        cudaStream_t cs;
-        S_CUDA(s, cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking), "capture stream");
-        cudaGraph_t g;
-        cudaError_t e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
-        if (e == cudaSuccess) e = cudaMemsetAsync(sl.d_counter.ptr, 0, 2 * sizeof(unsigned int), cs);
-        if (e == cudaSuccess) e = cudaMemsetAsync(sl.d_done.ptr, 0, sizeof(int) * cap, cs);
-        if (e == cudaSuccess) e = cudaMemsetAsync(sl.d_status.ptr, 0, sizeof(int), cs);
-        if (e == cudaSuccess && split) {
-            tab<<<grid_tab, kBlock, 0, cs>>>(args);
-            e = cudaGetLastError();
-        }
-        if (e == cudaSuccess) {
-            kern<<<grid, kBlock, 0, cs>>>(args);
-            e = cudaGetLastError();
-        }
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(sl.h_status.ptr, sl.d_status.ptr, sizeof(int), cudaMemcpyDeviceToHost, cs);
-        const cudaError_t e2 = cudaStreamEndCapture(cs, &g);
-        if (e == cudaSuccess) e = e2;
-        if (e == cudaSuccess) e = cudaGraphInstantiate(&sl.graph[kinds], g, 0);
-        if (e2 == cudaSuccess) cudaGraphDestroy(g);
-        cudaStreamDestroy(cs);
-        if (e != cudaSuccess) return scuda(s, e, "graph capture");
+        int occ = 0;
+        S_CUDA(s, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, bin_kernel(kinds), kBlock, 0), "occupancy");
+        s->grid_bins[kinds] = std::max(1, s->sms * std::max(occ, 1));
+        S_CUDA(s, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, table_kernel(kinds), kBlock, 0), "occupancy");
+        s->grid_tab[kinds] = std::max(1, s->sms * std::max(occ, 1));
     }
     return CP3_OK;
 }
@@ -497,8 +502,6 @@ cp3_server::~cp3_server() {
     cudaSetDevice(device);
     for (Slot& sl : slots) {
         if (sl.stream) cudaStreamSynchronize(sl.stream);
-        for (cudaGraphExec_t gx : sl.graph)
-            if (gx) cudaGraphExecDestroy(gx);
         if (sl.stream) cudaStreamDestroy(sl.stream);
     }
 }
@@ -627,8 +630,9 @@ int cp3_server_start(cp3_server* s) {
     for (const Template& T : s->tmpls)
         if ((T.tab_floats + T.out_floats) / kUnit > units)
             return sfail(s, CP3_ERR_BAD_SIZE, "a registered grid does not fit in the pool");
+    if (int rc = resident_grids(s)) return rc;
     for (Slot& sl : s->slots)
-        if (int rc = capture_slot(s, sl)) return rc;
+        if (int rc = make_slot(s, sl)) return rc;
     s->queues.assign(s->tmpls.size(), {});
     s->by_size.resize(s->tmpls.size());
     for (size_t g = 0; g < s->tmpls.size(); g++) s->by_size[g] = (int)g;

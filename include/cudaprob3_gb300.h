@@ -231,8 +231,7 @@ int cp3_kernel_times(cp3_propagator* h, double* eigen_ms, double* bins_ms);
  * problems (one Earth model and production height per batch, own cosine/energy grid each)
  * and beam problems (own energies, density and baselines), each with its own oscillation
  * parameters and neutrino type, computed in MIXED precision by one persistent kernel
- * replayed from a CUDA graph (one launch, or a table launch and a bin launch: see
- * cp3_batch_set_split_tables).  Results stay on the device:
+ * (one launch, or a table launch and a bin launch: see cp3_batch_set_split_tables).  Results stay on the device:
  *   atmospheric problem  [9][n_cosines][n_energies] floats
  *   beam problem         [n_baselines][9][n_energies] floats */
 typedef struct cp3_batch cp3_batch;
@@ -254,7 +253,7 @@ int cp3_batch_add_beam(cp3_batch* b, const double* energies, int n_energies, dou
 int cp3_batch_set_params(cp3_batch* b, int id, double theta12, double theta13, double theta23,
                          double dcp, int knutype, double dm12sq, double dm23sq,
                          int neutrino_type);
-/* Freezes the problem list: trajectories, device arenas, the CUDA graph. */
+/* Freezes the problem list: trajectories, device arenas, the launches. */
 int cp3_batch_commit(cp3_batch* b);
 /* Tile shape of the persistent kernel (results do not depend on it): cosine rows per
  * atmospheric tile (1..16; a tile is 32 energies), resident blocks per SM (0 = as many as
@@ -335,7 +334,7 @@ int cp3_server_add_atmos_grid(cp3_server* s, const double* cosines, int n_cosine
                               const double* energies, int n_energies, int* grid);
 int cp3_server_add_beam_grid(cp3_server* s, const double* energies, int n_energies, double rho,
                              const double* path_km, int n_baselines, int* grid);
-/* Uploads the grids, allocates the pool, captures the launch graphs, starts the loop. */
+/* Uploads the grids, allocates the pool and the launch slots, starts the loop. */
 int cp3_server_start(cp3_server* s);
 int cp3_server_submit(cp3_server* s, int grid, double theta12, double theta13, double theta23,
                       double dcp, int knutype, double dm12sq, double dm23sq, int neutrino_type,
