@@ -154,9 +154,13 @@ CP3_HD constexpr bool clears_counters(int kinds, int phases) {
 // and beam workloads than 64 registers (8 blocks), which spill more; 6 blocks is slower.  The
 // kPhaseBins instance fits 72 registers without spills; 64 or 56 (8 or 9 blocks) measured
 // no faster on the batched atmospheric workload.
+// The beam-only instance takes 80 registers, 6 blocks per SM: its polynomial solve spills at
+// 72 (64 problems x 2 baselines x 1e5 energies, runs among others: 142 us; with 7, 5 and 4
+// blocks 146, 149 and 151).  It is bound by the issue of its ~650 instructions an energy, of
+// which a packed one takes two slots.
 // Internal linkage: each translation unit that launches it (batches, the server) has its own.
 template <int kKinds, int kPhases = kPhaseAll>
-static __global__ void __launch_bounds__(kBlock, 7) batch_kernel(const Args a) {
+static __global__ void __launch_bounds__(kBlock, kKinds == kBeam ? 6 : 7) batch_kernel(const Args a) {
     constexpr int kWarps = kBlock / 32;
     constexpr int kTableLoad = kPhases == kPhaseBins ? kLoadReadOnly : kLoadL2;
     __shared__ float2 s_len[kWarps][kMaxSegments];  // one trajectory per warp
@@ -302,13 +306,19 @@ static __global__ void __launch_bounds__(kBlock, 7) batch_kernel(const Args a) {
                 continue;
             }
 #endif
-            for (int k = 0; k < hdr.beam_chunk; k++) {
-                const long long e = e0 + (long long)k * kTileE + lane;
-                if (e < P.ne) {
-                    const float2 E2 = a.energies[P.e_off + e];
-                    beam_bin_mixed(prm, w, df{E2.x, E2.y}, rho, a.baselines + P.row_off, P.nrows,
-                                   a.out + P.out_off + e, (size_t)P.ne, (size_t)9 * P.ne);
-                }
+            // A group's energies are loaded while the group before is worked on: waited for at
+            // their use, they held a warp up for a third of its time (a run alone 200 us against
+            // 191).
+            const float2* en = a.energies + P.e_off;
+            long long e = e0 + lane;
+            float2 E2 = e < P.ne ? __ldg(en + e) : make_float2(0.f, 0.f);
+            for (int k = 0; k < hdr.beam_chunk && e < P.ne; k++) {
+                const long long e_next = e + kTileE;
+                const float2 E2n = k + 1 < hdr.beam_chunk && e_next < P.ne ? __ldg(en + e_next) : E2;
+                beam_bin_mixed(prm, w, df{E2.x, E2.y}, rho, a.baselines + P.row_off, P.nrows,
+                               a.out + P.out_off + e, (size_t)P.ne, (size_t)9 * P.ne);
+                e = e_next;
+                E2 = E2n;
             }
         }
         t = __shfl_sync(0xffffffffu, next, 0);

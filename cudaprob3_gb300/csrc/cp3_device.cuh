@@ -269,20 +269,28 @@ CP3_HD df df_mulf(df x, float y) {
     const float e = fmaf(x.hi, y, -p);
     return df_fast2sum(p, fmaf(x.lo, y, e));
 }
-// 1 / x to df64 accuracy: float reciprocal, then one Newton step in df64.
+// 1 / x to df64 accuracy from a float estimate r: with e = 1 - x r (its leading part exact
+// through the FMA), 1 / x = r (1 + e + e^2), to e^3 ~ 2^-66.  The approximate reciprocal is
+// enough as the estimate (8 operations; the divide and a Newton step in df64 arithmetic took
+// 50, 5 % of a beam energy's).
 CP3_HD df df_recip(df x) {
+#ifdef __CUDA_ARCH__
+    const float r = __fdividef(1.0f, x.hi);
+#else
     const float r = 1.0f / x.hi;
-    const df one_minus = df_sub(df{1.0f, 0.0f}, df_mulf(x, r));  // 1 - x r, small
-    return df_add(df{r, 0.0f}, df_mulf(one_minus, r));
+#endif
+    const float e = fmaf(-x.lo, r, fmaf(-x.hi, r, 1.0f));
+    return df_fast2sum(r, CP3_FMUL(r, fmaf(e, e, e)));
 }
 
 #ifdef __CUDACC__
 // ---------------------------------------------------------------------------------------
 // Paired FP32.  sm_100+ executes FFMA2 / FMUL2 / FADD2: one instruction, two independent
-// FP32 lanes, each rounded exactly as fmaf / __fmul_rn / __fadd_rn.  On GB300 the FMA pipe
-// retires paired and scalar FMAs at the same FLOP rate, so pairing does not add arithmetic
-// throughput; it halves the issue slots of the paired work, and issue is what binds the
-// mixed kernels.  Lanes pair independent computations: the real and imaginary parts of a
+// FP32 lanes, each rounded exactly as fmaf / __fmul_rn / __fadd_rn.  On GB300 a paired FMA
+// takes the issue and the pipe of two scalar ones (measured cycles a warp and sub-partition:
+// FFMA2 2.4, two FFMA 2.0; with an independent logic operation 3.4 and 3.1), so pairing adds no
+// throughput; it halves the instructions and their operand fetches.  What binds the mixed
+// kernels is the number of lane operations.  Lanes pair independent computations: the real and imaginary parts of a
 // complex entry, the two phases of a layer, the two refined roots, the two projectors.
 
 __device__ __forceinline__ float2 bc2(float x) { return make_float2(x, x); }
@@ -318,6 +326,11 @@ __device__ __forceinline__ df2 df2_mul(const df2& x, const df2& y) {
     float2 e = __ffma2_rn(x.hi, y.hi, neg2(p));
     e = __ffma2_rn(x.hi, y.lo, __ffma2_rn(x.lo, y.hi, e));
     return df2_fast2sum(p, e);
+}
+// the same for a factor of one float
+__device__ __forceinline__ df2 df2_mulf(const df2& x, float2 y) {
+    const float2 p = __fmul2_rn(x.hi, y);
+    return df2_fast2sum(p, __ffma2_rn(x.lo, y, __ffma2_rn(x.hi, y, neg2(p))));
 }
 #endif
 
@@ -483,20 +496,22 @@ __device__ __forceinline__ bool rotated_eigen_mixed_try(const OscParams* __restr
     df2 x{make_float2(l0, l1), bc2(0.0f)};
     {
         const df2 C2 = df2_bc(c2), C1 = df2_bc(c1), C0 = df2_bc(c0);
-        auto newton = [&]() {
-            const df2 f = df2_sub(df2_mul(df2_add(df2_mul(df2_sub(x, C2), x), C1), x), C0);
+        auto step = [&](const df2& f) {
             const float2 d = __ffma2_rn(__ffma2_rn(bc2(3.0f), x.hi, bc2(-2.0f * c2.hi)), x.hi,
                                         bc2(c1.hi));
-            x = df2_sub(x, df2{make_float2(__fdividef(f.hi.x, d.x), __fdividef(f.hi.y, d.y)), bc2(0.0f)});
+            return make_float2(__fdividef(-f.hi.x, d.x), __fdividef(-f.hi.y, d.y));
         };
-        newton();
-        bool again = kDf;
-        if (!kDf) {
-            const float m2 = c2.hi - x.hi.x - x.hi.y;
-            const float d01 = fabsf(x.hi.x - x.hi.y), d02 = fabsf(x.hi.x - m2),
-                        d12 = fabsf(x.hi.y - m2);
-            again = !(fminf(d01, fminf(d02, d12)) > 0.05f * fmaxf(d01, fmaxf(d02, d12)));
-        }
+        auto newton = [&]() {
+            const df2 f = df2_sub(df2_mul(df2_add(df2_mul(df2_sub(x, C2), x), C1), x), C0);
+            x = df2_add(x, df2{step(f), bc2(0.0f)});
+        };
+        // The first step starts from floats: products with one float, and the sum of the root
+        // and its small correction in order of size.
+        const df2 f = df2_sub(df2_mulf(df2_add(df2_mulf(df2_sub(x, C2), x.hi), C1), x.hi), C0);
+        x = df2_fast2sum(x.hi, step(f));
+        // gap > 0.05 spread on the starting roots: sin(th) > 0.05 sin(th + pi/3), or the same of
+        // pi/3 - th
+        const bool again = kDf || !(th > 0.045f && th < 1.0471976f - 0.045f);
         if (again) newton();
     }
     df r[3] = {df2_x(x), df2_y(x), df{0.0f, 0.0f}};

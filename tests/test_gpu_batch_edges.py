@@ -78,3 +78,28 @@ def test_a_run_cannot_be_captured():
     b.run()
     b.synchronize()
     assert np.abs(b.result(0).sum(axis=1) - 3.0).max() < 1e-4  # three initial flavours
+
+
+MIXED_TOL = 1e-5  # the mixed path's bound against the oracle
+
+
+@pytest.mark.parametrize("chunk", [1, 2, 3, 4, 64])
+def test_beam_tile_edges(oracle, chunk):
+    """A beam tile loads a group's energies one group ahead: problems that end inside, at and
+    just after a group and a tile, every energy against the oracle."""
+    from oracle.oracle import Mixing as OMix
+    sizes = (1, 31, 32, 33, 32 * chunk - 1, 32 * chunk, 32 * chunk + 1)
+    b = Batch(0)
+    m = earth.gaussian_sets(1, seed=4)[0]
+    om = OMix(m.theta12, m.theta13, m.theta23, m.dcp, m.dm12sq, m.dm23sq, 1)
+    grids = [np.linspace(0.2, 9.0, n) if n > 1 else np.array([0.7]) for n in sizes]
+    for en in grids:
+        b.set_params(b.add_beam(en, 2.6, [295.0, 1300.0]), m, False)
+    b.set_shape(beam_chunk=chunk)
+    b.commit()
+    b.run()
+    b.synchronize()
+    for i, en in enumerate(grids):
+        got = b.result(i)
+        for j, L in enumerate((295.0, 1300.0)):
+            assert np.abs(got[j].T - oracle.beam(om, False, en, 2.6, L)).max() <= MIXED_TOL
