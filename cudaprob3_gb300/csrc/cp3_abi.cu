@@ -428,11 +428,33 @@ int launch(cp3_propagator* h, int type, cudaStream_t s, void* host_dst = nullptr
         const int fx_classes = fx ? h->ncls_used : 1;
         if (!mixed)
             CP3_CUDA(h, h->d_table_fx.reserve(table_fx_words(fx_classes, h->ne)), "allocate eigen table");
+        const bool tables = !mixed || !h->model.poly;
+        // The row pieces of a download.  The first one is half the size of the others, so that
+        // the link starts sooner (measured 1.5 % off the 59-shell 2000 x 2000 step against
+        // equal pieces).
+        const size_t plane = (size_t)h->nc * h->ne * esz, row = (size_t)h->ne * esz;
+        std::vector<int> cuts{0};
+        int np = 0;
+        bool same = false;  // the same pieces as the last download: each waits for its own copy
+        if (host_dst) {
+            const int chunks = std::max(1, std::min(n_chunks, h->nc));
+            const long long den = 2LL * chunks - 1;
+            for (int c = 0; c < chunks; c++) {
+                const int r1 = (int)((long long)h->nc * (2 * c + 1) / den);
+                if (r1 > cuts.back()) cuts.push_back(r1);
+            }
+            np = (int)cuts.size() - 1;
+            e = ensure_copy_events(h, np);
+            same = cuts == h->copy_rows;
+            // (a single piece waits before its table, so that nothing lies between the two)
+            if (e == cudaSuccess && !same && !h->copy_rows.empty()) e = cudaStreamWaitEvent(s, h->ev_copied, 0);
+            if (e == cudaSuccess && same && np == 1) e = cudaStreamWaitEvent(s, h->ev_piece_copied[0], 0);
+        }
         mark(0);
-        if (!mixed)
+        if (e == cudaSuccess && !mixed)
             e = launch_table_fx(p, h->d_energies.ptr, h->ne, h->d_cls_rho.ptr, fx_classes,
                                 h->d_table_fx.ptr, s);
-        else if (!h->model.poly)
+        else if (e == cudaSuccess && !h->model.poly)
             e = launch_table_mixed(p, h->d_energies_df.ptr, h->ne, h->d_cls_rho_df.ptr,
                                    h->ncls_used, h->d_table32.ptr, s);
         mark(1);
@@ -463,30 +485,15 @@ int launch(cp3_propagator* h, int type, cudaStream_t s, void* host_dst = nullptr
                                           !h->model.poly, h->nc, av, (double*)h->d_result.ptr, s, rr);
         };
         if (!host_dst) {
-            if (e == cudaSuccess) e = bins(RowRange{});
+            // (with an event between the two launches, for the profile, the second one waits)
+            if (e == cudaSuccess) e = bins(RowRange{0, -1, tables && !profile});
         } else {
             // each piece: rows [r0, r1) of all 9 channel planes, one 2-D copy on the copy
-            // stream once the piece is computed.  The first piece is half the size of the
-            // others, so that the link starts sooner (measured 1.5 % off the 59-shell
-            // 2000 x 2000 step against equal pieces).
-            const int chunks = std::max(1, std::min(n_chunks, h->nc));
-            const size_t plane = (size_t)h->nc * h->ne * esz, row = (size_t)h->ne * esz;
-            const long long den = 2LL * chunks - 1;
-            std::vector<int> cuts{0};
-            for (int c = 0; c < chunks; c++) {
-                const int r1 = (int)((long long)h->nc * (2 * c + 1) / den);
-                if (r1 > cuts.back()) cuts.push_back(r1);
-            }
-            const int np = (int)cuts.size() - 1;
-            if (e == cudaSuccess) e = ensure_copy_events(h, np);
-            // the same row pieces as the last download: each waits for its own copy
-            const bool same = cuts == h->copy_rows;
-            if (e == cudaSuccess && !same && !h->copy_rows.empty())
-                e = cudaStreamWaitEvent(s, h->ev_copied, 0);
+            // stream once the piece is computed
             for (int c = 0; c < np && e == cudaSuccess; c++) {
                 const int r0 = cuts[c], r1 = cuts[c + 1];
-                if (same) e = cudaStreamWaitEvent(s, h->ev_piece_copied[c], 0);
-                if (e == cudaSuccess) e = bins(RowRange{r0, r1});
+                if (same && np > 1) e = cudaStreamWaitEvent(s, h->ev_piece_copied[c], 0);
+                if (e == cudaSuccess) e = bins(RowRange{r0, r1, c == 0 && tables && (np == 1 || !same)});
                 if (e == cudaSuccess) e = cudaEventRecord(h->ev_piece[c], s);
                 if (e == cudaSuccess) e = cudaStreamWaitEvent(h->copy_stream, h->ev_piece[c], 0);
                 if (e == cudaSuccess)

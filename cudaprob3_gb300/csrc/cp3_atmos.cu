@@ -283,6 +283,7 @@ __global__ void __launch_bounds__(32 * kFxWarps, 4)
         for (int i = lane; i < nseg; i += 32) s_len[wv][i] = seg_len[s0 + i];
     }
     __syncthreads();
+    wait_for_previous();
     const int ie = blockIdx.x * 32 + lane;
     if (ic >= ic1 || ie >= ne) return;
     const FxColumn col{table + ie, table + (size_t)ncls * kFxFields * ne_pad + ie, (size_t)ne_pad,
@@ -341,11 +342,14 @@ __global__ void __launch_bounds__(32 * kFxWarps, 3)
     __syncthreads();
     if (ic >= ic1 || ie >= ne) return;
     const double E = energies[ie];
-    const FxAir air = load_air(table, ne_pad, ie, nseg == 1);
     double* o = out + (size_t)ic * ne + ie;
+    auto load = [&]() {
+        wait_for_previous();
+        return load_air(table, ne_pad, ie, nseg == 1);
+    };
     auto solve = [&](int l, FxClass& k) { fx_solve(&p, E, s_rho[wv][l], k); };
     long long P[4];
-    if (fx_bin_inline(solve, air, fx_w(p.w), s_len[wv], nseg - 1, s_trig, P))
+    if (fx_bin_inline(solve, load, fx_w(p.w), s_len[wv], nseg - 1, s_trig, P))
         fx_store(P, o, (size_t)nc * ne);
     else
         atmos_bin_out_of_range(&p, E, s_len[wv], s_rho[wv], nseg - 1, AvgInput{}, ic, nc, ie, ne, o);
@@ -380,6 +384,7 @@ __global__ void __launch_bounds__(32 * kFxWarps, 4)
     unsigned int bad = 0;
     const int first = nseg > 1 ? 1 : 0;  // of the warps that sum
     if (wv >= first && on) {
+        wait_for_previous();
         const FxColumn col{table + ie, nullptr, (size_t)ne_pad, 0};
         const double rate[2] = {col.rate(0, 0), col.rate(0, 1)};
         const size_t cell = (size_t)ic * av.nb;
@@ -398,9 +403,12 @@ __global__ void __launch_bounds__(32 * kFxWarps, 4)
     cfx a[2][3];
     if (wv == 0 && on) {
         E = energies[ie];
-        const FxAir air = load_air(table, ne_pad, ie, false);
+        auto load = [&]() {
+            wait_for_previous();
+            return load_air(table, ne_pad, ie, false);
+        };
         auto solve = [&](int l, FxClass& k) { fx_solve(&p, E, s_rho[l], k); };
-        fx_air_rows(solve, air, fx_w(p.w), s_len, nseg - 1, s_trig, bad, a);
+        fx_air_rows(solve, load, fx_w(p.w), s_len, nseg - 1, s_trig, bad, a);
     }
     __syncthreads();
     if (wv > 0 || !on) return;
@@ -448,9 +456,10 @@ __global__ void __launch_bounds__(kBlockMixed)
     const int nseg = seg_off[ic + 1] - s0;
     for (int i = threadIdx.x; i < nseg; i += kBlockMixed) s_len[i] = seg_len[s0 + i];
     __syncthreads();
+    wait_for_previous();
     const int ie = blockIdx.x * kBlockMixed + threadIdx.x;
     if (ie >= ne) return;
-    atmos_bin_mixed(table + (size_t)ie * kMixFields, (size_t)kMixFields * ne_pad, s_len, nseg - 1,
+    atmos_bin_mixed<kLoadCached>(table + (size_t)ie * kMixFields, (size_t)kMixFields * ne_pad, s_len, nseg - 1,
                     w, out + (size_t)ic * ne + ie, (size_t)nc * ne);
 }
 
@@ -504,11 +513,11 @@ cudaError_t launch_atmos_fx_inline(const OscParams& p, const double* energies, i
         const int ic1 = end - ic0 < step ? end : ic0 + step;
         dim3 grid((ne + 31) / 32, (ic1 - ic0 + rows - 1) / rows);
         if (averaged)
-            atmos_fx_avg_kernel<<<grid, 32 * kFxWarps, 0, s>>>(p, energies, ne, pad_energies(ne), table, seg_off,
-                                                               seg_len, rho, per_class, ic0, n_cosines, av, out);
+            launch_early(rr.early && ic0 == rr.begin, atmos_fx_avg_kernel, grid, 32 * kFxWarps, s, p, energies, ne,
+                         pad_energies(ne), table, seg_off, seg_len, rho, per_class, ic0, n_cosines, av, out);
         else
-            atmos_fx_inline_kernel<<<grid, 32 * kFxWarps, 0, s>>>(p, energies, ne, pad_energies(ne), table, seg_off,
-                                                                  seg_len, rho, ic0, ic1, n_cosines, out);
+            launch_early(rr.early && ic0 == rr.begin, atmos_fx_inline_kernel, grid, 32 * kFxWarps, s, p, energies, ne,
+                         pad_energies(ne), table, seg_off, seg_len, rho, ic0, ic1, n_cosines, out);
     }
     return cudaGetLastError();
 }
@@ -522,8 +531,8 @@ cudaError_t launch_atmos_fx(const OscParams& p, const double* energies, int ne, 
     for (int ic0 = rr.begin; ic0 < end; ic0 += step) {
         const int ic1 = end - ic0 < step ? end : ic0 + step;
         dim3 grid((ne + 31) / 32, (ic1 - ic0 + kFxWarps - 1) / kFxWarps);
-        atmos_fx_kernel<<<grid, 32 * kFxWarps, 0, s>>>(p, energies, ne, pad_energies(ne), table, cls_rho,
-                                                       ncls, seg_off, seg_len, ic0, ic1, n_cosines, out);
+        launch_early(rr.early && ic0 == rr.begin, atmos_fx_kernel, grid, 32 * kFxWarps, s, p, energies, ne,
+                     pad_energies(ne), table, cls_rho, ncls, seg_off, seg_len, ic0, ic1, n_cosines, out);
     }
     return cudaGetLastError();
 }
@@ -538,8 +547,8 @@ cudaError_t launch_atmos_mixed(const OscParams& p, const float* table, int ne,
     for (int ic0 = rr.begin; ic0 < end; ic0 += kMaxGridY) {
         const int rows = end - ic0 < kMaxGridY ? end - ic0 : kMaxGridY;
         dim3 grid((ne + kBlockMixed - 1) / kBlockMixed, rows);
-        atmos_mixed_kernel<<<grid, kBlockMixed, 0, s>>>(w, table, ne, ne_pad, seg_off, seg_len,
-                                                   ic0, n_cosines, out);
+        launch_early(rr.early && ic0 == rr.begin, atmos_mixed_kernel, grid, kBlockMixed, s, w, table, ne, ne_pad,
+                     seg_off, seg_len, ic0, n_cosines, out);
     }
     return cudaGetLastError();
 }
@@ -705,15 +714,16 @@ __global__ void __launch_bounds__(kBlock)
     const int nseg = seg_off[ic + 1] - s0;
     for (int i = threadIdx.x; i < nseg; i += kBlock) s_len[i] = seg_len[s0 + i];
     __syncthreads();
+    wait_for_previous();
     const int ie = blockIdx.x * kBlock + threadIdx.x;
     if (ie >= ne) return;
     const float* tab = table + (size_t)ie * kMixFields;
     const size_t cls_stride = (size_t)kMixFields * ne_pad;
-    auto seg = [&](int l, Layer& F) { layer_from_table(tab + l * cls_stride, s_len[l], F); };
+    auto seg = [&](int l, Layer& F) { layer_from_table<kLoadCached>(tab + l * cls_stride, s_len[l], F); };
     Layer F0;
     const float* t0 = tab;  // class 0: the air
-    layer_from_table(t0, s_len[0], F0);
-    const df om1{__ldg(t0 + 6), __ldg(t0 + 8)}, om2{__ldg(t0 + 7), __ldg(t0 + 9)};
+    layer_from_table<kLoadCached>(t0, s_len[0], F0);
+    const df om1{__ldca(t0 + 6), __ldca(t0 + 8)}, om2{__ldca(t0 + 7), __ldca(t0 + 9)};
     atmos_bin_mixed_avg(seg, nseg - 1, F0, om1, om2, w, av, ic, nc, ie, ne, out);
 }
 
@@ -760,8 +770,8 @@ cudaError_t launch_atmos_mixed_avg(const OscParams& p, const float* table, int n
     for (int ic0 = rr.begin; ic0 < end; ic0 += kMaxGridY) {
         const int rows = end - ic0 < kMaxGridY ? end - ic0 : kMaxGridY;
         dim3 grid((ne + kBlock - 1) / kBlock, rows);
-        atmos_mixed_avg_kernel<<<grid, kBlock, 0, s>>>(w, table, ne, ne_pad, seg_off, seg_len,
-                                                       ic0, n_cosines, a, out);
+        launch_early(rr.early && ic0 == rr.begin, atmos_mixed_avg_kernel, grid, kBlock, s, w, table, ne, ne_pad,
+                     seg_off, seg_len, ic0, n_cosines, a, out);
     }
     return cudaGetLastError();
 }

@@ -290,8 +290,9 @@ CP3_HD df df_recip(df x) {
 // takes the issue and the pipe of two scalar ones (measured cycles a warp and sub-partition:
 // FFMA2 2.4, two FFMA 2.0; with an independent logic operation 3.4 and 3.1), so pairing adds no
 // throughput; it halves the instructions and their operand fetches.  What binds the mixed
-// kernels is the number of lane operations.  Lanes pair independent computations: the real and imaginary parts of a
-// complex entry, the two phases of a layer, the two refined roots, the two projectors.
+// kernels is the number of lane operations.  Lanes pair independent computations: the real and
+// imaginary parts of a complex entry, the two phases of a layer, the two refined roots, the two
+// projectors.
 
 __device__ __forceinline__ float2 bc2(float x) { return make_float2(x, x); }
 __device__ __forceinline__ float2 neg2(float2 v) { return make_float2(-v.x, -v.y); }

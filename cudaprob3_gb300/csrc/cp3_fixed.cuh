@@ -249,7 +249,7 @@ struct FxColumn {
     size_t stride, cls_stride;
     CP3_HD int2 load(const int2* p) const {
 #ifdef __CUDA_ARCH__
-        return __ldg(p);
+        return __ldca(p);  // (written while this grid is already there: launch_early)
 #else
         return *p;
 #endif
@@ -903,19 +903,21 @@ CP3_HD void fx_chain(Solve solve, const double* len, int M, const longlong2* tri
     }
 }
 
-// One bin; false where it needs the FP64 path.
-template <class Solve>
-CP3_HD bool fx_bin_inline(Solve solve, const FxAir& air, const FxW& w, const double* len, int M,
+// One bin; false where it needs the FP64 path.  load() gives the air layer, which is not asked
+// for before the chain of the others is done.
+template <class Solve, class Load>
+CP3_HD bool fx_bin_inline(Solve solve, Load load, const FxW& w, const double* len, int M,
                           const longlong2* trig, long long P[4]) {
     unsigned int bad = 0;
+    FxAmplitude g;
+    if (M > 0) fx_chain(solve, len, M, trig, bad, g);
+    const FxAir air = load();
     cfx e0[2];
     fx_layer(air.rate, len[0], trig, e0, bad);
     if (M == 0) {
         fx_one_layer(air.coef, e0, P);
         return (bad >> 20) == 0;
     }
-    FxAmplitude g;
-    fx_chain(solve, len, M, trig, bad, g);
 #pragma unroll 1
     for (int j = 0; j < 2; j++) {  // initial flavours e, mu: S_0 W^+ column j
         cfx k[3];
@@ -1028,12 +1030,13 @@ CP3_HD void fx_shift_factors(const long long sum[3][3][2], const unsigned long l
         for (int f = 0; f < 3; f++) t[q][f] = cfx{fx_split(sum[q][f][0]), fx_split(sum[q][f][1])};
 }
 
-// The rows e, mu of a_k = W G u_k.
-template <class Solve>
-CP3_HD void fx_air_rows(Solve solve, const FxAir& air, const FxW& w, const double* len, int M,
+// The rows e, mu of a_k = W G u_k; load() as above.
+template <class Solve, class Load>
+CP3_HD void fx_air_rows(Solve solve, Load load, const FxW& w, const double* len, int M,
                         const longlong2* trig, unsigned int& bad, cfx a[2][3]) {
     FxAmplitude g;
     fx_chain(solve, len, M, trig, bad, g);
+    const FxAir air = load();
 #pragma unroll 1
     for (int k = 0; k < 3; k++) {
         cfx v[3];

@@ -43,10 +43,38 @@ struct AvgArrays {
     int n_bins = 0;
 };
 
-// Cosine rows [begin, end) of a result (end < 0: through the last row).
+// Cosine rows [begin, end) of a result (end < 0: through the last row).  early: the launch
+// follows its table's with nothing in between, and may be scheduled while that one runs.
 struct RowRange {
     int begin = 0, end = -1;
+    bool early = false;
 };
+
+#ifdef __CUDACC__
+// Programmatic dependent launch: a table's launch lets the bins' be scheduled as soon as all its
+// blocks run (launch_dependents); the bins stage what the table does not hold and wait for its
+// end before they read it (wait_for_previous; no wait where the launch was an ordinary one).
+// They read it with __ldca: its lines are written during their own grid's life, which the
+// read-only path does not allow for.  A call, before and after: FP64 PREM-4 400 x 400 40.2 and
+// 35.7 us, PREM-12 307 x 811 73 and 68, quadratic 500 x 500 75 and 68 (its bins need the air's
+// table only once their chain of layers is done); mixed PREM-4 200 x 200 to host memory 37 and 32.
+__device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;"); }
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <class... Params, class... Args>
+void launch_early(bool early, void (*kernel)(Params...), dim3 grid, int block, cudaStream_t s, Args... args) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c{};
+    c.gridDim = grid;
+    c.blockDim = dim3(block);
+    c.stream = s;
+    c.attrs = &at;
+    c.numAttrs = early ? 1 : 0;
+    cudaLaunchKernelEx(&c, kernel, Params(args)...);  // the error is read with cudaGetLastError
+}
+#endif
 
 // Atmospheric bins of an n_cosines-row result ([9][n_cosines][ne]), rows rr only.  The
 // trajectory of row i is segments seg_off[i]..seg_off[i+1]-1 (air, then shells inwards); the

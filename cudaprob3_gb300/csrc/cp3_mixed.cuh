@@ -99,8 +99,9 @@ __device__ __forceinline__ void unit_turn_minus_one2_hw(float2 r, float2 lo, flo
 }
 
 // How a kernel reads the eigen table: the read-only path (__ldg) for tables an earlier
-// launch wrote, L2 only (__ldcg) for tables written earlier in the same launch.
-enum TableLoad { kLoadReadOnly = 0, kLoadL2 = 1 };
+// launch wrote, L2 only (__ldcg) for tables written earlier in the same launch, ordinary cached
+// loads (__ldca) for tables whose launch may still run when the kernel is scheduled.
+enum TableLoad { kLoadReadOnly = 0, kLoadL2 = 1, kLoadCached = 2 };
 
 // t points at this bin's 48-byte table entry: u1 (3), u2 (3), then the phase rates
 // omega_1, omega_2 in turns per km (omega / 2 pi) as double-floats, the two high parts side
@@ -114,6 +115,7 @@ template <int kLoad = kLoadReadOnly>
 __device__ __forceinline__ TableEntry load_table_entry(const float* __restrict__ t) {
     const float4* t4 = reinterpret_cast<const float4*>(t);
     if (kLoad == kLoadL2) return TableEntry{__ldcg(t4), __ldcg(t4 + 1), __ldcg(t4 + 2)};
+    if (kLoad == kLoadCached) return TableEntry{__ldca(t4), __ldca(t4 + 1), __ldca(t4 + 2)};
     return TableEntry{__ldg(t4), __ldg(t4 + 1), __ldg(t4 + 2)};
 }
 

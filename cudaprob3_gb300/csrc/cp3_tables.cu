@@ -32,6 +32,7 @@ __global__ void __launch_bounds__(32 * (kFxRun + 1))
                     int ne, int ne_pad, const double* __restrict__ cls_rho, int ncls,
                     int2* __restrict__ table) {
     __shared__ int2 s_u[kFxRun + 1][9][32];
+    launch_dependents();
     const int lane = threadIdx.x & 31, wv = threadIdx.x >> 5;
     const int ie = blockIdx.x * 32 + lane, c = blockIdx.y * kFxRun + wv;
     const bool on = c < ncls && ie < ne;
@@ -87,6 +88,7 @@ __global__ void __launch_bounds__(kTableBlock)
     table_mixed_kernel(const __grid_constant__ OscParams p, const Real* __restrict__ energies,
                        int ne, int ne_pad, const Real* __restrict__ cls_rho,
                        float* __restrict__ table) {
+    launch_dependents();
     const int ie = blockIdx.x * kTableBlock + threadIdx.x;
     const int c = blockIdx.y;
     if (ie >= ne) return;

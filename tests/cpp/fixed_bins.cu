@@ -114,7 +114,7 @@ extern "C" int fixed_inline(const double* mix, int knutype, int anti, const doub
             const size_t plane = (size_t)nc * ne;
             if (nb == 0) {
                 long long P[4];
-                outside += !fx_bin_inline(solve, air, w, len, t.maxlayers[ic], trig, P);
+                outside += !fx_bin_inline(solve, [&]() { return air; }, w, len, t.maxlayers[ic], trig, P);
                 fx_store(P, o, plane);
                 continue;
             }
@@ -139,7 +139,7 @@ extern "C" int fixed_inline(const double* mix, int knutype, int anti, const doub
             cfx f[3][3], rows[2][3];
             long long P[3][2];
             fx_shift_factors(sum, total, bad, f);
-            fx_air_rows(solve, air, w, len, t.maxlayers[ic], trig, bad, rows);
+            fx_air_rows(solve, [&]() { return air; }, w, len, t.maxlayers[ic], trig, bad, rows);
             fx_average(rows, air, w, len[0], trig, f, bad, P);
             outside += (bad >> 20) != 0;
             for (int j = 0; j < 3; j++) {
