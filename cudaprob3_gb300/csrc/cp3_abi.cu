@@ -422,10 +422,10 @@ int launch(cp3_propagator* h, int type, cudaStream_t s, void* host_dst = nullptr
         rc = prepare_averaging(h, &av, &avm);
         if (rc) return rc;
         const bool mixed = h->precision == CP3_MIXED;
-        // FP64: constant densities come from the fixed-point table; quadratic densities and the
-        // averaging solve their layers in place and read only the air's class
+        // FP64: constant densities come from the fixed-point table; quadratic densities solve
+        // their layers in place and read only the air's class
         const bool fx = !mixed && !h->model.poly && av.n_bins == 0;
-        const int fx_classes = fx ? h->ncls_used : 1;
+        const int fx_classes = h->model.poly ? 1 : h->ncls_used;
         if (!mixed)
             CP3_CUDA(h, h->d_table_fx.reserve(table_fx_words(fx_classes, h->ne)), "allocate eigen table");
         const bool tables = !mixed || !h->model.poly;
@@ -482,7 +482,7 @@ int launch(cp3_propagator* h, int type, cudaStream_t s, void* host_dst = nullptr
             return launch_atmos_fx_inline(p, h->d_energies.ptr, h->ne, h->d_table_fx.ptr,
                                           h->d_seg_off.ptr, h->d_seg_len.ptr,
                                           h->model.poly ? h->d_seg_rho.ptr : h->d_cls_rho.ptr,
-                                          !h->model.poly, h->nc, av, (double*)h->d_result.ptr, s, rr);
+                                          h->model.poly ? 0 : fx_classes, h->nc, av, (double*)h->d_result.ptr, s, rr);
         };
         if (!host_dst) {
             // (with an event between the two launches, for the profile, the second one waits)

@@ -355,20 +355,26 @@ __global__ void __launch_bounds__(32 * kFxWarps, 3)
         atmos_bin_out_of_range(&p, E, s_len[wv], s_rho[wv], nseg - 1, AvgInput{}, ic, nc, ie, ne, o);
 }
 
-// Production-height averaging (rho per segment or, per_class, per class).  A block is one row x
-// 32 energies: its first warp runs the chain of layers while the others sum the shift factors of
-// the height bins, a third each (on a row that crosses no shell all four take a quarter) -- the
-// two are independent, and a grid of a few hundred rows and energies leaves the chip half empty
-// with one warp a bin.  PREM-4, 200 x 150, 20 heights:
-// 59 us (688 in FP64 arithmetic with the weights read across energies).
+// Production-height averaging; kTable: the layers from a table (rho per class), else solved in
+// place (rho per segment).  A block is one row x 32 energies: its first warp runs the chain of
+// layers while the others sum the shift factors of the height bins, a third each (on a row that
+// crosses no shell all four take a quarter); then three of them form the probabilities of one
+// initial flavour each.  The parts are independent, and a grid of a few hundred rows and
+// energies leaves the chip half empty with one warp a bin.  Bound by the latency of these
+// chains (ALU 35 %, FP64 33 %, issue 36 %; 1000 blocks on 608 places).  PREM-4, 200 x 150, 20
+// heights: 49 us (688 in FP64 arithmetic with the weights read across energies; 59 with the
+// layers solved in place and one warp for the last part; 53 and 61 with three and five blocks
+// an SM).
+template <bool kTable>
 __global__ void __launch_bounds__(32 * kFxWarps, 4)
     atmos_fx_avg_kernel(const __grid_constant__ OscParams p, const double* __restrict__ energies, int ne,
-                        int ne_pad, const int2* __restrict__ table, const int* __restrict__ seg_off,
-                        const double* __restrict__ seg_len, const double* __restrict__ rho, bool per_class,
+                        int ne_pad, const int2* __restrict__ table, int ncls, const int* __restrict__ seg_off,
+                        const double* __restrict__ seg_len, const double* __restrict__ rho,
                         int ic0, int nc, AvgInput av, double* __restrict__ out) {
     __shared__ longlong2 s_trig[kTrigSize];
     __shared__ double s_len[kMaxSegments], s_rho[kMaxSegments];
     __shared__ long long s_sum[kFxWarps][21][32];
+    __shared__ int2 s_a[12][32];
     __shared__ unsigned int s_bad[kFxWarps][32];
     for (int i = threadIdx.x; i < kTrigSize; i += 32 * kFxWarps)
         s_trig[i] = make_longlong2(g_trig.cs[i][0], g_trig.cs[i][1]);
@@ -377,15 +383,16 @@ __global__ void __launch_bounds__(32 * kFxWarps, 4)
     const int s0 = seg_off[ic], nseg = seg_off[ic + 1] - s0;
     for (int i = threadIdx.x; i < nseg; i += 32 * kFxWarps) {
         s_len[i] = seg_len[s0 + i];
-        s_rho[i] = rho[per_class ? i : s0 + i];
+        s_rho[i] = rho[kTable ? i : s0 + i];
     }
     __syncthreads();
     const bool on = ie < ne;
+    const FxColumn col{table + ie, table + (size_t)ncls * kFxFields * ne_pad + ie, (size_t)ne_pad,
+                       (size_t)kFxFields * ne_pad};
     unsigned int bad = 0;
     const int first = nseg > 1 ? 1 : 0;  // of the warps that sum
     if (wv >= first && on) {
         wait_for_previous();
-        const FxColumn col{table + ie, nullptr, (size_t)ne_pad, 0};
         const double rate[2] = {col.rate(0, 0), col.rate(0, 1)};
         const size_t cell = (size_t)ic * av.nb;
         FxShift sum;
@@ -397,50 +404,64 @@ __global__ void __launch_bounds__(32 * kFxWarps, 4)
 #pragma unroll
             for (int q = 0; q < 6; q++) s_sum[wv][6 * f + q][lane] = sum.value(q >> 1, f, q & 1);
         }
-        s_bad[wv][lane] = bad;
     }
-    double E = 0.0;
-    cfx a[2][3];
     if (wv == 0 && on) {
-        E = energies[ie];
-        auto load = [&]() {
+        cfx a[2][3];
+        if (kTable) {
             wait_for_previous();
-            return load_air(table, ne_pad, ie, false);
-        };
-        auto solve = [&](int l, FxClass& k) { fx_solve(&p, E, s_rho[l], k); };
-        fx_air_rows(solve, load, fx_w(p.w), s_len, nseg - 1, s_trig, bad, a);
+            fx_air_rows(col, s_len, nseg - 1, s_trig, bad, a);
+        } else {
+            const double E = energies[ie];
+            auto load = [&]() {
+                wait_for_previous();
+                return load_air(table, ne_pad, ie, false);
+            };
+            auto solve = [&](int l, FxClass& k) { fx_solve(&p, E, s_rho[l], k); };
+            fx_air_rows(solve, load, fx_w(p.w), s_len, nseg - 1, s_trig, bad, a);
+        }
+#pragma unroll
+        for (int i = 0; i < 6; i++) {
+            const cfx v = a[i / 3][i % 3];
+            s_a[2 * i][lane] = make_int2(v.re.h, v.re.l);
+            s_a[2 * i + 1][lane] = make_int2(v.im.h, v.im.l);
+        }
     }
+    s_bad[wv][lane] = bad;
     __syncthreads();
-    if (wv > 0 || !on) return;
-    long long sum[3][3][2] = {};
+    const int j = wv;  // the initial flavour
+    if (j > 2 || !on) return;
+    bad = 0;
+    long long sum[6] = {};
     unsigned long long total[3] = {};
 #pragma unroll
     for (int k = 0; k < kFxWarps; k++) {
-        if (k < first) continue;
         bad |= s_bad[k][lane];
+        if (k < first) continue;
 #pragma unroll
-        for (int f = 0; f < 3; f++) {
-            total[f] += (unsigned long long)s_sum[k][18 + f][lane];
+        for (int f = 0; f < 3; f++) total[f] += (unsigned long long)s_sum[k][18 + f][lane];
 #pragma unroll
-            for (int q = 0; q < 6; q++) sum[q >> 1][f][q & 1] += s_sum[k][6 * f + q][lane];
-        }
+        for (int q = 0; q < 6; q++) sum[q] += s_sum[k][6 * j + q][lane];
     }
-    cfx t[3][3];
-    fx_shift_factors(sum, total, bad, t);
-    const FxAir air = load_air(table, ne_pad, ie, false);
-    long long P[3][2];
-    fx_average(a, air, fx_w(p.w), s_len[0], s_trig, t, bad, P);
+    fx_check_weights(total, bad);
+    cfx a[2][3], t[3];
+    fx row[9];
+#pragma unroll
+    for (int i = 0; i < 6; i++) a[i / 3][i % 3] = cfx{fx_of(s_a[2 * i][lane]), fx_of(s_a[2 * i + 1][lane])};
+#pragma unroll
+    for (int q = 0; q < 3; q++) t[q] = cfx{fx_split(sum[2 * q]), fx_split(sum[2 * q + 1])};
+#pragma unroll
+    for (int f = 0; f < 9; f++) row[f] = col.extra(kFxV0 + f);
+    const double rate[2] = {col.rate(0, 0), col.rate(0, 1)};
+    long long P[2];
+    fx_average(j, a, row, rate, s_len[0], s_trig, t, bad, P);
     double* o = out + (size_t)ic * ne + ie;
     const size_t plane = (size_t)nc * ne;
     if ((bad >> 20) == 0) {
-#pragma unroll
-        for (int j = 0; j < 3; j++) {
-            o[(size_t)(3 * j) * plane] = fx_to_double(P[j][0]);
-            o[(size_t)(3 * j + 1) * plane] = fx_to_double(P[j][1]);
-            o[(size_t)(3 * j + 2) * plane] = fx_to_double((1LL << 62) - P[j][0] - P[j][1]);
-        }
-    } else {
-        atmos_bin_out_of_range(&p, E, s_len, s_rho, nseg - 1, av, ic, nc, ie, ne, o);
+        o[(size_t)(3 * j) * plane] = fx_to_double(P[0]);
+        o[(size_t)(3 * j + 1) * plane] = fx_to_double(P[1]);
+        o[(size_t)(3 * j + 2) * plane] = fx_to_double((1LL << 62) - P[0] - P[1]);
+    } else if (j == 0) {  // (the three agree on it)
+        atmos_bin_out_of_range(&p, energies[ie], s_len, s_rho, nseg - 1, av, ic, nc, ie, ne, o);
     }
 }
 
@@ -502,7 +523,7 @@ __global__ void __launch_bounds__(kBlock)
 
 cudaError_t launch_atmos_fx_inline(const OscParams& p, const double* energies, int ne,
                                    const int2* table, const int* seg_off, const double* seg_len, const double* rho,
-                                   bool per_class, int n_cosines, const AvgArrays& avg, double* out,
+                                   int ncls, int n_cosines, const AvgArrays& avg, double* out,
                                    cudaStream_t s, RowRange rr) {
     if (ne <= 0 || n_cosines <= 0) return cudaSuccess;
     const AvgInput av{avg.prob, avg.mid, avg.wid, avg.n_bins, p.anti};
@@ -513,8 +534,9 @@ cudaError_t launch_atmos_fx_inline(const OscParams& p, const double* energies, i
         const int ic1 = end - ic0 < step ? end : ic0 + step;
         dim3 grid((ne + 31) / 32, (ic1 - ic0 + rows - 1) / rows);
         if (averaged)
-            launch_early(rr.early && ic0 == rr.begin, atmos_fx_avg_kernel, grid, 32 * kFxWarps, s, p, energies, ne,
-                         pad_energies(ne), table, seg_off, seg_len, rho, per_class, ic0, n_cosines, av, out);
+            launch_early(rr.early && ic0 == rr.begin, ncls > 0 ? atmos_fx_avg_kernel<true> : atmos_fx_avg_kernel<false>,
+                         grid, 32 * kFxWarps, s, p, energies, ne, pad_energies(ne), table, ncls > 0 ? ncls : 1, seg_off,
+                         seg_len, rho, ic0, n_cosines, av, out);
         else
             launch_early(rr.early && ic0 == rr.begin, atmos_fx_inline_kernel, grid, 32 * kFxWarps, s, p, energies, ne,
                          pad_energies(ne), table, seg_off, seg_len, rho, ic0, ic1, n_cosines, out);

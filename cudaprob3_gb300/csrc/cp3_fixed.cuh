@@ -388,6 +388,50 @@ CP3_HD void fx_one_layer(const fx v[13], const cfx e[2], long long P[4]) {
     P[3] = r[1];
 }
 
+// The columns of Y (see fx_bin) for M > 1 table layers; layer(l, e, &det) forms the phases of
+// layer l.
+template <class Layer>
+CP3_HD void fx_columns(const FxColumn& t, int M, Layer layer, const longlong2* trig, cfx y[3][3]) {
+    FxDet det;
+    cfx e[2];
+    layer(1, e, &det);
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        const fx a = t.rot(1, 3 * i), b = t.rot(1, 3 * i + 1);
+        fxacc r, m;
+        fx_mac(r, b, e[0].re);
+        fx_mac(m, b, e[0].im);
+        y[0][i] = cfx{a, fx{0, 0}};
+        y[1][i] = cfx{fx_res(r), fx_res(m)};
+    }
+#pragma unroll 1
+    for (int l = 2; l < M; l++) {
+        fx R[9];
+        fx_load_rotation(t, l, R);
+        layer(l, e, &det);
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            fx_phase(e, y[j]);
+            fx_rotate(R, y[j]);
+        }
+    }
+    fx_third_column(det, trig, y);
+}
+
+// (W U_1) k, rows e and mu: the table's flavour rows of class 1 on a vector in its eigenbasis.
+CP3_HD void fx_rows_of(const FxColumn& t, const cfx k[3], cfx& ae, cfx& am) {
+    fxacc r, m;
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        const fx v = t.extra(kFxV1 + i);
+        fx_mac(r, v, k[i].re);
+        fx_mac(m, v, k[i].im);
+    }
+    ae = cfx{fx_res(r), fx_res(m)};
+    am = fx_cdot(cfx{t.extra(kFxV1 + 3), t.extra(kFxV1 + 6)}, k[0], cfx{t.extra(kFxV1 + 4), t.extra(kFxV1 + 7)}, k[1],
+                 cfx{t.extra(kFxV1 + 5), t.extra(kFxV1 + 8)}, k[2]);
+}
+
 // The four probabilities e->e, e->mu, mu->e, mu->mu (62 fraction bits) of one bin over M + 1
 // segments (lengths len[0..M] in km; segment l is class l); the other five follow from
 // unitarity.  Returns false where a phase left the reduction's range.
@@ -417,31 +461,7 @@ CP3_HD bool fx_bin(const FxColumn& t, const double* len, int M, const longlong2*
         return (bad >> 20) == 0;
     }
     cfx y[3][3];
-    if (M > 1) {
-        FxDet det;
-        layer(1, e, &det);
-#pragma unroll
-        for (int i = 0; i < 3; i++) {
-            const fx a = t.rot(1, 3 * i), b = t.rot(1, 3 * i + 1);
-            fxacc r, m;
-            fx_mac(r, b, e[0].re);
-            fx_mac(m, b, e[0].im);
-            y[0][i] = cfx{a, fx{0, 0}};
-            y[1][i] = cfx{fx_res(r), fx_res(m)};
-        }
-#pragma unroll 1
-        for (int l = 2; l < M; l++) {
-            fx R[9];
-            fx_load_rotation(t, l, R);
-            layer(l, e, &det);
-#pragma unroll
-            for (int j = 0; j < 2; j++) {
-                fx_phase(e, y[j]);
-                fx_rotate(R, y[j]);
-            }
-        }
-        fx_third_column(det, trig, y);
-    }
+    if (M > 1) fx_columns(t, M, layer, trig, y);
     cfx e0[2];
     layer(0, e0, nullptr);
     layer(M, e, nullptr);
@@ -462,18 +482,7 @@ CP3_HD bool fx_bin(const FxColumn& t, const double* len, int M, const longlong2*
         else
             fx_phase(e, k);
         cfx ae, am;
-        {
-            fxacc r, m;
-#pragma unroll
-            for (int i = 0; i < 3; i++) {
-                const fx v = t.extra(kFxV1 + i);
-                fx_mac(r, v, k[i].re);
-                fx_mac(m, v, k[i].im);
-            }
-            ae = cfx{fx_res(r), fx_res(m)};
-        }
-        am = fx_cdot(cfx{t.extra(kFxV1 + 3), t.extra(kFxV1 + 6)}, k[0], cfx{t.extra(kFxV1 + 4), t.extra(kFxV1 + 7)}, k[1],
-                     cfx{t.extra(kFxV1 + 5), t.extra(kFxV1 + 8)}, k[2]);
+        fx_rows_of(t, k, ae, am);
         P[2 * j] = fx_norm(ae);
         P[2 * j + 1] = fx_norm(am);
     }
@@ -976,6 +985,9 @@ CP3_HD void fx_shift_sums(const double rate[2], int b0, int step, int nb, const 
 #pragma unroll 1
     for (int b = b0; b < nb; b += step) {
         const double h = -mid[b], w = wid[b];
+        double weight[3];  // asked for before the phases, which cover their way (49 us against 51)
+#pragma unroll
+        for (int f = 0; f < 3; f++) weight[f] = prob[f * flavour + b * stride];
         cfx z[3];
         double x[3];
 #pragma unroll
@@ -997,7 +1009,7 @@ CP3_HD void fx_shift_sums(const double rate[2], int b0, int step, int nb, const 
         }
 #pragma unroll
         for (int f = 0; f < 3; f++) {
-            const double p = prob[f * flavour + b * stride];
+            const double p = weight[f];
             const long long pb = fx_bits(p) & 0x7fffffffffffffffLL;
             if (pb > 0x3ff0000000000000LL) bad |= 1u << 20;  // above 1, or not a number
             const long long pv = pb > 0x3ff0000000000000LL ? 0 : fx_scaled(p, 1023);
@@ -1015,19 +1027,6 @@ CP3_HD void fx_shift_sums(const double rate[2], int b0, int step, int nb, const 
                 }
         }
     }
-}
-
-// The factors t from the sums over all heights; weights that add up to more than 5/4 leave the
-// range.
-CP3_HD void fx_shift_factors(const long long sum[3][3][2], const unsigned long long total[3], unsigned int& bad,
-                             cfx t[3][3]) {
-#pragma unroll
-    for (int f = 0; f < 3; f++)
-        if (total[f] > (5ULL << 52)) bad |= 1u << 20;
-#pragma unroll
-    for (int q = 0; q < 3; q++)
-#pragma unroll
-        for (int f = 0; f < 3; f++) t[q][f] = cfx{fx_split(sum[q][f][0]), fx_split(sum[q][f][1])};
 }
 
 // The rows e, mu of a_k = W G u_k; load() as above.
@@ -1048,48 +1047,79 @@ CP3_HD void fx_air_rows(Solve solve, Load load, const FxW& w, const double* len,
     }
 }
 
-// One averaged bin from these rows and its shift factors; P[j][i] the probability of j -> i,
-// i = e, mu.
-CP3_HD void fx_average(const cfx a[2][3], const FxAir& air, const FxW& w, double air_km,
-                       const longlong2* trig, const cfx t[3][3], unsigned int& bad, long long P[3][2]) {
+// The same from a table of the layers.
+CP3_HD void fx_air_rows(const FxColumn& t, const double* len, int M, const longlong2* trig, unsigned int& bad,
+                        cfx a[2][3]) {
+    if (M == 0) {  // G = 1: the air layer's own flavour rows
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            a[0][k] = cfx{t.extra(kFxV0 + k), fx{0, 0}};
+            a[1][k] = cfx{t.extra(kFxV0 + 3 + k), t.extra(kFxV0 + 6 + k)};
+        }
+        return;
+    }
+    auto layer = [&](int l, cfx* f, FxDet* det) {
+        const double rate[2] = {t.rate(l, 0), t.rate(l, 1)};
+        fx_layer(rate, len[l], trig, f, bad, det);
+    };
+    cfx y[3][3], e[2];
+    if (M > 1) fx_columns(t, M, layer, trig, y);
+    layer(M, e, nullptr);
+#pragma unroll 1
+    for (int k = 0; k < 3; k++) {
+        cfx v[3];
+#pragma unroll
+        for (int i = 0; i < 3; i++) v[i] = cfx{t.rot(0, 3 * i + k), fx{0, 0}};  // U_1^T u_k
+        if (M > 1)
+            fx_palindrome(y, e, v);
+        else
+            fx_phase(e, v);
+        fx_rows_of(t, v, a[0][k], a[1][k]);
+    }
+}
+
+// Weights that add up to more than 5/4 leave the range of the factors t.
+CP3_HD void fx_check_weights(const unsigned long long total[3], unsigned int& bad) {
+#pragma unroll
+    for (int f = 0; f < 3; f++)
+        if (total[f] > (5ULL << 52)) bad |= 1u << 20;
+}
+
+// One averaged bin's probabilities of the initial flavour j, from these rows, the air layer's
+// own (fx_rows) and its rates, and j's shift factors t: P[i] that of j -> i, i = e, mu.  The
+// tau row's products follow from the others': the columns of W U_0 are orthonormal.
+CP3_HD void fx_average(int j, const cfx a[2][3], const fx row[9], const double rate[2], double air_km,
+                       const longlong2* trig, const cfx t[3], unsigned int& bad, long long P[2]) {
     cfx e[3];  // e_k conj(e_q) of the pairs (1,0), (2,0), (2,1)
-    fx_layer(air.rate, air_km, trig, e, bad);
+    fx_layer(rate, air_km, trig, e, bad);
     e[2] = fx_cmul(cfx{e[0].re, fx_neg(e[0].im)}, e[1]);
     const int hi[3] = {1, 2, 2}, lo[3] = {0, 0, 1};
-    fx n[2][3];
-    cfx d[2][3];  // conj(a_qi) a_ki
+    fxacc2 s[2], x[2];
 #pragma unroll
-    for (int i = 0; i < 2; i++)
+    for (int k = 0; k < 3; k++) {
+        const int h = hi[k], l = lo[k];
+        // |b_k|^2 and b_q conj(b_k)
+        fxacc er, en;
+        fx_mac(er, row[h], row[l]);
+        fx_mac(en, row[k], row[k]);
+        const cfx m = fx_cmul(cfx{row[3 + h], fx_neg(row[6 + h])}, cfx{row[3 + l], row[6 + l]});
+        const long long mn = fx_norm(cfx{row[3 + k], row[6 + k]});
+        const cfx c = j == 0   ? cfx{fx_res(er), fx{0, 0}}
+                      : j == 1 ? m
+                               : cfx{fx_split(-fx_sum(er) - fx_value(m.re)), fx_neg(m.im)};
+        const fx norm = fx_split(j == 0 ? fx_sum(en) : j == 1 ? mn : (1LL << 62) - fx_sum(en) - mn);
+        const cfx f = fx_cmul(t[k], fx_cmul(e[k], c));
 #pragma unroll
-        for (int k = 0; k < 3; k++) {
-            n[i][k] = fx_split(fx_norm(a[i][k]));
-            const cfx q = a[i][lo[k]];
-            d[i][k] = fx_cmul(cfx{q.re, fx_neg(q.im)}, a[i][hi[k]]);
+        for (int i = 0; i < 2; i++) {
+            const cfx q = a[i][l];
+            const cfx d = fx_cmul(cfx{q.re, fx_neg(q.im)}, a[i][h]);  // conj(a_qi) a_ki
+            fx_mac(s[i], fx_split(fx_norm(a[i][k])), norm);
+            fx_mac(x[i], d.re, f.re);
+            fx_mac(x[i], fx_neg(d.im), f.im);
         }
-#pragma unroll 1
-    for (int j = 0; j < 3; j++) {
-        cfx b[3];
-#pragma unroll
-        for (int k = 0; k < 3; k++)
-            b[k] = j == 0 ? cfx{air.row[k], fx{0, 0}}
-                   : j == 1 ? cfx{air.row[3 + k], air.row[6 + k]}
-                            : fx_flavour(fx_neg(w.s), w.cr, w.ci, cfx{air.U[1][k], fx{0, 0}}, cfx{air.U[2][k], fx{0, 0}});
-        fxacc2 s[2], x[2];
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-            const fx m = fx_split(fx_norm(b[k]));
-            const cfx c = b[hi[k]];
-            const cfx f = fx_cmul(t[k][j], fx_cmul(e[k], fx_cmul(cfx{c.re, fx_neg(c.im)}, b[lo[k]])));
-#pragma unroll
-            for (int i = 0; i < 2; i++) {
-                fx_mac(s[i], n[i][k], m);
-                fx_mac(x[i], d[i][k].re, f.re);
-                fx_mac(x[i], fx_neg(d[i][k].im), f.im);
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < 2; i++) P[j][i] = fx_sum(s[i]) + 2 * fx_sum(x[i]);
     }
+#pragma unroll
+    for (int i = 0; i < 2; i++) P[i] = fx_sum(s[i]) + 2 * fx_sum(x[i]);
 }
 
 }  // namespace cp3

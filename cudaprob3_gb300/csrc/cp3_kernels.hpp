@@ -115,12 +115,12 @@ cudaError_t launch_atmos_mixed_inline_avg(const OscParams& p, const double* ener
                                           RowRange rr = RowRange{});
 
 // Atmospheric bins whose layers are solved in place.  FP64: quadratic densities (rho per
-// segment) and production-height averaging (avg.n_bins > 0; rho per segment, or per class with
-// per_class), with the fixed-point table of the air alone (launch_table_fx, one class); mixed:
-// quadratic densities.
+// segment) with the fixed-point table of the air alone (launch_table_fx, one class), and
+// production-height averaging (avg.n_bins > 0), for quadratic densities as that (ncls = 0), for
+// constant ones from the table of ncls classes (rho per class); mixed: quadratic densities.
 cudaError_t launch_atmos_fx_inline(const OscParams& p, const double* energies, int ne,
                                    const int2* table, const int* seg_off, const double* seg_len, const double* rho,
-                                   bool per_class, int n_cosines, const AvgArrays& avg, double* out,
+                                   int ncls, int n_cosines, const AvgArrays& avg, double* out,
                                    cudaStream_t s, RowRange rr = RowRange{});
 cudaError_t launch_atmos_mixed_inline(const OscParams& p, const double* energies, int ne,
                                       const int* seg_off, const float2* seg_len,

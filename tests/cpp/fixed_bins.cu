@@ -1,5 +1,6 @@
 // The fixed-point FP64 bins (cp3_fixed.cuh) on the host, one call for a whole grid; the number
 // of bins that asked for the FP64 path is returned (-1: bad model).
+#include <algorithm>
 #include <string>
 #include <vector>
 
@@ -9,6 +10,30 @@
 using namespace cp3;
 
 static constexpr TrigTable kTable = make_trig_table();
+
+// One energy's column of the table (launch_table_fx) from its solved classes.
+static void fill_column(const OscParams& p, const std::vector<FxClass>& cls, int2* tab, int2* ext) {
+    for (size_t c = 0; c < cls.size(); c++) {
+        fx v[13], row[9];
+        if (c < 2) {
+            fx_rows(cls[c].U, p.w, row);
+            for (int f = 0; f < 9; f++) ext[(c ? kFxV1 : kFxV0) + f] = make_int2(row[f].h, row[f].l);
+        }
+        if (c == 0) {
+            fx_coefficients(row, v);
+            for (int f = 0; f < 13; f++) ext[kFxVac + f] = make_int2(v[f].h, v[f].l);
+        }
+        int2* d = tab + c * kFxFields;
+        for (int q = 0; q < 2; q++) {
+            const long long b = fx_bits(cls[c].rate[q]);
+            d[kFxRates + q] = make_int2((int)b, (int)(b >> 32));
+        }
+        if (c + 1 == cls.size()) break;
+        fx R[3][3];
+        fx_rotation(cls[c + 1].U, cls[c].U, R);
+        for (int f = 0; f < 9; f++) d[f] = make_int2(R[f / 3][f % 3].h, R[f / 3][f % 3].l);
+    }
+}
 
 extern "C" void fixed_trig(long long* out) { std::memcpy(out, &kTable, sizeof kTable); }
 
@@ -42,27 +67,8 @@ extern "C" int fixed_atmos(const double* mix, int knutype, int anti, const doubl
                 fx_third(cls[c].U);
                 if (!fx_refine(&p, E, 1.0 / E, rho_e, cls[c])) fx_class_f64(u, dmv, E, cls[c]);
             }
-            fx v[13], row[9];
-            if (c < 2) {
-                fx_rows(cls[c].U, p.w, row);
-                for (int f = 0; f < 9; f++) ext[(c ? kFxV1 : kFxV0) + f] = make_int2(row[f].h, row[f].l);
-            }
-            if (c == 0) {
-                fx_coefficients(row, v);
-                for (int f = 0; f < 13; f++) ext[kFxVac + f] = make_int2(v[f].h, v[f].l);
-            }
         }
-        for (int c = 0; c < ncls; c++) {
-            int2* d = tab.data() + (size_t)c * kFxFields;
-            for (int q = 0; q < 2; q++) {
-                const long long b = fx_bits(cls[c].rate[q]);
-                d[kFxRates + q] = make_int2((int)b, (int)(b >> 32));
-            }
-            if (c + 1 == ncls) break;
-            fx R[3][3];
-            fx_rotation(cls[c + 1].U, cls[c].U, R);
-            for (int f = 0; f < 9; f++) d[f] = make_int2(R[f / 3][f % 3].h, R[f / 3][f % 3].l);
-        }
+        fill_column(p, cls, tab.data(), ext);
         const FxColumn col{tab.data(), ext, 1, (size_t)kFxFields};
         for (int ic = 0; ic < nc; ic++) {
             long long P[4];
@@ -107,6 +113,15 @@ extern "C" int fixed_inline(const double* mix, int knutype, int anti, const doub
         fx_rows(k0.U, p.w, air.row);
         fx_coefficients(air.row, air.coef);
         air.rate[0] = k0.rate[0], air.rate[1] = k0.rate[1];
+        std::vector<FxClass> cls;
+        for (int c = 0; c <= *std::max_element(t.maxlayers.begin(), t.maxlayers.end()) && !poly; c++) {
+            cls.emplace_back();
+            layer(c ? model.rho[c - 1] * model.ye[c - 1] : 0.0, cls.back());
+        }
+        std::vector<int2> tab(cls.size() * kFxFields + kFxExtra);
+        int2* ext = tab.data() + cls.size() * kFxFields;
+        fill_column(p, cls, tab.data(), ext);
+        const FxColumn col{tab.data(), ext, 1, (size_t)kFxFields};
         for (int ic = 0; ic < nc; ic++) {
             const double *len = t.len_km.data() + t.offset[ic], *rho = t.rho_e.data() + t.offset[ic];
             auto solve = [&](int l, FxClass& k) { layer(rho[l], k); };
@@ -136,11 +151,18 @@ extern "C" int fixed_inline(const double* mix, int knutype, int anti, const doub
                     for (int q = 0; q < 6; q++) sum[q >> 1][j][q & 1] += one.value(q >> 1, j, q & 1);
                 }
             }
-            cfx f[3][3], rows[2][3];
+            cfx rows[2][3];
             long long P[3][2];
-            fx_shift_factors(sum, total, bad, f);
-            fx_air_rows(solve, [&]() { return air; }, w, len, t.maxlayers[ic], trig, bad, rows);
-            fx_average(rows, air, w, len[0], trig, f, bad, P);
+            fx_check_weights(total, bad);
+            if (poly)
+                fx_air_rows(solve, [&]() { return air; }, w, len, t.maxlayers[ic], trig, bad, rows);
+            else
+                fx_air_rows(col, len, t.maxlayers[ic], trig, bad, rows);
+            for (int j = 0; j < 3; j++) {
+                cfx f[3];
+                for (int q = 0; q < 3; q++) f[q] = cfx{fx_split(sum[q][j][0]), fx_split(sum[q][j][1])};
+                fx_average(j, rows, air.row, air.rate, len[0], trig, f, bad, P[j]);
+            }
             outside += (bad >> 20) != 0;
             for (int j = 0; j < 3; j++) {
                 o[(size_t)(3 * j) * plane] = fx_to_double(P[j][0]);
