@@ -607,7 +607,7 @@ __device__ __forceinline__ float sinc_reference_f(float x) {
     return 1.0f - x * x / 6.0f + x * x * x * x / 120.0f;
 }
 
-// Flavour-basis amplitude A = W A2 W^+ in FP32 (the transform of store_probabilities).
+// Flavour-basis amplitude A = W A2 W^+ in FP32.
 __device__ __forceinline__ void to_flavour_f32(const cg9& A2, const WParams& w, cg9& A) {
     cg9 Y;
 #pragma unroll

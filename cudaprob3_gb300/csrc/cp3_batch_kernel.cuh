@@ -150,17 +150,19 @@ CP3_HD constexpr bool clears_counters(int kinds, int phases) {
     return phases == kPhaseBins || (phases == kPhaseAll && kinds == kBeam);
 }
 
-// 72 registers per thread, 7 blocks per SM: measured 1-2 % faster on the batched atmospheric
-// and beam workloads than 64 registers (8 blocks), which spill more; 6 blocks is slower.  The
-// kPhaseBins instance fits 72 registers without spills; 64 or 56 (8 or 9 blocks) measured
-// no faster on the batched atmospheric workload.
-// The beam-only instance takes 80 registers, 6 blocks per SM: its polynomial solve spills at
-// 72 (64 problems x 2 baselines x 1e5 energies, runs among others: 142 us; with 7, 5 and 4
-// blocks 146, 149 and 151).  It is bound by the issue of its ~650 instructions an energy, of
-// which a packed one takes two slots.
+// Resident blocks: 7 (72 registers per thread) for the atmospheric instances, 1-2 % faster on the
+// batched workload than 8 (64 registers, which spill more) and 3 % than 6.  6 (80 registers) for
+// the beam-only ones, whose polynomial solve spills at 72 (64 problems x 2 baselines x 1e5
+// energies, runs among others: 142 us; with 7, 5 and 4 blocks 146, 149 and 151; bound by the
+// issue of ~650 instructions an energy, of which a packed one takes two slots), and for the
+// single launch of both kinds (16 problems of each: 430 us; with 7 and 5 blocks 445 and 453).
+CP3_HD constexpr int blocks_per_sm(int kinds, int phases) {
+    return kinds == kBeam || (kinds == kBoth && phases == kPhaseAll) ? 6 : 7;
+}
+
 // Internal linkage: each translation unit that launches it (batches, the server) has its own.
 template <int kKinds, int kPhases = kPhaseAll>
-static __global__ void __launch_bounds__(kBlock, kKinds == kBeam ? 6 : 7) batch_kernel(const Args a) {
+static __global__ void __launch_bounds__(kBlock, blocks_per_sm(kKinds, kPhases)) batch_kernel(const Args a) {
     constexpr int kWarps = kBlock / 32;
     constexpr int kTableLoad = kPhases == kPhaseBins ? kLoadReadOnly : kLoadL2;
     __shared__ float2 s_len[kWarps][kMaxSegments];  // one trajectory per warp

@@ -168,24 +168,6 @@ __device__ __forceinline__ void apply_left(const Layer& f, cg9& G) {
     }
 }
 
-// G <- G S.  Per row: w = G u, y = w z, G += y u^T.
-__device__ __forceinline__ void apply_right(const Layer& f, cg9& G) {
-#pragma unroll
-    for (int k = 0; k < 2; k++) {
-        const float* u = f.u[k];
-        const float zr = f.z[k][0], zi = f.z[k][1];
-#pragma unroll
-        for (int i = 0; i < 3; i++) {
-            float2 w = __fmul2_rn(f2(G.a[i][0]), bc2(u[0]));
-            w = __ffma2_rn(f2(G.a[i][1]), bc2(u[1]), w);
-            w = __ffma2_rn(f2(G.a[i][2]), bc2(u[2]), w);
-            const float2 y = make_float2(fmaf(zr, w.x, -zi * w.y), fmaf(zr, w.y, zi * w.x));
-#pragma unroll
-            for (int j = 0; j < 3; j++) G.a[i][j] = fc(__ffma2_rn(y, bc2(u[j]), f2(G.a[i][j])));
-        }
-    }
-}
-
 // G = S = 1 + z1 u1 u1^T + z2 u2 u2^T
 __device__ __forceinline__ void layer_to_gen(const Layer& f, cg9& G) {
     const float2 z0 = make_float2(f.z[0][0], f.z[0][1]), z1 = make_float2(f.z[1][0], f.z[1][1]);
@@ -252,41 +234,10 @@ __device__ __forceinline__ void newton_schulz(cg9& A) {
     A = R;
 }
 
-// Probabilities of A = W A2 W^+, W = [[1,0,0],[0,c,s e],[0,-s,c e]], e = e^{i d}; stores
-// channel a*3+b = |A[b][a]|^2 at out[ch * plane].
-__device__ __forceinline__ void store_probabilities(const cg9& A2, float c, float s, float ed_re,
-                                                    float ed_im, float* __restrict__ out,
-                                                    size_t plane) {
-    cg9 Y;  // Y = A2 W^+ : columns 1, 2 mix through (c, -s) and e* (s, c)
-#pragma unroll
-    for (int i = 0; i < 3; i++) {
-        const cf a1 = A2.a[i][1], a2 = A2.a[i][2];
-        const cf f{a2.re * ed_re + a2.im * ed_im, a2.im * ed_re - a2.re * ed_im};  // e* a2
-        Y.a[i][0] = A2.a[i][0];
-        Y.a[i][1] = cf{fmaf(c, a1.re, s * f.re), fmaf(c, a1.im, s * f.im)};
-        Y.a[i][2] = cf{fmaf(-s, a1.re, c * f.re), fmaf(-s, a1.im, c * f.im)};
-    }
-#pragma unroll
-    for (int j = 0; j < 3; j++) {
-        const cf y1 = Y.a[1][j], y2 = Y.a[2][j];
-        const cf g{y2.re * ed_re - y2.im * ed_im, y2.re * ed_im + y2.im * ed_re};  // e y2
-        const cf r0 = Y.a[0][j];
-        const cf r1{fmaf(c, y1.re, s * g.re), fmaf(c, y1.im, s * g.im)};
-        const cf r2{fmaf(-s, y1.re, c * g.re), fmaf(-s, y1.im, c * g.im)};
-        // column j = initial flavour j; rows 0..2 = final flavours
-        out[(size_t)(j * 3 + 0) * plane] = fmaf(r0.re, r0.re, r0.im * r0.im);
-        out[(size_t)(j * 3 + 1) * plane] = fmaf(r1.re, r1.re, r1.im * r1.im);
-        out[(size_t)(j * 3 + 2) * plane] = fmaf(r2.re, r2.re, r2.im * r2.im);
-    }
-}
-
-// Trajectories crossing at least this many shells get the Newton-Schulz step.  Measured max
-// |mixed - FP64| on the 59-shell 2000 x 2000 grid (nu and nubar) with the step from M >= 6 /
-// 12 / 20 / never: 2.6e-6 / 5.2e-6 / 5.4e-6 / 9.5e-6, the per-bin kernel 0.186 / 0.184 /
-// 0.182 / 0.180 ms; on a PREM-12 grid 1.9e-6 / 3.8e-6 / 3.8e-6 / 3.8e-6, the batched PREM-12
-// workload 9.00 / 8.63 / 8.62 / 8.62 ms.  Without the step the error grows with the number
-// of FP32 layer applications (unitarity drift: 1.5e-6 at M = 2, 4.4e-6 at M = 12, 9.3e-6 at
-// M = 59).
+// Averaged bins of trajectories crossing at least this many shells get the Newton-Schulz step:
+// without it the error grows with the number of FP32 layer applications (unitarity drift:
+// 1.5e-6 at M = 2, 4.4e-6 at M = 12, 9.3e-6 at M = 59).  (Plain bins orthonormalise their two
+// columns whatever M.)
 constexpr int kNewtonSchulzMinShells = 6;
 
 struct WParams {
@@ -422,6 +373,123 @@ __device__ __forceinline__ void chain_mixed(SegFn seg, int M, cg9& G) {
     }
 }
 
+// ---- the end of a bin on two vectors -------------------------------------------------------
+// Of the amplitude A = W (B^T S_M B) S_0 W^+ only the columns e and mu are formed, each by
+// taking S_0 W^+'s column through the matrices: 2 x 104 operations after the chain, where
+// forming B^T S_M B and the product with S_0 took 276.  The tau column is conj(a_e x a_mu) up
+// to a phase, which its moduli do not see.
+
+// S_0 W^+'s columns e and mu: W^+ e = (1, 0, 0), W^+ mu = (0, c, s e^{-i delta}).
+__device__ __forceinline__ void initial_columns(const Layer& f, const WParams& w, float2 a[3], float2 b[3]) {
+    const float sr = w.s * w.er, si = -w.s * w.ei;
+    a[0] = make_float2(1.0f, 0.0f), a[1] = a[2] = make_float2(0.0f, 0.0f);
+    b[0] = make_float2(0.0f, 0.0f), b[1] = make_float2(w.c, 0.0f), b[2] = make_float2(sr, si);
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        const float* u = f.u[k];
+        const float zr = f.z[k][0], zi = f.z[k][1];
+        const float2 y = __fmul2_rn(bc2(u[0]), make_float2(zr, zi));
+        const float vr = fmaf(u[2], sr, u[1] * w.c), vi = u[2] * si;
+        const float2 x = make_float2(fmaf(zr, vr, -zi * vi), fmaf(zr, vi, zi * vr));
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+            a[i] = __ffma2_rn(bc2(u[i]), y, a[i]);
+            b[i] = __ffma2_rn(bc2(u[i]), x, b[i]);
+        }
+    }
+}
+
+// k <- S k
+__device__ __forceinline__ void apply_layer(const Layer& f, float2 k[3]) {
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+        const float* u = f.u[q];
+        const float zr = f.z[q][0], zi = f.z[q][1];
+        float2 v = __fmul2_rn(bc2(u[0]), k[0]);
+        v = __ffma2_rn(bc2(u[1]), k[1], v);
+        v = __ffma2_rn(bc2(u[2]), k[2], v);
+        const float2 y = make_float2(fmaf(zr, v.x, -zi * v.y), fmaf(zr, v.y, zi * v.x));
+#pragma unroll
+        for (int i = 0; i < 3; i++) k[i] = __ffma2_rn(bc2(u[i]), y, k[i]);
+    }
+}
+
+// k <- B^T S B k
+__device__ __forceinline__ void apply_palindrome(const cg9& B, const Layer& f, float2 k[3]) {
+    float2 m[3];
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        const cacc h = cdot3(B.a[i][0], fc(k[0]), B.a[i][1], fc(k[1]), B.a[i][2], fc(k[2]));
+        m[i] = make_float2(h.r.x - h.i.y, h.r.y + h.i.x);
+    }
+    apply_layer(f, m);
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        const cacc h = cdot3(B.a[0][i], fc(m[0]), B.a[1][i], fc(m[1]), B.a[2][i], fc(m[2]));
+        k[i] = make_float2(h.r.x - h.i.y, h.r.y + h.i.x);
+    }
+}
+
+__device__ __forceinline__ float norm2(const float2 a[3]) {
+    float2 q = __fmul2_rn(a[0], a[0]);
+    q = __ffma2_rn(a[1], a[1], q);
+    q = __ffma2_rn(a[2], a[2], q);
+    return q.x + q.y;
+}
+
+// One Newton-Schulz step toward orthonormal columns, [a b] <- [a b] (3 - [a b]^+ [a b]) / 2: the
+// rounding of FP32 layers leaves each slightly non-unitary, and that part of the error
+// accumulates over the ~2M products of a deep trajectory; the step removes it to second order.
+// It is taken whatever M: the third column is formed from these two.  2-norm error against the
+// FP64 bins, and the per-bin kernel's time, with this end of the bin and with the matrix formed
+// whole and corrected from M = 6: PREM-4 400 x 400 0.9e-7 and 1.5e-7, 7.9 and 7.8 us; PREM-12
+// 1000 x 1000 1.0e-7 and 1.4e-7, 30.3 and 32.4 us; 59 shells 2000 x 2000 1.4e-7 and 1.5e-7, 178
+// and 185 us.
+__device__ __forceinline__ void orthonormalize(float2 a[3], float2 b[3]) {
+    const float na = fmaf(-0.5f, norm2(a), 1.5f), nb = fmaf(-0.5f, norm2(b), 1.5f);
+    const cacc h = cdot3(fc(a[0]), fc(b[0]), fc(a[1]), fc(b[1]), fc(a[2]), fc(b[2]));
+    const float dr = -0.5f * (h.r.x + h.i.y), di = -0.5f * (h.r.y - h.i.x);  // -a^+ b / 2
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        const float2 x = a[i], y = b[i];
+        a[i] = make_float2(fmaf(na, x.x, fmaf(dr, y.x, di * y.y)), fmaf(na, x.y, fmaf(dr, y.y, -di * y.x)));
+        b[i] = make_float2(fmaf(nb, y.x, fmaf(dr, x.x, -di * x.y)), fmaf(nb, y.y, fmaf(dr, x.y, di * x.x)));
+    }
+}
+
+// The nine probabilities from the two columns in the rotated basis: W = [[1,0,0],[0,c,s e],
+// [0,-s,c e]], e = e^{i delta}; channel j*3+i = |A_ij|^2 at out[ch * plane].
+__device__ __forceinline__ void store_columns(const float2 a[3], const float2 b[3], const WParams& w,
+                                              float* __restrict__ out, size_t plane) {
+    cf v[2][3];
+#pragma unroll
+    for (int j = 0; j < 2; j++) {
+        const float2* k = j == 0 ? a : b;
+        const cf g{fmaf(k[2].x, w.er, -k[2].y * w.ei), fmaf(k[2].x, w.ei, k[2].y * w.er)};  // e k2
+        v[j][0] = fc(k[0]);
+        v[j][1] = cf{fmaf(w.c, k[1].x, w.s * g.re), fmaf(w.c, k[1].y, w.s * g.im)};
+        v[j][2] = cf{fmaf(-w.s, k[1].x, w.c * g.re), fmaf(-w.s, k[1].y, w.c * g.im)};
+#pragma unroll
+        for (int i = 0; i < 3; i++)
+            out[(size_t)(j * 3 + i) * plane] = fmaf(v[j][i].re, v[j][i].re, v[j][i].im * v[j][i].im);
+    }
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        const cf p = v[0][(i + 1) % 3], q = v[0][(i + 2) % 3], r = v[1][(i + 1) % 3], t = v[1][(i + 2) % 3];
+        const float re = fmaf(p.re, t.re, fmaf(-p.im, t.im, fmaf(-q.re, r.re, q.im * r.im)));
+        const float im = fmaf(p.re, t.im, fmaf(p.im, t.re, fmaf(-q.re, r.im, -q.im * r.re)));
+        out[(size_t)(6 + i) * plane] = fmaf(re, re, im * im);
+    }
+}
+
+// One or two FP32 layers are unitary to ~1e-7 already; the correction pays off from the longer
+// chains on.
+__device__ __forceinline__ void finish_columns(float2 a[3], float2 b[3], int M, const WParams& w,
+                                               float* __restrict__ out, size_t plane) {
+    orthonormalize(a, b);
+    store_columns(a, b, w, out, plane);
+}
+
 // One atmospheric bin over M+1 segments, generic in where each segment's layer comes from:
 // seg(l, F) fills F for segment l (0 = air, then shells inwards).
 template <class SegFn>
@@ -433,14 +501,28 @@ __device__ __forceinline__ void atmos_bin_mixed_with(SegFn seg, int M, const WPa
         store_one_layer(F, w, out, plane);
         return;
     }
-    cg9 A2;
-    chain_mixed(seg, M, A2);
+    cg9 B;
+    if (M > 1) {
+        seg(1, F);
+        layer_to_gen(F, B);  // B = S_{M-1}..S_1
+        for (int l = 2; l < M; l++) {
+            seg(l, F);
+            apply_left(F, B);
+        }
+    }
+    float2 a[3], b[3];
     seg(0, F);
-    apply_right(F, A2);  // ... S_0
-    // One or two FP32 layer matrices are unitary to ~1e-7 already; the correction pays off
-    // from the longer chains on (it removes the drift accumulated over ~2M products).
-    if (M >= kNewtonSchulzMinShells) newton_schulz(A2);
-    store_probabilities(A2, w.c, w.s, w.er, w.ei, out, plane);
+    initial_columns(F, w, a, b);
+    seg(M, F);
+    if (M > 1) {
+        apply_palindrome(B, F, a);
+        apply_palindrome(B, F, b);
+    } else {
+        apply_layer(F, a);
+        apply_layer(F, b);
+    }
+    orthonormalize(a, b);
+    store_columns(a, b, w, out, plane);
 }
 
 // One atmospheric bin from the eigen table: the trajectory's segment lengths are in shared
@@ -450,7 +532,7 @@ __device__ __forceinline__ void atmos_bin_mixed_with(SegFn seg, int M, const WPa
 //
 // kPrefetch: each segment's entry is loaded one layer ahead of its use, so that the L2
 // latency of the table overlaps the previous layer's arithmetic (the air segment's entry
-// comes last).  Measured: 2 % faster in the batched kernel, whose tables are written in the
+// comes after the chain's, the innermost one's last).  Measured: 2 % faster in the batched kernel, whose tables are written in the
 // same launch; 1 % slower in the single-grid kernel, which therefore loads on use.
 template <int kLoad = kLoadReadOnly, bool kPrefetch = false>
 __device__ __forceinline__ void atmos_bin_mixed(const float* __restrict__ tab, size_t cls_stride,
@@ -468,26 +550,36 @@ __device__ __forceinline__ void atmos_bin_mixed(const float* __restrict__ tab, s
         store_one_layer(F, w, out, plane);
         return;
     }
-    cg9 A2;
-    TableEntry e = entry(1), n = entry(M > 1 ? 2 : 0);
-    layer_from_entry(e, s_len[1], F);
-    layer_to_gen(F, A2);  // B = S_1
+    cg9 B;
+    TableEntry n = entry(1);
     if (M > 1) {
+        TableEntry e = n;
+        n = entry(M > 2 ? 2 : 0);
+        layer_from_entry(e, s_len[1], F);
+        layer_to_gen(F, B);  // B = S_{M-1}..S_1
         for (int l = 2; l < M; l++) {
             e = n;
-            n = entry(l + 1);
+            n = entry(l + 1 < M ? l + 1 : 0);
             layer_from_entry(e, s_len[l], F);
-            apply_left(F, A2);
+            apply_left(F, B);
         }
-        e = n;
+    } else {
         n = entry(0);
-        layer_from_entry(e, s_len[M], F);
-        close_palindrome(F, A2);
     }
+    float2 a[3], b[3];
     layer_from_entry(n, s_len[0], F);
-    apply_right(F, A2);  // ... S_0
-    if (M >= kNewtonSchulzMinShells) newton_schulz(A2);  // as in atmos_bin_mixed_with
-    store_probabilities(A2, w.c, w.s, w.er, w.ei, out, plane);
+    n = entry(M);
+    initial_columns(F, w, a, b);
+    layer_from_entry(n, s_len[M], F);
+    if (M > 1) {
+        apply_palindrome(B, F, a);
+        apply_palindrome(B, F, b);
+    } else {
+        apply_layer(F, a);
+        apply_layer(F, b);
+    }
+    orthonormalize(a, b);  // as in atmos_bin_mixed_with
+    store_columns(a, b, w, out, plane);
 }
 
 // Layer of a segment whose density is its own (quadratic density model): the
