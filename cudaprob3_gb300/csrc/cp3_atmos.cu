@@ -4,7 +4,8 @@
 // for the mixed table kernel), one thread = one (cosine, energy) bin.  The row's trajectory
 // (its segment lengths, a few hundred bytes; segment l reads density class l) is staged in
 // shared memory; every thread of the CTA then walks the same segment list, so control flow
-// is uniform.  The per-(class, energy) eigen tables are read contiguously across a warp
+// is uniform.  (FP64 results in fixed point: one warp = one row x 32 energies, a block's four
+// warps consecutive rows of the same energies.)  The eigen tables are read contiguously across a warp
 // (one entry per energy) and stay L2-resident.  The result
 // [9][n_cosines][n_energies] is written one channel plane at a time: each warp store is
 // 32 consecutive elements (128 B in FP32, 256 B in FP64).

@@ -1,7 +1,8 @@
-// cp3_f64.cuh -- building blocks of the FP64 kernels in the rotated real basis: one layer as
+// cp3_f64.cuh -- FP64 arithmetic in the rotated real basis: one layer as
 // S = 1 + z1 u1 u1^T + z2 u2 u2^T with the reference's own phases, the layer matrix, and the
-// flavour-basis amplitude A = W A2 W^+.  Shared by the atmospheric kernels (cp3_atmos.cu) and
-// the beam kernel (cp3_tables.cu, which is compiled without FMA contraction).
+// flavour-basis amplitude A = W A2 W^+.  For the bins that the fixed-point kernels
+// (cp3_fixed.cuh) hand over: atmospheric ones (cp3_atmos.cu) and the beam's (cp3_tables.cu,
+// which is compiled without FMA contraction).
 #pragma once
 
 #include "cp3_device.cuh"

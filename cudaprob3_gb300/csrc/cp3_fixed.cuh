@@ -45,7 +45,8 @@ CP3_HD fx fx_split(long long v) {
     return fx{(int)(v >> 32) + (int)((unsigned int)v >> 31), (int)v};
 }
 CP3_HD long long fx_value(fx a) { return (long long)(((unsigned long long)(long long)a.h << 32) + (unsigned long long)(long long)a.l); }
-CP3_HD fx fx_neg(fx a) { return fx{-a.h, -a.l}; }
+// To one unit, 2^-62: the low word's lowest value has no negative (-l of it is off by 2^-30).
+CP3_HD fx fx_neg(fx a) { return fx{-a.h, ~a.l}; }
 CP3_HD fx fx_of(int2 v) { return fx{v.x, v.y}; }
 
 // |v| < 2

@@ -1,5 +1,5 @@
 // cp3_tables.cu -- eigen work: the per-(density class, energy) tables of the atmospheric
-// kernels and the per-bin FP64 beam kernel.
+// kernels and the FP64 beam kernel.
 //
 // This translation unit is compiled with -fmad=false: where two levels nearly meet, its FP64
 // arithmetic is the reference's (physics.hpp getMfast) in the reference's order, and keeping

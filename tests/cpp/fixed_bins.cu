@@ -173,3 +173,5 @@ extern "C" int fixed_inline(const double* mix, int knutype, int anti, const doub
     }
     return outside;
 }
+
+extern "C" long long fixed_negated(long long v) { return fx_value(fx_neg(fx_split(v))); }

@@ -55,6 +55,16 @@ def test_trig_table(host):
     assert np.abs(t[:, 1] * 2.0 ** -62 - np.sin(a)).max() <= 4e-16
 
 
+def test_negation_at_the_low_words_ends(host):
+    """-v to one unit for every low word, its lowest value (which has no 32-bit negative) among
+    them; a bin in 4e6 met it, 2e-11 off."""
+    host.fixed_negated.restype = C.c_longlong
+    for high in (0, 1, -1, 12345, -(1 << 30), (1 << 30) - 1):
+        for low in (-(1 << 31), -(1 << 31) + 1, -1, 0, 1, (1 << 31) - 1):
+            v = high * (1 << 32) + low
+            assert abs(host.fixed_negated(C.c_longlong(v)) + v) <= 1
+
+
 @pytest.mark.parametrize("shells,h", [(1, 22.0), (2, 0.0), (3, 15.0), (12, 22.0), (59, 100.0), (128, 22.0)])
 def test_host_bins_against_oracle(host, oracle, shells, h):
     """Both orderings, nu and nubar, vacuum-only rows, vertical and shell-grazing rows, at the
