@@ -154,15 +154,14 @@ CP3_HD constexpr bool clears_counters(int kinds, int phases) {
 // batched workload than 8 (64 registers, which spill more) and 3 % than 6.  6 (80 registers) for
 // the beam-only ones, whose polynomial solve spills at 72 (64 problems x 2 baselines x 1e5
 // energies, runs among others: 142 us; with 7, 5 and 4 blocks 146, 149 and 151; bound by the
-// issue of ~650 instructions an energy, of which a packed one takes two slots), and for the
-// single launch of both kinds (16 problems of each: 430 us; with 7 and 5 blocks 445 and 453).
-CP3_HD constexpr int blocks_per_sm(int kinds, int phases) {
-    return kinds == kBeam || (kinds == kBoth && phases == kPhaseAll) ? 6 : 7;
-}
+// issue of ~650 instructions an energy, of which a packed one takes two slots), and for those of
+// both kinds, which spill most (a mix of PREM-4 grids and beams, runs among others: 181 us, with
+// 7 blocks 185; the single launch of 16 problems of each: 430, with 7 and 5 blocks 445 and 453).
+CP3_HD constexpr int blocks_per_sm(int kinds) { return kinds & kBeam ? 6 : 7; }
 
 // Internal linkage: each translation unit that launches it (batches, the server) has its own.
 template <int kKinds, int kPhases = kPhaseAll>
-static __global__ void __launch_bounds__(kBlock, blocks_per_sm(kKinds, kPhases)) batch_kernel(const Args a) {
+static __global__ void __launch_bounds__(kBlock, blocks_per_sm(kKinds)) batch_kernel(const Args a) {
     constexpr int kWarps = kBlock / 32;
     constexpr int kTableLoad = kPhases == kPhaseBins ? kLoadReadOnly : kLoadL2;
     __shared__ float2 s_len[kWarps][kMaxSegments];  // one trajectory per warp

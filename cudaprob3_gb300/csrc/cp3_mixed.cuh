@@ -236,8 +236,7 @@ __device__ __forceinline__ void newton_schulz(cg9& A) {
 
 // Averaged bins of trajectories crossing at least this many shells get the Newton-Schulz step:
 // without it the error grows with the number of FP32 layer applications (unitarity drift:
-// 1.5e-6 at M = 2, 4.4e-6 at M = 12, 9.3e-6 at M = 59).  (Plain bins orthonormalise their two
-// columns whatever M.)
+// 1.5e-6 at M = 2, 4.4e-6 at M = 12, 9.3e-6 at M = 59).  (Plain bins: orthonormalize.)
 constexpr int kNewtonSchulzMinShells = 6;
 
 struct WParams {
@@ -440,13 +439,26 @@ __device__ __forceinline__ float norm2(const float2 a[3]) {
 // One Newton-Schulz step toward orthonormal columns, [a b] <- [a b] (3 - [a b]^+ [a b]) / 2: the
 // rounding of FP32 layers leaves each slightly non-unitary, and that part of the error
 // accumulates over the ~2M products of a deep trajectory; the step removes it to second order.
-// It is taken whatever M: the third column is formed from these two.  2-norm error against the
-// FP64 bins, and the per-bin kernel's time, with this end of the bin and with the matrix formed
-// whole and corrected from M = 6: PREM-4 400 x 400 0.9e-7 and 1.5e-7, 7.9 and 7.8 us; PREM-12
-// 1000 x 1000 1.0e-7 and 1.4e-7, 30.3 and 32.4 us; 59 shells 2000 x 2000 1.4e-7 and 1.5e-7, 178
-// and 185 us.
-__device__ __forceinline__ void orthonormalize(float2 a[3], float2 b[3]) {
+// Below kOrthogonalMinShells only the norms are put right, which is nearly all of it there; not
+// even these, and the third column, formed from the two, is further off than a matrix formed
+// whole (PREM-4 2-norm 1.7e-7).  With the step whatever M the error is the same and the batches
+// are slower (32 PREM-12 problems alone 634 us, norms below M = 6 632, below 12 623; a mix of
+// PREM-4 grids 229, 225 and 225).
+// 2-norm error against the FP64 bins, and the per-bin kernel's time, with this end of the bin
+// and with the matrix formed whole and corrected from M = 6: PREM-4 400 x 400 0.9e-7 and 1.5e-7,
+// 7.9 and 7.8 us; PREM-12 1000 x 1000 1.1e-7 and 1.4e-7, 30.3 and 32.4 us; 59 shells 2000 x 2000
+// 1.4e-7 and 1.5e-7, 178 and 185 us.
+constexpr int kOrthogonalMinShells = 12;
+__device__ __forceinline__ void orthonormalize(float2 a[3], float2 b[3], int M) {
     const float na = fmaf(-0.5f, norm2(a), 1.5f), nb = fmaf(-0.5f, norm2(b), 1.5f);
+    if (M < kOrthogonalMinShells) {  // the norms alone
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+            a[i] = __fmul2_rn(a[i], bc2(na));
+            b[i] = __fmul2_rn(b[i], bc2(nb));
+        }
+        return;
+    }
     const cacc h = cdot3(fc(a[0]), fc(b[0]), fc(a[1]), fc(b[1]), fc(a[2]), fc(b[2]));
     const float dr = -0.5f * (h.r.x + h.i.y), di = -0.5f * (h.r.y - h.i.x);  // -a^+ b / 2
 #pragma unroll
@@ -486,7 +498,7 @@ __device__ __forceinline__ void store_columns(const float2 a[3], const float2 b[
 // chains on.
 __device__ __forceinline__ void finish_columns(float2 a[3], float2 b[3], int M, const WParams& w,
                                                float* __restrict__ out, size_t plane) {
-    orthonormalize(a, b);
+    orthonormalize(a, b, M);
     store_columns(a, b, w, out, plane);
 }
 
@@ -521,7 +533,7 @@ __device__ __forceinline__ void atmos_bin_mixed_with(SegFn seg, int M, const WPa
         apply_layer(F, a);
         apply_layer(F, b);
     }
-    orthonormalize(a, b);
+    orthonormalize(a, b, M);
     store_columns(a, b, w, out, plane);
 }
 
@@ -578,7 +590,7 @@ __device__ __forceinline__ void atmos_bin_mixed(const float* __restrict__ tab, s
         apply_layer(F, a);
         apply_layer(F, b);
     }
-    orthonormalize(a, b);  // as in atmos_bin_mixed_with
+    orthonormalize(a, b, M);  // as in atmos_bin_mixed_with
     store_columns(a, b, w, out, plane);
 }
 
