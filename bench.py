@@ -41,31 +41,32 @@ BATCH_SETS = 0  # --batch-sets: fewer parameter sets for the batched workloads (
 # summary).  A launch of another size is scaled by its result bytes, since traffic is the
 # output stream plus a small table/descriptor read that grows with it.
 NCU_TRAFFIC = {
-    ("atmos59", "mixed"): (5.910016e6 + 84.903680e6, 144.0e6,
+    ("atmos59", "mixed"): (5.912320e6 + 84.921856e6, 144.0e6,
                            "profiles/atmos_mixed_kernel_59shells_2000x2000.md"),
     # the table launch and the bin launch of one run
-    ("batch_atmos", "mixed"): (0.431616e6 + 0.060672e6 + 205.593088e6 + 982.776320e6, 912.332288e6,
+    ("batch_atmos", "mixed"): (0.429312e6 + 0.039936e6 + 200.539904e6 + 977.089792e6, 912.332288e6,
                                "profiles/batch_kernel_prem12_48problems.md"),
-    ("batch_beam", "mixed"): (115.457024e6 + 911.392000e6, 921.6e6,
+    ("batch_beam", "mixed"): (106.884864e6 + 875.584000e6, 921.6e6,
                               "profiles/batch_kernel_beam_128problems.md"),
-    ("atmos59", "fp64"): (9.871104e6 + 244.749312e6, 288.0e6,
-                          "profiles/atmos_f64_kernel_59shells_2000x2000.md"),
+    ("atmos59", "fp64"): (11.075072e6 + 232.746752e6, 288.0e6,
+                          "profiles/atmos_fx_kernel_59shells_2000x2000.md"),
     # the 7.2 MB output is still in L2 when the captured launch ends
-    ("beam", "fp64"): (0.865792e6, 7.2e6, "profiles/beam_f64_kernel_1e5energies.md"),
+    ("beam", "fp64"): (0.876800e6, 7.2e6, "profiles/beam_f64_kernel_1e5energies.md"),
 }
 
 
 # The dominant kernel's measured pipe utilisation in the same captures: the fraction of the
-# FMA (FP32) or FP64 pipe's peak the kernel keeps busy.  The canonical roofline fraction
+# FMA (FP32; its heavy half for the fixed-point kernels' integer multiply-adds) or FP64 pipe's
+# peak the kernel keeps busy.  The canonical roofline fraction
 # counts the reference formulation's flops, more than these kernels execute (it can exceed
 # 1); this is the utilisation of what they do execute.
 NCU_PIPE = {
-    ("atmos59", "mixed"): ("sm__pipe_fma_cycles_active", 0.7099),
-    ("batch_atmos", "mixed"): ("sm__pipe_fma_cycles_active", 0.6572),  # the bin launch
-    ("batch_beam", "mixed"): ("sm__pipe_fma_cycles_active", 0.6007),
-    ("atmos59", "fp64"): ("sm__pipe_fp64_cycles_active", 0.8930),
-    ("beam", "fp64"): ("sm__pipe_fp64_cycles_active", 0.8518),
-    ("batch_beam", "fp64"): ("sm__pipe_fp64_cycles_active", 0.8518),
+    ("atmos59", "mixed"): ("sm__pipe_fma_cycles_active", 0.7109),
+    ("batch_atmos", "mixed"): ("sm__pipe_fma_cycles_active", 0.6337),  # the bin launch
+    ("batch_beam", "mixed"): ("sm__pipe_fma_cycles_active", 0.6269),
+    ("atmos59", "fp64"): ("sm__pipe_fmaheavy_cycles_active", 0.7154),
+    ("beam", "fp64"): ("sm__pipe_fp64_cycles_active", 0.5477),
+    ("batch_beam", "fp64"): ("sm__pipe_fp64_cycles_active", 0.5477),
 }
 
 
@@ -143,7 +144,7 @@ def workload(name, rank=0):
                     beam=None,
                     desc="batched atmospheric: 256 Gaussian parameter sets (half inverted "
                          "ordering), own grids n_cos U[100,1000] x n_E U[100,2000], PREM "
-                         "12-layer, h=22 km, nu+nubar (512 problems), one CUDA-graph run (table "
+                         "12-layer, h=22 km, nu+nubar (512 problems), one run (table "
                          "launch + persistent bin launch)")
     if name == "batch_beam":
         sets = earth.gaussian_sets(BATCH_SETS or 4096, seed=rank_seed(2026, rank))
@@ -915,7 +916,7 @@ def fp64_arm(w, m, stream, flush, steps, warmup, gpu, world, refs, peaks, flops_
     eig_ms, kern_ms = serial_kernel_times(props, stream.cuda_stream, flush, 3)
     out = {"value": world * probs_step / (t_ms * 1e-3), "unit": "probabilities/s",
            "ms_per_step": t_ms, "steps": steps,
-           "kernel": "atmos_f64_kernel" if w["kind"] == "atmos" else "beam_f64_kernel",
+           "kernel": "atmos_fx_kernel" if w["kind"] == "atmos" else "beam_f64_kernel",
            "kernel_ms": round(kern_ms, 4), "eigen_table_ms": round(eig_ms, 4)}
     if peaks.get("fp64"):
         achieved = flops_launch / (kern_ms * 1e-3) / 1e12
@@ -1206,7 +1207,7 @@ def run_ours(args, rank, world):
         "peak_source": "live FMA-chain microbenchmark in this run (cp3_peaks.cu); the pool's "
                        "measured HBM/bf16 peaks do not apply to scalar FP pipes",
         "kernel": "atmos_mixed_kernel" if (w["kind"] == "atmos" and prec == "mixed") else
-                  ("atmos_f64_kernel" if w["kind"] == "atmos" else
+                  ("atmos_fx_kernel" if w["kind"] == "atmos" else
                    ("beam_mixed_kernel" if prec == "mixed" else "beam_f64_kernel")),
         "kernel_ms": round(kernel_ms, 4),
         "eigen_table_ms": round(eig_ms, 4),
