@@ -82,6 +82,20 @@ def test_host_bins_against_oracle(host, oracle, shells, h):
                 assert np.abs(got - ref).max() <= 1e-12
 
 
+@pytest.mark.parametrize("shells", [1, 4, 59, 128])
+@pytest.mark.parametrize("theta12,theta13", [(0.0, 0.0), (0.0, 0.15), (0.59, 0.0)])
+def test_host_bins_are_probabilities(host, shells, theta12, theta13):
+    """Nothing below 0 or above 1 where a channel is exactly zero or one (a decoupled flavour) and
+    the rounding of a deep chain could leave it on either side."""
+    m = earth.NOMINAL
+    m = type(m)(theta12, theta13, m.theta23, m.dcp, m.dm12sq, m.dm23sq)
+    cz, en = np.linspace(-1, 0.3, 53), np.logspace(-1, 3, 101)
+    for anti in (False, True):
+        got, outside = host_bins(host, m, anti, cz, en, earth.synthetic_shells(shells), 22.0)
+        assert outside == 0
+        assert got.min() >= 0.0 and got.max() <= 1.0
+
+
 def test_out_of_range_bins_ask_for_the_fp64_path(host):
     """Energies that are not finite or zero, and phases past 2^42 turns (13 000 km at 1e-13 GeV
     and below); the neighbouring energies stay inside."""
@@ -157,6 +171,29 @@ def test_gpu_averaged_bins_at_the_edges_and_out_of_range(oracle, nb, nc, ne):
         for prec, tol in (("fp64", 1e-12), ("mixed", 1e-5)):
             got = run_avg(prec, mix6, -1, True, cz, en, r, rho, ye, 20.0, nb, w, edges)
             assert np.abs(got - ref).max() <= tol * max(1.0, scale)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shells", [59, 128])
+@pytest.mark.parametrize("nb", [0, 1, 20])
+def test_gpu_results_are_probabilities(shells, nb):
+    """As test_host_bins_are_probabilities, plain bins and bins averaged with weights that add up
+    to one."""
+    from tests.gpu_helpers import run_atmos
+    from tests.test_gpu_averaging import run_avg
+    m = earth.NOMINAL
+    mix6 = [0.0, 0.0, m.theta23, m.dcp, m.dm12sq, m.dm23sq]
+    cz, en = np.linspace(-1, 0.3, 53), np.logspace(-1, 3, 101)
+    w = np.random.default_rng(3).uniform(0.1, 1.0, (2, 3, len(en), len(cz), max(nb, 1)))
+    w /= w.sum(axis=-1, keepdims=True)
+    model = earth.synthetic_shells(shells)
+    for anti in (False, True):
+        if nb:
+            got = run_avg("fp64", mix6, -1 if anti else 1, anti, cz, en, *model, 22.0, nb, w.ravel(),
+                          np.linspace(5.0, 45.0, nb + 1))
+        else:
+            got = run_atmos("fp64", mix6, -1 if anti else 1, anti, cz, en, *model, 22.0)
+        assert got.min() >= 0.0 and got.max() <= 1.0
 
 
 @pytest.mark.gpu
