@@ -108,7 +108,8 @@ struct cp3_batch {
     Buf<float> d_tables, d_out;
     Buf<unsigned int> d_counter;
     OscParams* h_params = nullptr;  // pinned staging
-    int* h_status = nullptr;        // the last run's status word, in page-locked memory
+    int* h_status = nullptr;        // the runs' status word, in page-locked memory (status_word)
+    unsigned int run = 0;           // the last run's number
     bool params_dirty = true;
     bool counters_dirty = false;    // the last run did not leave the counters zero
 
@@ -344,7 +345,7 @@ int commit(cp3_batch* b) {
     return configure(b);
 }
 
-// The start of a run: the parameters, if they changed, and the status word.  The counters are
+// The start of a run: the parameters, if they changed, and the run's number.  The counters are
 // zero where the last run's launches left them so.
 int begin_run(cp3_batch* b, bool clears, cudaStream_t s) {
     if (b->params_dirty) {
@@ -358,7 +359,7 @@ int begin_run(cp3_batch* b, bool clears, cudaStream_t s) {
         B_CUDA(b, cudaMemsetAsync(b->d_done.ptr, 0, sizeof(int) * b->probs.size(), s), "reset");
     }
     b->counters_dirty = true;  // until the run's last launch is queued
-    *(volatile int*)b->h_status = 0;
+    b->args.run = ++b->run;
     return CP3_OK;
 }
 
@@ -679,7 +680,7 @@ int cp3_batch_synchronize(cp3_batch* b, double* ms) {
         B_CUDA(b, cudaEventElapsedTime(&f, b->ev0, b->ev1), "elapsed");
         *ms = f;
     }
-    const int st = *(volatile int*)b->h_status;
+    const int st = status_of(*(volatile int*)b->h_status, b->run);
     if (st == kStatusWaitLimit)
         return bfail(b, CP3_ERR_CUDA, "batch kernel: eigen tables did not complete (wait limit)");
     if (st == kStatusBounds)

@@ -73,6 +73,9 @@ struct Args {
     // [bin_lo, min(bin_hi, total_b)).  The default is all of them; a run in pieces
     // (cp3_batch_run_to_host) launches one window of whole problems per piece.
     int bin_lo = 0, bin_hi = 0x7fffffff;
+    // The run a status belongs to: a batch's runs share the word and may be queued behind one
+    // another, so that the host cannot clear it for a run while an earlier one may still write it.
+    unsigned int run = 0;
 };
 
 constexpr int kCounters = 3;
@@ -82,8 +85,17 @@ constexpr int kCounters = 3;
 // arena, which is then skipped.
 constexpr int kStatusWaitLimit = 1, kStatusKind = 2, kStatusBounds = 3;
 
+// The status word: the code in the low bits, the run above them.
+constexpr int kStatusBits = 2;
+CP3_HD int status_word(unsigned int run, int code) { return (int)(run << kStatusBits | (unsigned int)code); }
+// The code of the given run: 0 where the word is another's.
+CP3_HD int status_of(int word, unsigned int run) {
+    const int code = word & ((1 << kStatusBits) - 1);
+    return word == status_word(run, code) ? code : 0;
+}
+
 // Rare: a plain store to the host's word (the end of the kernel makes it visible there).
-__device__ __forceinline__ void report(int* status, int code) { *(volatile int*)status = code; }
+__device__ __forceinline__ void report(const Args& a, int code) { *(volatile int*)a.status = status_word(a.run, code); }
 
 __device__ __forceinline__ unsigned long long global_timer_ns() {
     unsigned long long t;
@@ -201,7 +213,7 @@ static __global__ void __launch_bounds__(kBlock, blocks_per_sm(kKinds)) batch_ke
 
         if (ph == 0) {
             if (!(kKinds & kAtmos)) {  // cannot happen: the host picks kKinds from the problems
-                if (lane == 0) report(a.status, kStatusKind);
+                if (lane == 0) report(a, kStatusKind);
                 break;
             }
             // ---- eigen-table tile: one class x 32 energies ----------------------------
@@ -212,7 +224,7 @@ static __global__ void __launch_bounds__(kBlock, blocks_per_sm(kKinds)) batch_ke
             if (!(c >= 0 && c < P.ncls && span_ok(P.e_off, P.ne, a.n_energies) &&
                   span_ok(P.tab_off, (long long)P.ncls * P.ne_pad * kMixFields, a.n_tables) &&
                   P.ne <= P.ne_pad)) {
-                if (lane == 0) report(a.status, kStatusBounds);
+                if (lane == 0) report(a, kStatusBounds);
                 __syncwarp();
                 if (kPhases == kPhaseAll && lane == 0) atomicAdd(a.done_a + p, 1);  // no waiter is left hanging
                 t = __shfl_sync(0xffffffffu, next, 0);
@@ -233,7 +245,7 @@ static __global__ void __launch_bounds__(kBlock, blocks_per_sm(kKinds)) batch_ke
             }
         } else if (P.kind == 0) {
             if (!(kKinds & kAtmos)) {
-                if (lane == 0) report(a.status, kStatusKind);
+                if (lane == 0) report(a, kStatusKind);
                 break;
             }
             // ---- atmospheric bin tile: rows_per_tile rows x 32 energies ------------------
@@ -248,7 +260,7 @@ static __global__ void __launch_bounds__(kBlock, blocks_per_sm(kKinds)) batch_ke
                     while (*done < need) {
                         __nanosleep(256);
                         if (++it > kSpinLimit || global_timer_ns() - t0 > kWaitLimitNs) {
-                            report(a.status, kStatusWaitLimit);  // tables never completed: report
+                            report(a, kStatusWaitLimit);  // tables never completed: report
                             break;
                         }
                     }
@@ -276,7 +288,7 @@ static __global__ void __launch_bounds__(kBlock, blocks_per_sm(kKinds)) batch_ke
                 tile_ok = tile_ok && nseg >= 1 && nseg <= kMaxSegments && nseg <= P.ncls &&
                           span_ok(s0, nseg, a.n_seg);
                 if (!tile_ok) {
-                    if (lane == 0) report(a.status, kStatusBounds);
+                    if (lane == 0) report(a, kStatusBounds);
                     break;
                 }
 #endif
@@ -292,7 +304,7 @@ static __global__ void __launch_bounds__(kBlock, blocks_per_sm(kKinds)) batch_ke
             }
         } else {
             if (!(kKinds & kBeam)) {
-                if (lane == 0) report(a.status, kStatusKind);
+                if (lane == 0) report(a, kStatusKind);
                 break;
             }
             // ---- beam tile: beam_chunk x 32 energies, every baseline --------------------
@@ -302,7 +314,7 @@ static __global__ void __launch_bounds__(kBlock, blocks_per_sm(kKinds)) batch_ke
 #ifdef CP3_DEVICE_CHECKS
             if (!(span_ok(P.out_off, 9LL * P.nrows * P.ne, a.n_out) &&
                   span_ok(P.e_off, P.ne, a.n_energies))) {
-                if (lane == 0) report(a.status, kStatusBounds);
+                if (lane == 0) report(a, kStatusBounds);
                 t = __shfl_sync(0xffffffffu, next, 0);
                 continue;
             }

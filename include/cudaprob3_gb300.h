@@ -291,7 +291,9 @@ int cp3_batch_run(cp3_batch* b, void* stream);
  * results in calculateProbabilities.) */
 int cp3_batch_run_to_host(cp3_batch* b, void* dst, int n_pieces, void* stream);
 /* Waits for the last run and for everything queued on the batch's own stream (result
- * copies with a NULL stream); *ms = the run's device time. */
+ * copies with a NULL stream); *ms = the run's device time.  CP3_ERR_CUDA where the last run
+ * reported a failure; an earlier one's, queued before it without a wait between, is not
+ * reported. */
 int cp3_batch_synchronize(cp3_batch* b, double* ms);
 /* Device pointer and float count of one problem's result. */
 int cp3_batch_result(cp3_batch* b, int id, const float** ptr, size_t* count);

@@ -62,6 +62,35 @@ def test_runs_leave_their_counters_cleared(kinds, split):
     assert same(results(), other)
 
 
+@pytest.mark.parametrize("last_fails", [False, True])
+def test_a_status_belongs_to_its_run(last_fails):
+    """Two runs queued without a wait between them, one of which times out (2 s): what the wait
+    after them reports is the last one's end, whichever of the two failed."""
+    import time
+    import torch
+    from cudaprob3_gb300._abi import CP3Error
+    b = Batch(0)
+    b.set_earth(*earth.PREM_4LAYER, 22.0)
+    b.set_params(b.add_atmos(earth.cosine_grid(24), earth.log_energy_grid(40)), earth.NOMINAL, False)
+    b.commit()
+    b.run()
+    b.synchronize()
+    want = b.result(0).copy()
+    s = torch.cuda.Stream()
+    b.debug_withhold_tables(not last_fails)
+    b.run(s.cuda_stream)
+    time.sleep(0.3)  # the first run has read its descriptors
+    b.debug_withhold_tables(last_fails)
+    b.run()
+    if last_fails:
+        with pytest.raises(CP3Error, match="did not complete"):
+            b.synchronize()
+        b.debug_withhold_tables(False)
+        b.run()
+    b.synchronize()
+    assert np.array_equal(b.result(0), want)
+
+
 def test_a_run_cannot_be_captured():
     """Refused with its reason, and the batch runs on afterwards."""
     import torch
