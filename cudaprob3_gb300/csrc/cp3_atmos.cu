@@ -458,10 +458,9 @@ __global__ void __launch_bounds__(32 * kFxWarps, 4)
     double* o = out + (size_t)ic * ne + ie;
     const size_t plane = (size_t)nc * ne;
     if ((bad >> 20) == 0) {
-        const unsigned long long w = j == 0 ? total[0] : j == 1 ? total[1] : total[2];
-        o[(size_t)(3 * j) * plane] = fx_averaged(P[0], w);
-        o[(size_t)(3 * j + 1) * plane] = fx_averaged(P[1], w);
-        o[(size_t)(3 * j + 2) * plane] = fx_averaged((1LL << 62) - P[0] - P[1], w);
+        o[(size_t)(3 * j) * plane] = fx_to_double(P[0]);
+        o[(size_t)(3 * j + 1) * plane] = fx_to_double(P[1]);
+        o[(size_t)(3 * j + 2) * plane] = fx_to_double((1LL << 62) - P[0] - P[1]);
     } else if (j == 0) {  // (the three agree on it)
         atmos_bin_out_of_range(&p, energies[ie], s_len, s_rho, nseg - 1, av, ic, nc, ie, ne, o);
     }

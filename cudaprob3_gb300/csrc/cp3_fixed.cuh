@@ -77,20 +77,24 @@ CP3_HD double fx_bits_to_double(long long b) {
 #endif
 }
 
-// A fixed-point number as a double (within 2^-50 below zero: zero).
-CP3_HD double fx_to_double(long long v) {
-    if (v <= 0 && v > -4096) return 0.0;
-    return fx_bits_to_double(fx_bits((double)v) - (62LL << 52));
+// A layer's phases are of length 1 to the 2^-56 of their sines and cosines, and the palindrome takes
+// a chain twice, so that a probability or a difference of some from 1 leaves [0, 1] by up to about
+// M 2^-54 on M shells: -1.1e-15 was met on 59 shells and -2.2e-15 on 128, with theta12 = theta13 = 0,
+// where a channel is exactly zero.  A probability as a double, in [0, 1]:
+constexpr long long kFxOne = 1LL << 62;
+CP3_HD double fx_probability(long long v) {
+    if (v <= 0) return 0.0;
+    return fx_bits_to_double(fx_bits((double)(v < kFxOne ? v : kFxOne)) - (62LL << 52));
 }
 
-// A probability as a double, in [0, 1].  A layer's phases are of length 1 to the 2^-56 of their
-// sines and cosines, and the palindrome takes a chain twice, so that a probability or a difference
-// of some from 1 leaves the interval by up to about M 2^-54 on M shells: -1.1e-15 was met on 59
-// shells and -2.2e-15 on 128, with theta12 = theta13 = 0, where a channel is exactly zero.
-CP3_HD double fx_probability(long long v) {
-    constexpr long long one = 1LL << 62;
-    if (v <= 0) return 0.0;
-    return fx_bits_to_double(fx_bits((double)(v < one ? v : one)) - (62LL << 52));
+// An averaged one: the end of the interval within that rounding (2^-47) outside it, else what it is.
+// Weights that are no distribution, and the jump of the sinc series (fx_sinc) where two states are
+// nearly degenerate, take it out.
+CP3_HD double fx_to_double(long long v) {
+    constexpr long long window = 1LL << 15;
+    if (v <= 0 && v > -window) return 0.0;
+    if (v > kFxOne && v < kFxOne + window) return 1.0;
+    return fx_bits_to_double(fx_bits((double)v) - (62LL << 52));
 }
 
 // Accumulators: fxacc for at most three products of unit-vector entries (two of complex ones),
@@ -1093,13 +1097,6 @@ CP3_HD void fx_check_weights(const unsigned long long total[3], unsigned int& ba
 #pragma unroll
     for (int f = 0; f < 3; f++)
         if (total[f] > (5ULL << 52)) bad |= 1u << 20;
-}
-
-// An averaged probability of an initial flavour whose weights add up (in magnitude) to `total`: in
-// [0, 1] where that is 1, but for its rounding (twenty normalised weights: 40 units of 2^-54);
-// weights that add up to more can take it out of the interval.
-CP3_HD double fx_averaged(long long v, unsigned long long total) {
-    return total <= (1ULL << 54) + 64 ? fx_probability(v) : fx_to_double(v);
 }
 
 // One averaged bin's probabilities of the initial flavour j, from these rows, the air layer's

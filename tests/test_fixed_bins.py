@@ -197,6 +197,24 @@ def test_gpu_results_are_probabilities(shells, nb):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("nb", [1, 2, 20])
+def test_gpu_averages_with_negative_weights(oracle, nb):
+    """Weights below zero can take an averaged value out of [0, 1], which it keeps."""
+    from tests.test_gpu_averaging import run_avg
+    cz, en = np.linspace(-1, 0.4, 7), earth.log_energy_grid(33)
+    prob = np.random.default_rng(12).uniform(0.1, 1.0, (2, 3, len(en), len(cz), nb))
+    prob /= prob.sum(axis=-1, keepdims=True)
+    prob[:, :, ::2, :, 0] *= -1.0
+    edges = np.linspace(3.0, 60.0, nb + 1)
+    m = earth.gaussian_sets(2, seed=10)[1]
+    mix6 = [m.theta12, m.theta13, m.theta23, m.dcp, m.dm12sq, m.dm23sq]
+    ref = oracle.atmos(omix(m, False), False, cz, en, *earth.PREM_4LAYER, 20.0, avg=(nb, prob.ravel(), edges))
+    assert ref.min() < -0.01 or nb == 20  # (with twenty it stays inside)
+    got = run_avg("fp64", mix6, 1, False, cz, en, *earth.PREM_4LAYER, 20.0, nb, prob.ravel(), edges)
+    assert np.abs(got - ref).max() <= 1e-12
+
+
+@pytest.mark.gpu
 def test_gpu_out_of_range_bins():
     """A NaN energy gives NaN in its own column and leaves the others as they are.  An energy too
     low for the fixed-point reduction takes the FP64 path: its phases (1e18 rad) have lost every
