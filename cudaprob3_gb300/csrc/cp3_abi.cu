@@ -79,6 +79,8 @@ struct cp3_propagator {
     DevBuf<int> d_seg_off;
     DevBuf<double> d_seg_len, d_cls_rho, d_seg_rho;
     DevBuf<double> d_ph_prob, d_ph_mid, d_ph_wid;  // production-height averaging (FP64)
+    DevBuf<signed char> d_ph_scale;                // of weights that are no distribution
+    bool avg_scaled = false;
     DevBuf<float> d_ph_prob_f, d_ph_hw;            // ... and its float form (mixed)
     DevBuf<float2> d_ph_hm;
     bool avg_dirty = true;
@@ -354,14 +356,24 @@ int prepare_averaging(cp3_propagator* h, AvgArrays* av, AvgMixed* avm) {
         // one (type, flavour) slab [ne][nc bins] at a time, through a buffer freed at the end
         DevBuf<double> raw;
         const size_t slab = cells * h->ne;
-        CP3_CUDA(h, raw.reserve(slab), "allocate averaging");
+        CP3_CUDA(h, raw.reserve(slab + 1), "allocate averaging");
         for (int k = 0; k < 6; k++) {
             CP3_CUDA(h, cudaMemcpyAsync(raw.ptr, h->avg_prob.data() + k * slab, sizeof(double) * slab,
                                         cudaMemcpyHostToDevice, h->stream), "upload averaging");
             void* dst = mixed ? (void*)(h->d_ph_prob_f.ptr + k * slab) : (void*)(h->d_ph_prob.ptr + k * slab);
             CP3_CUDA(h, launch_weights_transpose(raw.ptr, h->ne, (long long)cells, dst, mixed, h->stream), "transpose averaging");
         }
+        int scaled = 0;
+        if (!mixed) {  // weights that are no distribution: their scales, used where one is not zero
+            int* any = reinterpret_cast<int*>(raw.ptr + slab);
+            CP3_CUDA(h, h->d_ph_scale.reserve(6 * (size_t)h->nc * h->ne), "allocate averaging");
+            CP3_CUDA(h, cudaMemsetAsync(any, 0, sizeof(int), h->stream), "scale averaging");
+            CP3_CUDA(h, launch_weight_scales(h->d_ph_prob.ptr, h->nc, nb, h->ne, h->d_ph_scale.ptr, any, h->stream),
+                     "scale averaging");
+            CP3_CUDA(h, cudaMemcpyAsync(&scaled, any, sizeof(int), cudaMemcpyDeviceToHost, h->stream), "scale averaging");
+        }
         CP3_CUDA(h, cudaStreamSynchronize(h->stream), "upload averaging");
+        h->avg_scaled = scaled != 0;
         h->avg_dirty = false;
     }
     if (mixed) {
@@ -374,6 +386,7 @@ int prepare_averaging(cp3_propagator* h, AvgArrays* av, AvgMixed* avm) {
     av->prob = h->d_ph_prob.ptr;
     av->mid = h->d_ph_mid.ptr;
     av->wid = h->d_ph_wid.ptr;
+    av->scale = h->avg_scaled ? h->d_ph_scale.ptr : nullptr;
     av->n_bins = nb;
     return CP3_OK;
 }

@@ -366,12 +366,19 @@ __global__ void __launch_bounds__(32 * kFxWarps, 3)
 // heights: 49 us (688 in FP64 arithmetic with the weights read across energies; 59 with the
 // layers solved in place and one warp for the last part; 53 and 61 with three and five blocks
 // an SM).
-template <bool kTable>
+//   kScaled: a cell's weights are taken times a power of two (fx_weight_scale), which the cross
+// terms get back at the end.  Chosen where a cell needs it, since it costs 3 us of a call; through
+// the FP64 path such weights cost ten times that and, on deep models, more than FP64 kernels did
+// (a call with weights that add up to 3, so / FP64 path / FP64 kernels: PREM-12, 200 x 150, 20
+// heights 71 / 649 / 790 us; PREM-12, 300 x 300, one height 92 / 669 / 357; 59 shells, 200 x 150,
+// 20 heights 125 / 1393 / 1092).
+template <bool kTable, bool kScaled>
 __global__ void __launch_bounds__(32 * kFxWarps, 4)
     atmos_fx_avg_kernel(const __grid_constant__ OscParams p, const double* __restrict__ energies, int ne,
                         int ne_pad, const int2* __restrict__ table, int ncls, const int* __restrict__ seg_off,
                         const double* __restrict__ seg_len, const double* __restrict__ rho,
-                        int ic0, int nc, AvgInput av, double* __restrict__ out) {
+                        int ic0, int nc, AvgInput av, double* __restrict__ out,
+                        const signed char* __restrict__ weight_scale) {
     __shared__ longlong2 s_trig[kTrigSize];
     __shared__ double s_len[kMaxSegments], s_rho[kMaxSegments];
     __shared__ long long s_sum[kFxWarps][21][32];
@@ -397,8 +404,16 @@ __global__ void __launch_bounds__(32 * kFxWarps, 4)
         const double rate[2] = {col.rate(0, 0), col.rate(0, 1)};
         const size_t cell = (size_t)ic * av.nb;
         FxShift sum;
-        fx_shift_sums(rate, wv - first, kFxWarps - first, av.nb, av.prob + ((size_t)av.type * 3 * nc * av.nb + cell) * ne + ie,
-                      (size_t)nc * av.nb * ne, (size_t)ne, av.mid + cell, av.wid + cell, s_trig, bad, sum);
+        int scale[3];
+        if (kScaled)
+#pragma unroll
+            for (int f = 0; f < 3; f++) {
+                scale[f] = weight_scale[((size_t)(av.type * 3 + f) * nc + ic) * ne + ie];
+                if (scale[f] == kFxNoScale) bad |= 1u << 20;
+            }
+        fx_shift_sums<kScaled>(rate, wv - first, kFxWarps - first, av.nb,
+                               av.prob + ((size_t)av.type * 3 * nc * av.nb + cell) * ne + ie, (size_t)nc * av.nb * ne,
+                               (size_t)ne, av.mid + cell, av.wid + cell, s_trig, bad, sum, scale);
 #pragma unroll
         for (int f = 0; f < 3; f++) {
             s_sum[wv][18 + f][lane] = (long long)sum.total[f];
@@ -453,17 +468,45 @@ __global__ void __launch_bounds__(32 * kFxWarps, 4)
 #pragma unroll
     for (int f = 0; f < 9; f++) row[f] = col.extra(kFxV0 + f);
     const double rate[2] = {col.rate(0, 0), col.rate(0, 1)};
-    long long P[2];
-    fx_average(j, a, row, rate, s_len[0], s_trig, t, bad, P);
+    long long P[2], cross[2];
+    fx_average(j, a, row, rate, s_len[0], s_trig, t, bad, P, cross);
     double* o = out + (size_t)ic * ne + ie;
     const size_t plane = (size_t)nc * ne;
-    if ((bad >> 20) == 0) {
+    const int scale = kScaled ? weight_scale[((size_t)(av.type * 3 + j) * nc + ic) * ne + ie] : 0;
+    if ((bad >> 20) == 0 && scale == 0) {
+#pragma unroll
+        for (int i = 0; i < 2; i++) P[i] += 2 * cross[i];
         o[(size_t)(3 * j) * plane] = fx_to_double(P[0]);
         o[(size_t)(3 * j + 1) * plane] = fx_to_double(P[1]);
-        o[(size_t)(3 * j + 2) * plane] = fx_to_double((1LL << 62) - P[0] - P[1]);
+        o[(size_t)(3 * j + 2) * plane] = fx_to_double(kFxOne - P[0] - P[1]);
+    } else if (kScaled && (bad >> 20) == 0) {  // the cross terms take the weights' scale back
+        double d[2];
+#pragma unroll
+        for (int i = 0; i < 2; i++) d[i] = ldexp((double)P[i], -62) + ldexp((double)cross[i], scale - 61);
+        o[(size_t)(3 * j) * plane] = d[0];
+        o[(size_t)(3 * j + 1) * plane] = d[1];
+        o[(size_t)(3 * j + 2) * plane] = 1.0 - d[0] - d[1];
     } else if (j == 0) {  // (the three agree on it)
         atmos_bin_out_of_range(&p, energies[ie], s_len, s_rho, nseg - 1, av, ic, nc, ie, ne, o);
     }
+}
+
+// fx_weight_scale of the weights [2 x 3][nc][nb][ne], a cell a thread.
+__global__ void __launch_bounds__(kBlock)
+    weight_scales_kernel(const double* __restrict__ prob, long long cells, int nb, int ne,
+                         signed char* __restrict__ scale, int* __restrict__ any) {
+    const long long i = (long long)blockIdx.x * kBlock + threadIdx.x;
+    if (i >= cells) return;
+    const double* w = prob + (size_t)(i / ne) * nb * ne + i % ne;
+    double total = 0.0, largest = 0.0;
+    for (int b = 0; b < nb; b++) {
+        const double v = fabs(w[(size_t)b * ne]);
+        total += v;
+        largest = fmax(largest, v);
+    }
+    const int s = fx_weight_scale(total, largest);
+    scale[i] = (signed char)s;
+    if (s != 0) *any = 1;  // (every writer writes the same)
 }
 
 // Mixed atmospheric bins (the physics of calculate_atmos rearranged for FP32: see
@@ -529,15 +572,16 @@ cudaError_t launch_atmos_fx_inline(const OscParams& p, const double* energies, i
     if (ne <= 0 || n_cosines <= 0) return cudaSuccess;
     const AvgInput av{avg.prob, avg.mid, avg.wid, avg.n_bins, p.anti};
     const bool averaged = avg.n_bins > 0;
+    const auto kernel = avg.scale ? (ncls > 0 ? atmos_fx_avg_kernel<true, true> : atmos_fx_avg_kernel<false, true>)
+                                  : (ncls > 0 ? atmos_fx_avg_kernel<true, false> : atmos_fx_avg_kernel<false, false>);
     const int rows = averaged ? 1 : kFxWarps;  // of a block
     const int end = rr.end < 0 ? n_cosines : rr.end, step = kMaxGridY * rows;
     for (int ic0 = rr.begin; ic0 < end; ic0 += step) {
         const int ic1 = end - ic0 < step ? end : ic0 + step;
         dim3 grid((ne + 31) / 32, (ic1 - ic0 + rows - 1) / rows);
         if (averaged)
-            launch_early(rr.early && ic0 == rr.begin, ncls > 0 ? atmos_fx_avg_kernel<true> : atmos_fx_avg_kernel<false>,
-                         grid, 32 * kFxWarps, s, p, energies, ne, pad_energies(ne), table, ncls > 0 ? ncls : 1, seg_off,
-                         seg_len, rho, ic0, n_cosines, av, out);
+            launch_early(rr.early && ic0 == rr.begin, kernel, grid, 32 * kFxWarps, s, p, energies, ne,
+                         pad_energies(ne), table, ncls > 0 ? ncls : 1, seg_off, seg_len, rho, ic0, n_cosines, av, out, avg.scale);
         else
             launch_early(rr.early && ic0 == rr.begin, atmos_fx_inline_kernel, grid, 32 * kFxWarps, s, p, energies, ne,
                          pad_energies(ne), table, seg_off, seg_len, rho, ic0, ic1, n_cosines, out);
@@ -874,6 +918,14 @@ cudaError_t launch_weights_transpose(const double* src, int rows, long long cols
         weights_transpose_kernel<float><<<(unsigned)blocks, block, 0, s>>>(src, rows, cols, (float*)dst);
     else
         weights_transpose_kernel<double><<<(unsigned)blocks, block, 0, s>>>(src, rows, cols, (double*)dst);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_weight_scales(const double* prob, int nc, int n_bins, int ne, signed char* scale,
+                                 int* any, cudaStream_t s) {
+    const long long cells = 6LL * nc * ne, blocks = (cells + kBlock - 1) / kBlock;
+    if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
+    weight_scales_kernel<<<(unsigned)blocks, kBlock, 0, s>>>(prob, cells, n_bins, ne, scale, any);
     return cudaGetLastError();
 }
 

@@ -980,6 +980,22 @@ CP3_HD fx fx_sinc(double x) {
     return fx_split((1LL << 62) - fx_sum(c));
 }
 
+// Weights that are no distribution: the smallest s >= 0 for which the weights times 2^-s are at
+// most 1 and add up to less than 5/4 (total, largest: of the magnitudes; the margin covers the sum's
+// rounding); kFxNoScale where there is none, and the bin takes the FP64 path.
+constexpr int kFxNoScale = -1;
+CP3_HD int fx_weight_scale(double total, double largest) {
+    constexpr double most = 1.2499999;
+    if (!(total <= 1e30)) return kFxNoScale;
+    if (largest <= 1.0 && total <= most) return 0;
+    int et, el;
+    const double mt = frexp(total, &et), ml = frexp(largest, &el);  // m 2^e, 1/2 <= m < 1
+    if (mt <= 0.5 * most) et--;
+    if (ml <= 0.5) el--;
+    const int s = et > el ? et : el;
+    return s > 0 ? s : 0;
+}
+
 // The sums t over some of a bin's heights (b0, b0 + step, ...), and the sums of the weights'
 // magnitudes (54 fraction bits).  The products' leading and cross terms accumulate over the
 // heights as they are, with the low words cut to 27 bits (2^-57): the cross terms of 20 heights
@@ -991,10 +1007,12 @@ struct FxShift {
 };
 
 // prob, mid, wid: the height bins' probabilities of the three initial flavours (b-th at
-// prob[f * flavour + b * stride]), their mid shifts and widths in km.
+// prob[f * flavour + b * stride]), their mid shifts and widths in km.  kScaled: flavour f's are
+// taken times 2^-scale[f].
+template <bool kScaled = false>
 CP3_HD void fx_shift_sums(const double rate[2], int b0, int step, int nb, const double* prob, size_t flavour,
                           size_t stride, const double* mid, const double* wid, const longlong2* trig,
-                          unsigned int& bad, FxShift& o) {
+                          unsigned int& bad, FxShift& o, const int* scale = nullptr) {
     const double pr[2] = {rate[0] * M_PI, rate[1] * M_PI};
 #pragma unroll 1
     for (int b = b0; b < nb; b += step) {
@@ -1025,8 +1043,10 @@ CP3_HD void fx_shift_sums(const double rate[2], int b0, int step, int nb, const 
         for (int f = 0; f < 3; f++) {
             const double p = weight[f];
             const long long pb = fx_bits(p) & 0x7fffffffffffffffLL;
-            if (pb > 0x3ff0000000000000LL) bad |= 1u << 20;  // above 1, or not a number
-            const long long pv = pb > 0x3ff0000000000000LL ? 0 : fx_scaled(p, 1023);
+            const int one = kScaled ? 1023 + scale[f] : 1023;  // exponent of the largest
+            const bool above = pb > (long long)one << 52;      // or not a number
+            if (above) bad |= 1u << 20;
+            const long long pv = above ? 0 : fx_scaled(p, one);
             o.total[f] += (unsigned long long)(pv < 0 ? -pv : pv) >> 8;
             fx pf = fx_split(pv);
             pf.l >>= 5;
@@ -1092,7 +1112,7 @@ CP3_HD void fx_air_rows(const FxColumn& t, const double* len, int M, const longl
     }
 }
 
-// Weights that add up to more than 5/4 leave the range of the factors t.
+// Weights (as scaled) that add up to more than 5/4 leave the range of the factors t.
 CP3_HD void fx_check_weights(const unsigned long long total[3], unsigned int& bad) {
 #pragma unroll
     for (int f = 0; f < 3; f++)
@@ -1100,10 +1120,12 @@ CP3_HD void fx_check_weights(const unsigned long long total[3], unsigned int& ba
 }
 
 // One averaged bin's probabilities of the initial flavour j, from these rows, the air layer's
-// own (fx_rows) and its rates, and j's shift factors t: P[i] that of j -> i, i = e, mu.  The
-// tau row's products follow from the others': the columns of W U_0 are orthonormal.
+// own (fx_rows) and its rates, and j's shift factors t: base[i] + 2 cross[i] is that of j -> i,
+// i = e, mu, and cross is proportional to t.  The tau row's products follow from the others': the
+// columns of W U_0 are orthonormal.
 CP3_HD void fx_average(int j, const cfx a[2][3], const fx row[9], const double rate[2], double air_km,
-                       const longlong2* trig, const cfx t[3], unsigned int& bad, long long P[2]) {
+                       const longlong2* trig, const cfx t[3], unsigned int& bad, long long base[2],
+                       long long cross[2]) {
     cfx e[3];  // e_k conj(e_q) of the pairs (1,0), (2,0), (2,1)
     fx_layer(rate, air_km, trig, e, bad);
     e[2] = fx_cmul(cfx{e[0].re, fx_neg(e[0].im)}, e[1]);
@@ -1133,7 +1155,17 @@ CP3_HD void fx_average(int j, const cfx a[2][3], const fx row[9], const double r
         }
     }
 #pragma unroll
-    for (int i = 0; i < 2; i++) P[i] = fx_sum(s[i]) + 2 * fx_sum(x[i]);
+    for (int i = 0; i < 2; i++) {
+        base[i] = fx_sum(s[i]);
+        cross[i] = fx_sum(x[i]);
+    }
+}
+CP3_HD void fx_average(int j, const cfx a[2][3], const fx row[9], const double rate[2], double air_km,
+                       const longlong2* trig, const cfx t[3], unsigned int& bad, long long P[2]) {
+    long long cross[2];
+    fx_average(j, a, row, rate, air_km, trig, t, bad, P, cross);
+#pragma unroll
+    for (int i = 0; i < 2; i++) P[i] += 2 * cross[i];
 }
 
 }  // namespace cp3

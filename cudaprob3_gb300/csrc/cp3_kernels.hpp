@@ -40,6 +40,7 @@ struct AvgArrays {
     const double* mid = nullptr;   // [nc][n_bins] mid path-length shift of each bin, km (0 where the
                                    // air segment has zero length)
     const double* wid = nullptr;   // [nc][n_bins] bin width, km (0 likewise)
+    const signed char* scale = nullptr;  // [2][3][nc][ne] fx_weight_scale, where one is not zero
     int n_bins = 0;
 };
 
@@ -127,6 +128,9 @@ cudaError_t launch_atmos_mixed_inline(const OscParams& p, const double* energies
                                       const double* seg_rho, int n_cosines, float* out,
                                       cudaStream_t s, RowRange rr = RowRange{});
 
+// The weights' scales [2][3][nc][ne] (fx_weight_scale); *any is set where one is not zero.
+cudaError_t launch_weight_scales(const double* prob, int nc, int n_bins, int ne, signed char* scale,
+                                 int* any, cudaStream_t s);
 // A matrix [rows][cols] of doubles transposed to [cols][rows], as floats or doubles.
 cudaError_t launch_weights_transpose(const double* src, int rows, long long cols, void* dst,
                                      bool to_float, cudaStream_t s);

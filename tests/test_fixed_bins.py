@@ -173,6 +173,71 @@ def test_gpu_averaged_bins_at_the_edges_and_out_of_range(oracle, nb, nc, ne):
             assert np.abs(got - ref).max() <= tol * max(1.0, scale)
 
 
+WEIGHT_SUMS = (1.0, 1.25, 1.2500001, 2.5, 3.0, 17.0, 1e6, 0.0, 1e-9)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("poly", [False, True])
+@pytest.mark.parametrize("nb", [1, 2, 20])
+def test_gpu_averaged_bins_with_weights_that_are_no_distribution(oracle, poly, nb):
+    """Every cell's weights of a sum of its own, some negative, one cell with a weight that is not
+    a number: each cell within the bar times its own sum, the NaN in its own cell alone."""
+    from tests.test_gpu_averaging import run_avg
+    r, abc, ye = ((earth.PREM_4LAYER_QUAD_V2[0], earth.PREM_4LAYER_QUAD_V2[1:4], earth.PREM_4LAYER_QUAD_V2[4]) if poly
+                  else (earth.PREM_12LAYER[0], (earth.PREM_12LAYER[1],) * 3, earth.PREM_12LAYER[2]))
+    cz, en = np.linspace(-1, 0.4, 9), earth.log_energy_grid(37)
+    rng = np.random.default_rng(11)
+    prob = rng.uniform(0.1, 1.0, (2, 3, len(en), len(cz), nb))
+    prob /= prob.sum(axis=-1, keepdims=True)
+    sums = rng.choice(WEIGHT_SUMS, prob.shape[:-1])
+    prob *= sums[..., None]
+    prob[:, :, ::3, :, 0] *= -1.0
+    edges = np.linspace(3.0, 60.0, nb + 1)
+    m = earth.gaussian_sets(2, seed=10)[1]
+    mix6 = [m.theta12, m.theta13, m.theta23, m.dcp, m.dm12sq, m.dm23sq]
+    args = (r, None if poly else abc[0], ye, 20.0)
+    for anti in (False, True):
+        ref = oracle.atmos(omix(m, anti), anti, cz, en, *args, poly_abc=abc if poly else None, avg=(nb, prob.ravel(), edges))
+        # [cosine][energy][channel], the initial flavour of a channel its cell's
+        bar = 1e-12 * np.maximum(1.0, np.repeat(np.transpose(sums[int(anti)], (2, 1, 0)), 3, axis=2))
+        run = lambda w: run_avg("fp64", mix6, -1 if anti else 1, anti, cz, en, *args, nb, w.ravel(), edges,
+                                abc if poly else None)
+        got = run(prob)
+        assert (np.abs(got - ref) <= bar).all()
+        bad = prob.copy()
+        bad[int(anti), 1, 5, 3, 0] = np.nan
+        got = run(bad)
+        assert np.isnan(got[3, 5, 3:6]).all()
+        got[3, 5, 3:6] = ref[3, 5, 3:6]
+        assert (np.abs(got - ref) <= bar).all()
+
+
+@pytest.mark.gpu
+def test_gpu_weights_that_are_no_distribution_run_on_the_common_kernel():
+    """They cost what a distribution's cost (the FP64 path took ten times that)."""
+    import time
+    from cudaprob3_gb300 import AtmosCudaPropagatorSingle
+    nc, ne, nb, m = 200, 150, 20, earth.NOMINAL
+    best = {}
+    for scale in (1.0, 3.0):
+        p = AtmosCudaPropagatorSingle(0, nc, ne, precision="fp64")
+        p.setEnergyList(earth.log_energy_grid(ne))
+        p.setCosineList(earth.cosine_grid(nc))
+        p.setMNSMatrix(m.theta12, m.theta13, m.theta23, m.dcp, 1)
+        p.setNeutrinoMasses(m.dm12sq, m.dm23sq)
+        p.setDensity(*earth.PREM_12LAYER)
+        p.setProductionHeight(22.0)
+        p.SetNumberOfProductionHeightBinsForAveraging(nb)
+        p.setProductionHeightList(np.full(6 * nc * ne * nb, scale / nb), np.linspace(5.0, 45.0, nb + 1))
+        times = []
+        for _ in range(20):
+            t = time.perf_counter()
+            p.calculateProbabilities(0)
+            times.append(time.perf_counter() - t)
+        best[scale] = min(times)
+    assert best[3.0] < 3.0 * best[1.0], best
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("shells", [59, 128])
 @pytest.mark.parametrize("nb", [0, 1, 20])
