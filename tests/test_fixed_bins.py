@@ -82,6 +82,20 @@ def test_host_bins_against_oracle(host, oracle, shells, h):
                 assert np.abs(got - ref).max() <= 1e-12
 
 
+@pytest.mark.parametrize("dm23sq", [1e-10, 2e-11, -1e-11])
+def test_nearly_equal_levels_stay_in_fixed_point(host, oracle, dm23sq):
+    """Two vacuum levels a millionth of the spread apart: the FP64 vectors of the two are not
+    orthogonal after one step, which sent every bin to the FP64 path.  The roots of a nearly double
+    level are off by sqrt(2^-53) of the spread, 8e-13 eV^2: 3e-7 rad over 13 000 km at 0.1 GeV."""
+    m = earth.NOMINAL
+    m = type(m)(m.theta12, m.theta13, m.theta23, m.dcp, m.dm12sq, dm23sq)
+    cz, en = np.linspace(-1, 0.4, 15), np.logspace(-1, 2, 13)
+    for anti in (False, True):
+        got, outside = host_bins(host, m, anti, cz, en, earth.PREM_4LAYER, 22.0, refine=0)
+        assert outside == 0
+        assert np.abs(got - oracle.atmos(omix(m, anti), anti, cz, en, *earth.PREM_4LAYER, 22.0)).max() <= 3e-7
+
+
 @pytest.mark.parametrize("shells", [1, 4, 59, 128])
 @pytest.mark.parametrize("theta12,theta13", [(0.0, 0.0), (0.0, 0.15), (0.59, 0.0)])
 def test_host_bins_are_probabilities(host, shells, theta12, theta13):
