@@ -78,11 +78,12 @@ struct cp3_propagator {
     DevBuf<float2> d_energies_df, d_cls_rho_df;  // mixed kernels: (hi, lo) pairs split here
     DevBuf<int> d_seg_off;
     DevBuf<double> d_seg_len, d_cls_rho, d_seg_rho;
-    DevBuf<double> d_ph_prob, d_ph_mid, d_ph_wid;  // production-height averaging (FP64)
+    DevBuf<double> d_ph_prob, d_ph_geom;           // production-height averaging (FP64)
     DevBuf<signed char> d_ph_scale;                // of weights that are no distribution
+    DevBuf<double> d_ph_raw;                       // the weights as the client lays them out
     bool avg_scaled = false;
-    DevBuf<float> d_ph_prob_f, d_ph_hw;            // ... and its float form (mixed)
-    DevBuf<float2> d_ph_hm;
+    DevBuf<float> d_ph_prob_f;                     // ... and its float form (mixed)
+    DevBuf<float2> d_ph_geom_df;
     bool avg_dirty = true;
     DevBuf<float2> d_seg_len_df;
     DevBuf<int2> d_table_fx;
@@ -317,6 +318,11 @@ int prepare_atmos(cp3_propagator* h) {
     return CP3_OK;
 }
 
+// The weights are uploaded in pieces of at most this size (or one slab), through a buffer that is
+// kept up to that.  New weights of 40 x 40 bins and 3 heights, mixed, with the pass on them: 53 us
+// (102 slab by slab, the buffer allocated each time); 100 x 100 bins and 20 heights 140 (395).
+constexpr size_t kMaxWeightUpload = size_t(16) << 20;
+
 // Averaging inputs: the client's probabilities [2][3][ne][nc][bins], transposed on the device so
 // that consecutive energies are contiguous (the kernels' warps run over energies), and per
 // (cosine, bin) the mid path-length shift and the width in km; zero where the air segment is
@@ -330,42 +336,42 @@ int prepare_averaging(cp3_propagator* h, AvgArrays* av, AvgMixed* avm) {
         std::vector<double> shifts;
         production_height_shifts(h->cosines.data(), h->nc, h->height_cm, h->avg_edges.data(), nb, &shifts);
         const size_t cells = (size_t)h->nc * nb;
-        std::vector<double> mid(cells), wid(cells);
+        std::vector<double> geom(2 * cells);  // the mid shifts, then the widths
         for (int ic = 0; ic < h->nc; ic++)
             for (int b = 0; b < nb; b++) {
                 const double h0 = shifts[(size_t)ic * (nb + 1) + b], h1 = shifts[(size_t)ic * (nb + 1) + b + 1];
                 const bool zero = h->traj.air_cm[ic] == 0.0;
-                mid[(size_t)ic * nb + b] = zero ? 0.0 : 0.5 * (h1 + h0) / kKm2Cm;
-                wid[(size_t)ic * nb + b] = zero ? 0.0 : (h1 - h0) / kKm2Cm;
+                geom[(size_t)ic * nb + b] = zero ? 0.0 : 0.5 * (h1 + h0) / kKm2Cm;
+                geom[cells + (size_t)ic * nb + b] = zero ? 0.0 : (h1 - h0) / kKm2Cm;
             }
-        if (mixed) {
-            const std::vector<float2> hm = split_pairs(mid.data(), cells);
-            const std::vector<float> hw(wid.begin(), wid.end());
-            CP3_CUDA(h, h->d_ph_hm.reserve(cells), "allocate averaging");
-            CP3_CUDA(h, h->d_ph_hw.reserve(cells), "allocate averaging");
-            CP3_CUDA(h, cudaMemcpy(h->d_ph_hm.ptr, hm.data(), sizeof(float2) * cells, cudaMemcpyHostToDevice), "upload averaging");
-            CP3_CUDA(h, cudaMemcpy(h->d_ph_hw.ptr, hw.data(), sizeof(float) * cells, cudaMemcpyHostToDevice), "upload averaging");
+        if (mixed) {  // the mid shifts as float pairs, then the widths as floats
+            std::vector<float2> g = split_pairs(geom.data(), cells);
+            g.resize(cells + (cells + 1) / 2);
+            std::copy(geom.begin() + cells, geom.end(), reinterpret_cast<float*>(g.data() + cells));
+            CP3_CUDA(h, h->d_ph_geom_df.reserve(g.size()), "allocate averaging");
+            CP3_CUDA(h, cudaMemcpy(h->d_ph_geom_df.ptr, g.data(), sizeof(float2) * g.size(), cudaMemcpyHostToDevice), "upload averaging");
             CP3_CUDA(h, h->d_ph_prob_f.reserve(h->avg_prob.size()), "allocate averaging");
         } else {
-            CP3_CUDA(h, h->d_ph_mid.reserve(cells), "allocate averaging");
-            CP3_CUDA(h, h->d_ph_wid.reserve(cells), "allocate averaging");
-            CP3_CUDA(h, cudaMemcpy(h->d_ph_mid.ptr, mid.data(), sizeof(double) * cells, cudaMemcpyHostToDevice), "upload averaging");
-            CP3_CUDA(h, cudaMemcpy(h->d_ph_wid.ptr, wid.data(), sizeof(double) * cells, cudaMemcpyHostToDevice), "upload averaging");
+            CP3_CUDA(h, h->d_ph_geom.reserve(geom.size()), "allocate averaging");
+            CP3_CUDA(h, cudaMemcpy(h->d_ph_geom.ptr, geom.data(), sizeof(double) * geom.size(), cudaMemcpyHostToDevice), "upload averaging");
             CP3_CUDA(h, h->d_ph_prob.reserve(h->avg_prob.size()), "allocate averaging");
         }
-        // one (type, flavour) slab [ne][nc bins] at a time, through a buffer freed at the end
-        DevBuf<double> raw;
+        // as many of the six (type, flavour) slabs [ne][nc bins] at a time as fit
         const size_t slab = cells * h->ne;
-        CP3_CUDA(h, raw.reserve(slab + 1), "allocate averaging");
-        for (int k = 0; k < 6; k++) {
-            CP3_CUDA(h, cudaMemcpyAsync(raw.ptr, h->avg_prob.data() + k * slab, sizeof(double) * slab,
+        const int per = (int)std::max<size_t>(1, std::min<size_t>(6, kMaxWeightUpload / (sizeof(double) * slab)));
+        DevBuf<double> once;
+        DevBuf<double>& raw = sizeof(double) * slab * per <= kMaxWeightUpload ? h->d_ph_raw : once;
+        CP3_CUDA(h, raw.reserve(slab * per + 1), "allocate averaging");
+        for (int k = 0; k < 6; k += per) {
+            const int n = std::min(per, 6 - k);
+            CP3_CUDA(h, cudaMemcpyAsync(raw.ptr, h->avg_prob.data() + k * slab, sizeof(double) * slab * n,
                                         cudaMemcpyHostToDevice, h->stream), "upload averaging");
             void* dst = mixed ? (void*)(h->d_ph_prob_f.ptr + k * slab) : (void*)(h->d_ph_prob.ptr + k * slab);
-            CP3_CUDA(h, launch_weights_transpose(raw.ptr, h->ne, (long long)cells, dst, mixed, h->stream), "transpose averaging");
+            CP3_CUDA(h, launch_weights_transpose(raw.ptr, h->ne, (long long)cells, n, dst, mixed, h->stream), "transpose averaging");
         }
         int scaled = 0;
         if (!mixed) {  // weights that are no distribution: their scales, used where one is not zero
-            int* any = reinterpret_cast<int*>(raw.ptr + slab);
+            int* any = reinterpret_cast<int*>(raw.ptr + slab * per);
             CP3_CUDA(h, h->d_ph_scale.reserve(6 * (size_t)h->nc * h->ne), "allocate averaging");
             CP3_CUDA(h, cudaMemsetAsync(any, 0, sizeof(int), h->stream), "scale averaging");
             CP3_CUDA(h, launch_weight_scales(h->d_ph_prob.ptr, h->nc, nb, h->ne, h->d_ph_scale.ptr, any, h->stream),
@@ -378,14 +384,14 @@ int prepare_averaging(cp3_propagator* h, AvgArrays* av, AvgMixed* avm) {
     }
     if (mixed) {
         avm->prob = h->d_ph_prob_f.ptr;
-        avm->hm = h->d_ph_hm.ptr;
-        avm->hw = h->d_ph_hw.ptr;
+        avm->hm = h->d_ph_geom_df.ptr;
+        avm->hw = reinterpret_cast<const float*>(h->d_ph_geom_df.ptr + (size_t)h->nc * nb);
         avm->nb = nb;
         return CP3_OK;
     }
     av->prob = h->d_ph_prob.ptr;
-    av->mid = h->d_ph_mid.ptr;
-    av->wid = h->d_ph_wid.ptr;
+    av->mid = h->d_ph_geom.ptr;
+    av->wid = h->d_ph_geom.ptr + (size_t)h->nc * nb;
     av->scale = h->avg_scaled ? h->d_ph_scale.ptr : nullptr;
     av->n_bins = nb;
     return CP3_OK;

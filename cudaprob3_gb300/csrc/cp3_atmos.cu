@@ -893,7 +893,8 @@ cudaError_t launch_plane_transpose(const void* src, bool is_float, int nc, int n
     return cudaGetLastError();
 }
 
-// A matrix [rows][cols] of doubles transposed to [cols][rows] (as T): 32 x 32 tiles, one a block.
+// n matrices [rows][cols] of doubles, each transposed to [cols][rows] (as T): 32 x 32 tiles, one a
+// block, a matrix a grid row.
 template <class T>
 __global__ void __launch_bounds__(32 * 8)
     weights_transpose_kernel(const double* __restrict__ src, int rows, long long cols, T* __restrict__ dst) {
@@ -901,6 +902,8 @@ __global__ void __launch_bounds__(32 * 8)
     const int tiles = (rows + 31) / 32;
     const int r0 = (int)(blockIdx.x % tiles) * 32;
     const long long c0 = (long long)(blockIdx.x / tiles) * 32;
+    src += blockIdx.y * (size_t)rows * cols;
+    dst += blockIdx.y * (size_t)rows * cols;
     for (int k = threadIdx.y; k < 32; k += 8)
         if (r0 + k < rows && c0 + threadIdx.x < cols) tile[k][threadIdx.x] = src[(size_t)(r0 + k) * cols + c0 + threadIdx.x];
     __syncthreads();
@@ -908,16 +911,16 @@ __global__ void __launch_bounds__(32 * 8)
         if (c0 + k < cols && r0 + (int)threadIdx.x < rows) dst[(size_t)(c0 + k) * rows + r0 + threadIdx.x] = (T)tile[threadIdx.x][k];
 }
 
-cudaError_t launch_weights_transpose(const double* src, int rows, long long cols, void* dst,
+cudaError_t launch_weights_transpose(const double* src, int rows, long long cols, int n, void* dst,
                                      bool to_float, cudaStream_t s) {
-    if (rows <= 0 || cols <= 0) return cudaSuccess;
+    if (rows <= 0 || cols <= 0 || n <= 0) return cudaSuccess;
     const long long blocks = (long long)((rows + 31) / 32) * ((cols + 31) / 32);
-    if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
-    const dim3 block(32, 8);
+    if (blocks > 0x7fffffffLL || n > 65535) return cudaErrorInvalidValue;
+    const dim3 grid((unsigned)blocks, n), block(32, 8);
     if (to_float)
-        weights_transpose_kernel<float><<<(unsigned)blocks, block, 0, s>>>(src, rows, cols, (float*)dst);
+        weights_transpose_kernel<float><<<grid, block, 0, s>>>(src, rows, cols, (float*)dst);
     else
-        weights_transpose_kernel<double><<<(unsigned)blocks, block, 0, s>>>(src, rows, cols, (double*)dst);
+        weights_transpose_kernel<double><<<grid, block, 0, s>>>(src, rows, cols, (double*)dst);
     return cudaGetLastError();
 }
 

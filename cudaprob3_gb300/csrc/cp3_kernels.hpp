@@ -131,8 +131,8 @@ cudaError_t launch_atmos_mixed_inline(const OscParams& p, const double* energies
 // The weights' scales [2][3][nc][ne] (fx_weight_scale); *any is set where one is not zero.
 cudaError_t launch_weight_scales(const double* prob, int nc, int n_bins, int ne, signed char* scale,
                                  int* any, cudaStream_t s);
-// A matrix [rows][cols] of doubles transposed to [cols][rows], as floats or doubles.
-cudaError_t launch_weights_transpose(const double* src, int rows, long long cols, void* dst,
+// n matrices [rows][cols] of doubles, each transposed to [cols][rows], as floats or doubles.
+cudaError_t launch_weights_transpose(const double* src, int rows, long long cols, int n, void* dst,
                                      bool to_float, cudaStream_t s);
 
 // out[i] = (x[i] rounded to float, the remainder rounded to float), on the device.

@@ -149,3 +149,46 @@ def test_averaged_results_to_host_in_row_pieces(prec, poly):
         p.calculate_to_host_async(0, host.data_ptr(), chunks)
         p.synchronize()
         assert np.array_equal(host.numpy().reshape(want.shape), want), chunks
+
+
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+def test_weights_uploaded_in_pieces_equal_those_uploaded_at_once(prec):
+    """Weights beyond one upload's size (five of the six slabs, then one): the rows of a small
+    grid, uploaded at once, come out the same."""
+    nc, ne, nb, few = 100, 200, 20, 7
+    m = earth.NOMINAL
+    mix6 = [m.theta12, m.theta13, m.theta23, m.dcp, m.dm12sq, m.dm23sq]
+    cz, en = earth.cosine_grid(nc), earth.log_energy_grid(ne)
+    w = np.random.default_rng(8).uniform(0.1, 1.0, (2, 3, ne, nc, nb))
+    w /= w.sum(axis=-1, keepdims=True)
+    edges = np.linspace(5.0, 45.0, nb + 1)
+    for anti in (False, True):
+        args = (*earth.PREM_4LAYER, 22.0, nb)
+        knu = -1 if anti else 1
+        all_rows = run_avg(prec, mix6, knu, anti, cz, en, *args, w.ravel(), edges)
+        first = run_avg(prec, mix6, knu, anti, cz[:few], en, *args, w[:, :, :, :few].ravel(), edges)
+        assert np.array_equal(all_rows[:few], first)
+
+
+def test_new_weights_on_a_small_grid_cost_little():
+    """A pass on new weights of a small grid against one on the same weights: an upload and a
+    launch or two more (35 us; six uploads and launches, with buffers of their own, took 85)."""
+    import time
+    nc, ne, nb, m = 40, 40, 3, earth.NOMINAL
+    p = AtmosCudaPropagatorSingle(0, nc, ne, precision="mixed")
+    p.setEnergyList(earth.log_energy_grid(ne))
+    p.setCosineList(earth.cosine_grid(nc))
+    p.setMNSMatrix(m.theta12, m.theta13, m.theta23, m.dcp, 1)
+    p.setNeutrinoMasses(m.dm12sq, m.dm23sq)
+    p.setDensity(*earth.PREM_4LAYER)
+    p.setProductionHeight(22.0)
+    p.SetNumberOfProductionHeightBinsForAveraging(nb)
+    w, edges = np.full(6 * nc * ne * nb, 1.0 / nb), np.linspace(5.0, 45.0, nb + 1)
+    new, same = [], []
+    for _ in range(40):
+        p.setProductionHeightList(w, edges)
+        for times in (new, same):
+            t = time.perf_counter()
+            p.calculateProbabilities(0)
+            times.append(time.perf_counter() - t)
+    assert min(new) - min(same) < 60e-6, (min(new), min(same))
