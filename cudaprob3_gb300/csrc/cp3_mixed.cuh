@@ -494,167 +494,6 @@ __device__ __forceinline__ void store_columns(const float2 a[3], const float2 b[
     }
 }
 
-// One atmospheric bin over M+1 segments, generic in where each segment's layer comes from:
-// seg(l, F) fills F for segment l (0 = air, then shells inwards).
-// B <- B^T S_M B for the innermost layer F = S_M (complex symmetric: the upper triangle of
-// B^T X, X = S_M B, is formed and mirrored).
-__device__ __forceinline__ void close_palindrome(const Layer& F, cg9& B) {
-    cg9 X = B, Q;
-    apply_left(F, X);
-#pragma unroll
-    for (int i = 0; i < 3; i++)
-#pragma unroll
-        for (int j = i; j < 3; j++) {
-            const cacc h = cdot3(B.a[0][i], X.a[0][j], B.a[1][i], X.a[1][j], B.a[2][i], X.a[2][j]);
-            Q.a[i][j] = cf{h.r.x - h.i.y, h.r.y + h.i.x};
-        }
-#pragma unroll
-    for (int i = 0; i < 3; i++)
-#pragma unroll
-        for (int j = 0; j < i; j++) Q.a[i][j] = Q.a[j][i];
-    B = Q;
-}
-
-// The bin's amplitude before the air layer, for M >= 1: G = B^T S_M B (M >= 2) or S_1 (M = 1),
-// with B = S_{M-1}..S_1; seg(l, F) fills layer l.
-template <class SegFn>
-__device__ __forceinline__ void chain_mixed(SegFn seg, int M, cg9& G) {
-    Layer F;
-    seg(1, F);
-    layer_to_gen(F, G);  // B = S_1
-    if (M > 1) {
-        cg9& B = G;
-        for (int l = 2; l < M; l++) {
-            seg(l, F);
-            apply_left(F, B);
-        }
-        seg(M, F);
-        close_palindrome(F, G);
-    }
-}
-
-// ---- the end of a bin on two vectors -------------------------------------------------------
-// Of the amplitude A = W (B^T S_M B) S_0 W^+ only the columns e and mu are formed, each by
-// taking S_0 W^+'s column through the matrices: 2 x 104 operations after the chain, where
-// forming B^T S_M B and the product with S_0 took 276.  The tau column is conj(a_e x a_mu) up
-// to a phase, which its moduli do not see.
-
-// S_0 W^+'s columns e and mu: W^+ e = (1, 0, 0), W^+ mu = (0, c, s e^{-i delta}).
-__device__ __forceinline__ void initial_columns(const Layer& f, const WParams& w, float2 a[3], float2 b[3]) {
-    const float sr = w.s * w.er, si = -w.s * w.ei;
-    a[0] = make_float2(1.0f, 0.0f), a[1] = a[2] = make_float2(0.0f, 0.0f);
-    b[0] = make_float2(0.0f, 0.0f), b[1] = make_float2(w.c, 0.0f), b[2] = make_float2(sr, si);
-#pragma unroll
-    for (int k = 0; k < 2; k++) {
-        const float* u = f.u[k];
-        const float zr = f.z[k][0], zi = f.z[k][1];
-        const float2 y = __fmul2_rn(bc2(u[0]), make_float2(zr, zi));
-        const float vr = fmaf(u[2], sr, u[1] * w.c), vi = u[2] * si;
-        const float2 x = make_float2(fmaf(zr, vr, -zi * vi), fmaf(zr, vi, zi * vr));
-#pragma unroll
-        for (int i = 0; i < 3; i++) {
-            a[i] = __ffma2_rn(bc2(u[i]), y, a[i]);
-            b[i] = __ffma2_rn(bc2(u[i]), x, b[i]);
-        }
-    }
-}
-
-// k <- S k
-__device__ __forceinline__ void apply_layer(const Layer& f, float2 k[3]) {
-#pragma unroll
-    for (int q = 0; q < 2; q++) {
-        const float* u = f.u[q];
-        const float zr = f.z[q][0], zi = f.z[q][1];
-        float2 v = __fmul2_rn(bc2(u[0]), k[0]);
-        v = __ffma2_rn(bc2(u[1]), k[1], v);
-        v = __ffma2_rn(bc2(u[2]), k[2], v);
-        const float2 y = make_float2(fmaf(zr, v.x, -zi * v.y), fmaf(zr, v.y, zi * v.x));
-#pragma unroll
-        for (int i = 0; i < 3; i++) k[i] = __ffma2_rn(bc2(u[i]), y, k[i]);
-    }
-}
-
-// k <- B^T S B k
-__device__ __forceinline__ void apply_palindrome(const cg9& B, const Layer& f, float2 k[3]) {
-    float2 m[3];
-#pragma unroll
-    for (int i = 0; i < 3; i++) {
-        const cacc h = cdot3(B.a[i][0], fc(k[0]), B.a[i][1], fc(k[1]), B.a[i][2], fc(k[2]));
-        m[i] = make_float2(h.r.x - h.i.y, h.r.y + h.i.x);
-    }
-    apply_layer(f, m);
-#pragma unroll
-    for (int i = 0; i < 3; i++) {
-        const cacc h = cdot3(B.a[0][i], fc(m[0]), B.a[1][i], fc(m[1]), B.a[2][i], fc(m[2]));
-        k[i] = make_float2(h.r.x - h.i.y, h.r.y + h.i.x);
-    }
-}
-
-__device__ __forceinline__ float norm2(const float2 a[3]) {
-    float2 q = __fmul2_rn(a[0], a[0]);
-    q = __ffma2_rn(a[1], a[1], q);
-    q = __ffma2_rn(a[2], a[2], q);
-    return q.x + q.y;
-}
-
-// One Newton-Schulz step toward orthonormal columns, [a b] <- [a b] (3 - [a b]^+ [a b]) / 2: the
-// rounding of FP32 layers leaves each slightly non-unitary, and that part of the error
-// accumulates over the ~2M products of a deep trajectory; the step removes it to second order.
-// Below kOrthogonalMinShells only the norms are put right, which is nearly all of it there; not
-// even these, and the third column, formed from the two, is further off than a matrix formed
-// whole (PREM-4 2-norm 1.7e-7).  With the step whatever M the error is the same and the batches
-// are slower (32 PREM-12 problems alone 634 us, norms below M = 6 632, below 12 623; a mix of
-// PREM-4 grids 229, 225 and 225).
-// 2-norm error against the FP64 bins, and the per-bin kernel's time, with this end of the bin
-// and with the matrix formed whole and corrected from M = 6: PREM-4 400 x 400 0.9e-7 and 1.5e-7,
-// 7.9 and 7.8 us; PREM-12 1000 x 1000 1.1e-7 and 1.4e-7, 30.3 and 32.4 us; 59 shells 2000 x 2000
-// 1.4e-7 and 1.5e-7, 178 and 185 us.
-constexpr int kOrthogonalMinShells = 12;
-__device__ __forceinline__ void orthonormalize(float2 a[3], float2 b[3], int M) {
-    const float na = fmaf(-0.5f, norm2(a), 1.5f), nb = fmaf(-0.5f, norm2(b), 1.5f);
-    if (M < kOrthogonalMinShells) {  // the norms alone
-#pragma unroll
-        for (int i = 0; i < 3; i++) {
-            a[i] = __fmul2_rn(a[i], bc2(na));
-            b[i] = __fmul2_rn(b[i], bc2(nb));
-        }
-        return;
-    }
-    const cacc h = cdot3(fc(a[0]), fc(b[0]), fc(a[1]), fc(b[1]), fc(a[2]), fc(b[2]));
-    const float dr = -0.5f * (h.r.x + h.i.y), di = -0.5f * (h.r.y - h.i.x);  // -a^+ b / 2
-#pragma unroll
-    for (int i = 0; i < 3; i++) {
-        const float2 x = a[i], y = b[i];
-        a[i] = make_float2(fmaf(na, x.x, fmaf(dr, y.x, di * y.y)), fmaf(na, x.y, fmaf(dr, y.y, -di * y.x)));
-        b[i] = make_float2(fmaf(nb, y.x, fmaf(dr, x.x, -di * x.y)), fmaf(nb, y.y, fmaf(dr, x.y, di * x.x)));
-    }
-}
-
-// The nine probabilities from the two columns in the rotated basis: W = [[1,0,0],[0,c,s e],
-// [0,-s,c e]], e = e^{i delta}; channel j*3+i = |A_ij|^2 at out[ch * plane].
-__device__ __forceinline__ void store_columns(const float2 a[3], const float2 b[3], const WParams& w,
-                                              float* __restrict__ out, size_t plane) {
-    cf v[2][3];
-#pragma unroll
-    for (int j = 0; j < 2; j++) {
-        const float2* k = j == 0 ? a : b;
-        const cf g{fmaf(k[2].x, w.er, -k[2].y * w.ei), fmaf(k[2].x, w.ei, k[2].y * w.er)};  // e k2
-        v[j][0] = fc(k[0]);
-        v[j][1] = cf{fmaf(w.c, k[1].x, w.s * g.re), fmaf(w.c, k[1].y, w.s * g.im)};
-        v[j][2] = cf{fmaf(-w.s, k[1].x, w.c * g.re), fmaf(-w.s, k[1].y, w.c * g.im)};
-#pragma unroll
-        for (int i = 0; i < 3; i++)
-            out[(size_t)(j * 3 + i) * plane] = fmaf(v[j][i].re, v[j][i].re, v[j][i].im * v[j][i].im);
-    }
-#pragma unroll
-    for (int i = 0; i < 3; i++) {
-        const cf p = v[0][(i + 1) % 3], q = v[0][(i + 2) % 3], r = v[1][(i + 1) % 3], t = v[1][(i + 2) % 3];
-        const float re = fmaf(p.re, t.re, fmaf(-p.im, t.im, fmaf(-q.re, r.re, q.im * r.im)));
-        const float im = fmaf(p.re, t.im, fmaf(p.im, t.re, fmaf(-q.re, r.im, -q.im * r.re)));
-        out[(size_t)(6 + i) * plane] = fmaf(re, re, im * im);
-    }
-}
-
 // One or two FP32 layers are unitary to ~1e-7 already; the correction pays off from the longer
 // chains on.
 __device__ __forceinline__ void finish_columns(float2 a[3], float2 b[3], int M, const WParams& w,
