@@ -264,11 +264,6 @@ CP3_HD df df_mul(df x, df y) {
     e = fmaf(x.hi, y.lo, fmaf(x.lo, y.hi, e));
     return df_fast2sum(p, e);
 }
-CP3_HD df df_mulf(df x, float y) {
-    const float p = CP3_FMUL(x.hi, y);
-    const float e = fmaf(x.hi, y, -p);
-    return df_fast2sum(p, fmaf(x.lo, y, e));
-}
 // 1 / x to df64 accuracy from a float estimate r: with e = 1 - x r (its leading part exact
 // through the FMA), 1 / x = r (1 + e + e^2), to e^3 ~ 2^-66.  The approximate reciprocal is
 // enough as the estimate (8 operations; the divide and a Newton step in df64 arithmetic took

@@ -332,9 +332,6 @@ __device__ __forceinline__ void store_one_layer(const Layer& F, const WParams& w
                 make_float2(F.z[0][1], F.z[1][1]), out, plane);
 }
 
-
-// One atmospheric bin over M+1 segments, generic in where each segment's layer comes from:
-// seg(l, F) fills F for segment l (0 = air, then shells inwards).
 // B <- B^T S_M B for the innermost layer F = S_M (complex symmetric: the upper triangle of
 // B^T X, X = S_M B, is formed and mirrored).
 __device__ __forceinline__ void close_palindrome(const Layer& F, cg9& B) {
@@ -492,14 +489,6 @@ __device__ __forceinline__ void store_columns(const float2 a[3], const float2 b[
         const float im = fmaf(p.re, t.im, fmaf(p.im, t.re, fmaf(-q.re, r.im, -q.im * r.re)));
         out[(size_t)(6 + i) * plane] = fmaf(re, re, im * im);
     }
-}
-
-// One or two FP32 layers are unitary to ~1e-7 already; the correction pays off from the longer
-// chains on.
-__device__ __forceinline__ void finish_columns(float2 a[3], float2 b[3], int M, const WParams& w,
-                                               float* __restrict__ out, size_t plane) {
-    orthonormalize(a, b, M);
-    store_columns(a, b, w, out, plane);
 }
 
 // One atmospheric bin over M+1 segments, generic in where each segment's layer comes from:
