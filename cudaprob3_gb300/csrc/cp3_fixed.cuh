@@ -12,8 +12,11 @@
 // Cauchy-Schwarz a dot product of unit vectors with three terms (or two complex ones) keeps
 // the cross terms below 2^63 in one accumulator, longer ones use two.
 //
-// All functions are plain integer arithmetic but for the phase reduction (four FP64 operations
-// a phase), and run on the host as well.
+// Integer arithmetic but for: a phase's reduction (four FP64 operations), the determinant's of a
+// chain's end, the quotients of fx_refine (FP32) and the rates it returns (FP64), the arguments of
+// the height sums and sin(x) / x beyond the series (FP64), and the start from double-floats (FP32).
+// All of it runs on the host as well, except fx_solve, whose eigen-solver takes paired FP32
+// instructions.
 #pragma once
 
 #include <cstring>
@@ -702,39 +705,69 @@ CP3_HD void fx_class_f64(double u[2][3], const double dmv[3], double E, FxClass&
         o.rate[k] = ok ? (dmv[k + 1] - dmv[0]) * kFxTurns / E : fx_bits_to_double(0x7ff8000000000000LL);
 }
 
-#ifdef __CUDACC__
-// x as a float pair, from its bits (conversions between double and float take the FP64 pipe).
-__device__ __forceinline__ bool fx_float_pair(double x, df& o) {
-    const long long b = __double_as_longlong(x);
-    const int e = (int)((b >> 52) & 0x7ff);
-    if ((b << 1) == 0) {
+CP3_HD unsigned int fx_float_bits(float x) {
+#ifdef __CUDA_ARCH__
+    return __float_as_uint(x);
+#else
+    unsigned int b;
+    std::memcpy(&b, &x, sizeof b);
+    return b;
+#endif
+}
+CP3_HD float fx_bits_to_float(unsigned int b) {
+#ifdef __CUDA_ARCH__
+    return __uint_as_float(b);
+#else
+    float x;
+    std::memcpy(&x, &b, sizeof x);
+    return x;
+#endif
+}
+
+// x as a float pair, from its bits (conversions between double and float take the FP64 pipe);
+// false outside 2^-60..2^61 and for what is no number.
+CP3_HD bool fx_float_pair(double x, df& o) {
+    const long long b = fx_bits(x);
+    const int e = fx_exponent(x);
+    if ((unsigned long long)b << 1 == 0) {
         o = df{0.0f, 0.0f};
         return true;
     }
     if (e < 1023 - 60 || e > 1023 + 60) return false;
-    const unsigned int sign = (unsigned int)(b >> 63) << 31;
-    const float hi = __uint_as_float(sign | ((unsigned int)(e - 896) << 23) | ((unsigned int)(b >> 29) & 0x7fffffu));
-    const float lo = (float)(unsigned int)(b & 0x1fffffff) * __uint_as_float(sign | ((unsigned int)(e - 948) << 23));
+    const unsigned int sign = b < 0 ? 0x80000000u : 0u;
+    const float hi = fx_bits_to_float(sign | ((unsigned int)(e - 896) << 23) | ((unsigned int)(b >> 29) & 0x7fffffu));
+    const float lo = (float)(unsigned int)(b & 0x1fffffff) * fx_bits_to_float(sign | ((unsigned int)(e - 948) << 23));
     o = df_fast2sum(hi, lo);
     return true;
 }
-__device__ __forceinline__ double fx_to_f64(float x) {  // normal or zero (zero: 1e-38)
-    const unsigned int b = __float_as_uint(x);
-    return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + 0x38000000u)), (int)(b << 29));
+CP3_HD double fx_to_f64(float x) {  // normal or zero (zero: 1e-38)
+    const unsigned int b = fx_float_bits(x);
+    return fx_bits_to_double((long long)((unsigned long long)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + 0x38000000u)) << 32 |
+                                         (unsigned int)(b << 29)));
 }
-__device__ __forceinline__ fx fx_from_pair(float hi, float lo) {  // |hi + lo| <= 1
+CP3_HD fx fx_from_pair(float hi, float lo) {  // |hi + lo| <= 1
+#ifdef __CUDA_ARCH__
     const int i = __float2int_rn(hi * 1073741824.0f);
+#else
+    const int i = (int)rintf(hi * 1073741824.0f);
+#endif
     const float rest = fmaf(-(float)i, 9.31322574615478515625e-10f, hi) + lo;  // 2^-30
-    return fx_split(((long long)i << 32) + __float2ll_rn(rest * 4611686018427387904.0f));
+#ifdef __CUDA_ARCH__
+    const long long r = __float2ll_rn(rest * 4611686018427387904.0f);
+#else
+    const long long r = (long long)rintf(rest * 4611686018427387904.0f);
+#endif
+    return fx_split((long long)((unsigned long long)(long long)i << 32) + r);
 }
 
 // 1 / E, rounded once but for a last-place error of the correction
-__device__ __forceinline__ double fx_reciprocal(double E, df Ed) {
+CP3_HD double fx_reciprocal(double E, df Ed) {
     const df r = df_recip(Ed);
     const double r0 = fx_to_f64(r.hi) + fx_to_f64(r.lo);
     return fma(fma(-E, r0, 1.0), r0, r0);
 }
 
+#ifdef __CUDACC__
 static __device__ __noinline__ void fx_solve_f64(const OscParams* __restrict__ p, double E, double rho, FxClass* o) {
     double u[2][3], dmv[3];
     rotated_layer_f64(p, E, rho, u, dmv);

@@ -175,3 +175,13 @@ extern "C" int fixed_inline(const double* mix, int knutype, int anti, const doub
 }
 
 extern "C" long long fixed_negated(long long v) { return fx_value(fx_neg(fx_split(v))); }
+
+// x as a float pair (0 where it is refused), one over it, and a fixed-point number from a pair.
+extern "C" int fixed_pair(double x, float* pair, double* reciprocal) {
+    df d;
+    if (!fx_float_pair(x, d)) return 0;
+    pair[0] = d.hi, pair[1] = d.lo;
+    *reciprocal = fx_reciprocal(x, d);
+    return 1;
+}
+extern "C" long long fixed_from_pair(float hi, float lo) { return fx_value(fx_from_pair(hi, lo)); }

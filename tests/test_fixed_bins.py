@@ -42,6 +42,38 @@ def host_bins(lib, m, anti, cz, en, model, h, refine=1):
     return np.transpose(out, (1, 2, 0)), n
 
 
+def test_float_pairs_and_reciprocals(host):
+    """The start of the eigen-solver: a double as a float pair to 2^-48 (a low word of 29 bits
+    rounded to 24, below 2^-23), from 2^-60 to 2^61 and nothing else; its reciprocal to a unit and
+    a half of the last place; a fixed-point number from a pair to the rounding of 2^-30 2^-24."""
+    host.fixed_pair.argtypes = [C.c_double, C.c_void_p, C.c_void_p]
+    host.fixed_from_pair.argtypes = [C.c_float, C.c_float]
+    host.fixed_from_pair.restype = C.c_longlong
+    pair, rec = np.zeros(2, dtype=np.float32), C.c_double()
+
+    def split(x):
+        return host.fixed_pair(x, pair.ctypes.data, C.byref(rec))
+
+    rng = np.random.default_rng(13)
+    values = np.concatenate([np.exp(rng.uniform(np.log(1e-3), np.log(1e6), 4000)), 2.0 ** np.arange(-60, 61),
+                             np.nextafter(2.0 ** np.arange(-59, 62), 0), np.nextafter(2.0 ** np.arange(-60, 61), 1e99)])
+    for x in np.concatenate([values, -values]):
+        assert split(x), x
+        hi, lo = float(pair[0]), float(pair[1])
+        assert abs(lo) <= 2.0 ** -24 * abs(hi) * (1 + 2.0 ** -20)
+        assert abs((hi - x) + lo) <= 2.0 ** -48 * abs(x)
+        assert abs(rec.value * np.longdouble(x) - 1) <= 1.5 * 2.0 ** -52
+    for x in (0.0, -0.0):
+        assert split(x) and not pair.any()
+    for x in (np.nan, np.inf, -np.inf, 2.0 ** 61, 2.0 ** -60 * (1 - 2.0 ** -53), 5e-324, -1e300):
+        assert not split(x), x
+    for x in np.concatenate([rng.uniform(-1, 1, 4000), [1.0, -1.0, 0.0, 2.0 ** -31, 1e-12]]):
+        hi = np.float32(x)
+        lo = np.float32(x - float(hi))
+        exact = (int(float(hi) * 2.0 ** 80) + int(float(lo) * 2.0 ** 80)) / 2.0 ** 18
+        assert abs(host.fixed_from_pair(hi, lo) - exact) <= 2.0 ** (62 - 54) + 1
+
+
 def omix(m, anti):
     return OMix(m.theta12, m.theta13, m.theta23, m.dcp, m.dm12sq, m.dm23sq, -1 if anti else 1)
 
