@@ -185,3 +185,20 @@ extern "C" int fixed_pair(double x, float* pair, double* reciprocal) {
     return 1;
 }
 extern "C" long long fixed_from_pair(float hi, float lo) { return fx_value(fx_from_pair(hi, lo)); }
+
+// A row's segment lengths (km) and electron densities, as the bins take them; their number.
+extern "C" int fixed_segments(double cz, const double* radii, const double* rho, const double* ye, int n,
+                              double height_km, double* len, double* rho_e) {
+    EarthModel model;
+    std::string msg;
+    TrajectoryTable t;
+    if (make_earth_model(radii, rho, nullptr, nullptr, ye, n, false, &model, &msg) ||
+        build_trajectories(model, &cz, 1, height_km * 1e5, &t, &msg))
+        return -1;
+    const int m = t.maxlayers[0] + 1;
+    for (int l = 0; l < m; l++) {
+        len[l] = t.len_km[t.offset[0] + l];
+        rho_e[l] = l ? model.rho[l - 1] * model.ye[l - 1] : 0.0;
+    }
+    return m;
+}

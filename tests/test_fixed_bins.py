@@ -114,6 +114,53 @@ def test_host_bins_against_oracle(host, oracle, shells, h):
                 assert np.abs(got - ref).max() <= 1e-12
 
 
+@pytest.mark.parametrize("shells", [1, 4, 12, 59])
+def test_host_bins_against_forty_digits(host, shells):
+    """The parity bar of 1e-12 would not see two digits lost.  Against 40-digit arithmetic on the
+    same segments a probability is off by twice its phase's error: the rates are rounded four times
+    on the way (2.5 2^-52 of the phase, 2.534 |dm| L / E), a layer's sine and cosine are good to
+    2^-56, twice a layer and twice through the chain, and the mixing matrix is one of doubles."""
+    mp = pytest.importorskip("mpmath").mp.clone()
+    mp.dps = 40
+    model = earth.synthetic_shells(shells)
+    m = earth.gaussian_sets(3, seed=7)[2]
+    arrays = [np.ascontiguousarray(x, dtype=np.float64) for x in model]
+    cz, en = np.array([-1.0, -0.83, -0.41, -0.05, 0.3]), np.array([0.7, 3.0, 20.0, 150.0])
+    O = (mp.matrix([[mp.cos(m.theta13), 0, mp.sin(m.theta13)], [0, 1, 0], [-mp.sin(m.theta13), 0, mp.cos(m.theta13)]]) *
+         mp.matrix([[mp.cos(m.theta12), mp.sin(m.theta12), 0], [-mp.sin(m.theta12), mp.cos(m.theta12), 0], [0, 0, 1]]))
+    H0 = O * mp.diag([0, mp.mpf(m.dm12sq), mp.mpf(m.dm12sq) + mp.mpf(m.dm23sq)]) * O.T
+    for anti in (False, True):
+        got, outside = host_bins(host, m, anti, cz, en, model, 22.0)
+        assert outside == 0
+        W = (mp.matrix([[1, 0, 0], [0, mp.cos(m.theta23), mp.sin(m.theta23)], [0, -mp.sin(m.theta23), mp.cos(m.theta23)]]) *
+             mp.diag([1, 1, mp.expj(-m.dcp if anti else m.dcp)]))
+        for ie, E in enumerate(en):
+            eigen = {}
+            for ic, c in enumerate(cz):
+                length, rho_e = np.empty(200), np.empty(200)
+                n = host.fixed_segments(C.c_double(c), *(x.ctypes.data_as(dp) for x in arrays), len(arrays[0]),
+                                        C.c_double(22.0), length.ctypes.data_as(dp), rho_e.ctypes.data_as(dp))
+
+                def layer(l):
+                    if l not in eigen:
+                        H = H0.copy()
+                        H[0, 0] += (-1 if anti else 1) * mp.mpf(1.52588e-4) * mp.mpf(float(E)) * mp.mpf(float(rho_e[l]))
+                        eigen[l] = mp.eigsy(H)
+                    lam, U = eigen[l]
+                    f = mp.mpf(2.534) * mp.mpf(float(length[l])) / mp.mpf(float(E))
+                    return U * mp.diag([mp.expj(-(x - lam[0]) * f) for x in lam]) * U.T
+
+                G = mp.eye(3)
+                for l in range(1, n - 1):
+                    G = layer(l) * G
+                G = G.T * layer(n - 1) * G if n > 1 else G
+                A = W * G * layer(0) * W.H
+                ref = [float(abs(A[b, a]) ** 2) for a in range(3) for b in range(3)]
+                total = length[0] + 2 * length[1:n].sum()
+                phase = 2.534 * (abs(m.dm12sq) + abs(m.dm23sq) + 1.53e-4 * E * rho_e[:n].max()) * total / E
+                assert np.abs(got[ic, ie] - ref).max() <= 2 * (2.5 * 2.0 ** -52 * phase + 4 * n * 2.0 ** -56 + 2e-16), (c, E)
+
+
 @pytest.mark.parametrize("dm23sq", [1e-10, 2e-11, -1e-11])
 def test_nearly_equal_levels_stay_in_fixed_point(host, oracle, dm23sq):
     """Two vacuum levels a millionth of the spread apart: the FP64 vectors of the two are not
