@@ -28,6 +28,10 @@ constexpr int kMaxGridY = 65535;
 // ------------------------------------------------------------------------------------
 // FP64: physics::calculate_atmos (physics.hpp:789-1150), within 1e-12 of the reference.
 //
+// The bins run in fixed point (cp3_fixed.cuh, the kernels below).  What follows is the FP64
+// arithmetic that takes over the bins out of its range (atmos_bin_out_of_range: a phase past 2^42
+// turns or one that is not finite, a weight that is not a number), every layer solved in place.
+//
 // The same physics as the reference in the rotated real basis of the mixed kernels
 // (cp3_mixed.cuh), in double precision: every layer is S = sum_k e^{i arg_k} P_k with the
 // reference's own phases arg_k = -2.534 dmMatVac[k][0] L / E (getArg, physics.hpp:439-450)
@@ -246,13 +250,12 @@ __device__ __forceinline__ void atmos_bin_f64(SegFn seg, int M, const double* w,
 // Bound by the integer multiply-adds and the chain they stand in (72 % of the FMA pipe's heavy
 // half, ALU 46 %, FP64 pipe 40 %; three to five blocks an SM and two to eight warps a block are
 // within 8 %).  Measured against the FP64 kernel it replaced: 59 shells, 2000 x 2000, 1.12 ms
-// (10.14); PREM-12, 307 x 811, 53 us; PREM-4, 400 x 400, 22 us (140).
+// (10.14); PREM-12, 307 x 811, 53 us (346); PREM-4, 400 x 400, 22 us (122).
 constexpr int kFxWarps = 4;
 
 __device__ const TrigTable g_trig = make_trig_table();
 
-// A bin out of the fixed-point range (a phase beyond 2^42 turns, or one that is not finite): the
-// FP64 layers solved in place.
+// A bin out of the fixed-point range: the FP64 layers solved in place.
 __device__ __noinline__ void atmos_bin_out_of_range(const OscParams* p, double E, const double* len,
                                                     const double* rho, int M, const AvgInput& av,
                                                     int ic, int nc, int ie, int ne, double* out) {

@@ -58,7 +58,7 @@ struct RowRange {
 // They read it with __ldca: its lines are written during their own grid's life, which the
 // read-only path does not allow for.  A call, before and after: FP64 PREM-4 400 x 400 40.2 and
 // 35.7 us, PREM-12 307 x 811 73 and 68, quadratic 500 x 500 75 and 68 (its bins need the air's
-// table only once their chain of layers is done); mixed PREM-4 200 x 200 to host memory 37 and 32.
+// table only once their chain of layers is done); mixed PREM-4 200 x 200 to host memory 37 and 34.
 __device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;"); }
 __device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

@@ -277,7 +277,9 @@ int cp3_batch_debug_withhold_tables(cp3_batch* b, int on);
  * reads and appends the choice to $CP3_TUNE_CACHE (default ~/.cache/cp3gb300_tune.txt),
  * keyed by GPU and batch size. */
 int cp3_batch_tune(cp3_batch* b, int use_cache);
-/* One run over every problem on `stream` (NULL = the batch's own stream). */
+/* One run over every problem on `stream` (NULL = the batch's own stream).
+ * CP3_ERR_UNSUPPORTED for a stream that is being captured: a run uploads its parameters as
+ * they change and is ordered after the last one by events, which no graph can replay. */
 int cp3_batch_run(cp3_batch* b, void* stream);
 /* One run with every result copied to dst, laid out as the arena (result_bytes bytes; each
  * problem at its cp3_batch_result_offset).  The bins run in n_pieces windows of whole
@@ -286,7 +288,8 @@ int cp3_batch_run(cp3_batch* b, void* stream);
  * the download overlaps the computation.  `stream` (NULL = the batch's own stream) waits for
  * the last copy.  The run always uses the split form (a table launch, then the bin launches)
  * and gives the same results as cp3_batch_run.  CP3_ERR_BAD_ARGUMENT for a null dst or more
- * than 8 pieces, CP3_ERR_UNSUPPORTED while cp3_batch_debug_withhold_tables is on.  (No
+ * than 8 pieces, CP3_ERR_UNSUPPORTED while cp3_batch_debug_withhold_tables is on and for a
+ * stream that is being captured (as cp3_batch_run).  (No
  * reference counterpart: the reference has no batches; its propagators download their
  * results in calculateProbabilities.) */
 int cp3_batch_run_to_host(cp3_batch* b, void* dst, int n_pieces, void* stream);
